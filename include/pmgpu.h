@@ -381,7 +381,10 @@ int pm_n_systems(pm_handle *h);
 pm_status pm_refactor(pm_handle *h, double *ms);
 
 /* Diagnostics: launches of this library's kernels since the handle was
- * created, and device bytes held. */
+ * created, and device bytes held (without the packed copy of the matrix rows
+ * that the sweeps of one-block hexahedral levels use while memory allows: it
+ * counts towards max_device_bytes but is given back when another allocation
+ * needs the room). */
 long long pm_kernel_launches(pm_handle *h);
 long long pm_device_bytes(pm_handle *h);
 /* Host bytes page-locked by pm_add_level under pin_host (0 if none took). */

@@ -28,7 +28,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
               "-Xcompiler", "-fPIC,-O3,-fopenmp", f"-I{INCLUDE}", f"-I{CSRC}"]
 GXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fopenmp", f"-I{INCLUDE}", f"-I{CSRC}"]
 
-GPU_CU = ["pm_api.cu", "pm_sparse.cu", "pm_vanka.cu", "pm_vanka_schur.cu", "pm_vanka_tma.cu",
+GPU_CU = ["pm_api.cu", "pm_sparse.cu", "pm_vanka.cu", "pm_vanka_schur.cu", "pm_vanka_tma.cu", "pm_vanka_patch.cu",
           "pm_batch.cu",
           "pm_learned.cu", "pm_mlp_tc.cu", "pm_assemble.cu",
           "pm_noalloc.cu", "pm_diag.cu"]

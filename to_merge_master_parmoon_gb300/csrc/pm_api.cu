@@ -20,6 +20,7 @@
 #include <cstring>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "pm_kernels.h"
@@ -32,6 +33,8 @@ struct pm_mlp {
 };
 
 using namespace pm;
+
+static_assert(kPatchIds == kPatchIdsHost, "patch list layout");
 
 namespace {
 double now_s() {
@@ -86,6 +89,28 @@ struct LevelDev {
   // interleaved FP32 velocity (16 bytes per node) that the one-block sweep
   // gathers from and updates; mixed precision, hexahedral smoothed levels
   float4 *ux = nullptr;
+  // packed rows of a one-block hexahedral level (pm_vanka_patch.cu): 0 not
+  // looked at yet, 1 in use, -1 not available (mesh shape, memory)
+  int pk = 0;
+  bool pk_stale = true;  // matrix values newer than the packed copy
+  int *pk_ids = nullptr, *pk_pattern = nullptr;
+  uint8_t *pk_flips = nullptr;
+  void *pk_patterns = nullptr, *pk_values = nullptr, *pk_u = nullptr, *pk_p = nullptr;
+  long long pk_npat = 0;
+  // the arrays above with their sizes in bytes (es: bytes of a value)
+  struct PatchArray {
+    void *p;
+    long long bytes;
+  };
+  std::vector<PatchArray> patch_arrays(long long es) const {
+    return {{pk_ids, (long long)ncells * kPatchIds * 4},
+            {pk_pattern, (long long)ncells * 4},
+            {pk_flips, nu},
+            {pk_patterns, pk_npat * kPatchPatternBytes},
+            {pk_values, (long long)ncells * kPatchValues * es},
+            {pk_u, (long long)nu * 8 * es},
+            {pk_p, (long long)np * es}};
+  }
   double *x64 = nullptr, *y64 = nullptr, *z64 = nullptr;
   // unique bytes of one Vanka sweep per cell, split by kernel (see pm_setup)
   double vanka_res_bytes = 0.0, vanka_apply_bytes = 0.0;
@@ -110,6 +135,8 @@ struct LevelDev {
   bool one_block() const { return structured || diag == 2; }
   // the Schur block solve of one-block levels exists for Q2 hexahedra only
   bool schur() const { return one_block() && nl == NU_LOC; }
+  // sweeps run from the packed rows
+  bool packed() const { return pk == 1 && schur(); }
   // block elimination with three diagonal blocks (decoupled nine-block levels)
   bool schur3() const { return diag == 1 && nl == NU_LOC; }
   size_t fac_bytes = 0;  // allocated factor storage
@@ -170,6 +197,8 @@ DevOp<float> LevelDev::op<float>() const {
 
 struct pm_handle {
   pm_options opt;
+  bool patch_alloc = false;   // allocating packed rows (no eviction)
+  long long patch_bytes = 0;  // held for them, not part of `bytes`
   double t_update0 = 0.0;  // host clock at pm_update_matrices entry (verbose timing)
   cudaStream_t stream = nullptr;
   std::vector<LevelDev> L;
@@ -242,15 +271,15 @@ pm_status cuda_fail(pm_handle *h, const char *what) {
   return (e == cudaErrorMemoryAllocation) ? PM_OOM : PM_CUDA_ERROR;
 }
 
+bool release_patches(pm_handle *h);
+
 template <typename T>
-pm_status dalloc(pm_handle *h, T **p, size_t count) {
-  *p = nullptr;
-  if (count == 0) count = 1;
+pm_status dalloc_once(pm_handle *h, T **p, size_t count) {
   if (h->opt.max_device_bytes > 0 &&
-      h->bytes + (long long)(count * sizeof(T)) > h->opt.max_device_bytes) {
+      h->bytes + h->patch_bytes + (long long)(count * sizeof(T)) > h->opt.max_device_bytes) {
     h->err = "device allocation of " + std::to_string(count * sizeof(T)) +
              " bytes exceeds max_device_bytes (" + std::to_string(h->opt.max_device_bytes) +
-             ", " + std::to_string(h->bytes) + " held)";
+             ", " + std::to_string(h->bytes + h->patch_bytes) + " held)";
     return PM_OOM;
   }
   void *q = nullptr;
@@ -262,9 +291,20 @@ pm_status dalloc(pm_handle *h, T **p, size_t count) {
     return e == cudaErrorMemoryAllocation ? PM_OOM : PM_CUDA_ERROR;
   }
   h->allocs.push_back(q);
-  h->bytes += (long long)(count * sizeof(T));
+  (h->patch_alloc ? h->patch_bytes : h->bytes) += (long long)(count * sizeof(T));
   *p = static_cast<T *>(q);
   return PM_OK;
+}
+
+// Device memory of the handle.  The packed rows are a copy that the sweeps
+// can do without: when an allocation does not fit, they are given back first.
+template <typename T>
+pm_status dalloc(pm_handle *h, T **p, size_t count) {
+  *p = nullptr;
+  if (count == 0) count = 1;
+  const pm_status s = dalloc_once(h, p, count);
+  if (s != PM_OOM || h->patch_alloc || !release_patches(h)) return s;
+  return dalloc_once(h, p, count);
 }
 
 // CSR value / column arrays: padded by 8 zero entries so that the Vanka
@@ -358,6 +398,50 @@ pm_status level_defect(pm_handle *h, const LevelDev &Lv, const T *u, const T *f,
 }
 
 template <typename T>
+PatchLevel<T> patch_level(const pm_handle *h, const LevelDev &Lv) {
+  PatchLevel<T> L;
+  L.nu = Lv.nu;
+  L.patterns = static_cast<const PatchPattern *>(Lv.pk_patterns);
+  L.pattern = Lv.pk_pattern;
+  L.ids = Lv.pk_ids;
+  L.flips = Lv.pk_flips;
+  L.values = L.values_w = static_cast<T *>(Lv.pk_values);
+  L.u = Lv.pk_u;
+  L.p = static_cast<T *>(Lv.pk_p);
+  return L;
+}
+
+// `sweeps` sweeps from the packed rows (one launch per colour), with the
+// Dirichlet nodes set before, between and after them as vanka_sweep does
+template <typename T>
+pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps) {
+  const PatchLevel<T> L = patch_level<T>(h, Lv);
+  const int ncol = (int)Lv.colouring.ptr.size() - 1;
+  PM_LAUNCH(launch_patch_begin<T>(L, u, rhs, Lv.hb, Lv.np, h->stream));
+  for (int s = 0; s < sweeps; ++s) {
+    if (s > 0) PM_LAUNCH(launch_patch_between<T>(L, rhs, Lv.hb, h->stream));
+    for (int k = 0; k < ncol; ++k) {
+      const int b = Lv.colouring.ptr[k], n = Lv.colouring.ptr[k + 1] - b;
+      if (n == 0) continue;
+      const bool prof = h->prof && h->evused + 3 <= h->evpool.size();
+      if (prof) cudaEventRecord(h->evpool[h->evused], h->stream);
+      PM_LAUNCH(launch_patch_colour<T>(L, Lv.colour_cells + b, n,
+                                       static_cast<const T *>(Lv.factors), rhs,
+                                       (T)h->opt.smooth_damp, s & 1, h->stream));
+      if (prof) {  // residual and local solve are one launch: all of it is kernel 0
+        cudaEventRecord(h->evpool[h->evused + 1], h->stream);
+        cudaEventRecord(h->evpool[h->evused + 2], h->stream);
+        h->evused += 3;
+        h->prof_bytes.push_back((Lv.vanka_res_bytes + Lv.vanka_apply_bytes) * n);
+        h->prof_bytes.push_back(0.0);
+      }
+    }
+  }
+  PM_LAUNCH(launch_patch_end<T>(L, u, rhs, Lv.hb, Lv.np, sweeps & 1, h->stream));
+  return PM_OK;
+}
+
+template <typename T>
 pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
   const T damp = (T)h->opt.smooth_damp;
   const bool relax = std::fabs(1.0 - h->opt.alpha) > 1e-3;
@@ -366,6 +450,12 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
       cudaMemcpyAsync(Lv.uold, u, sizeof(T) * Lv.ndof, cudaMemcpyDeviceToDevice, h->stream) !=
           cudaSuccess)
     return cuda_fail(h, "uold copy");
+  if (Lv.packed()) {  // only with relaxation: smooth() runs the others together
+    PM_TRY(patch_sweeps<T>(h, Lv, u, rhs, 1));
+    if (relax) PM_LAUNCH(launch_relax<T>(u, static_cast<const T *>(Lv.uold), (T)h->opt.alpha, Lv.ndof, h->stream));
+    PM_LAUNCH(launch_dirichlet<T>(u, rhs, Lv.nu, Lv.hb, Lv.ndir, h->stream));
+    return PM_OK;
+  }
   const DevOp<T> op = Lv.op<T>();
   const DevCells cells = Lv.cells();
   const int ncol = (int)Lv.colouring.ptr.size() - 1;
@@ -433,6 +523,14 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
   if (aos) PM_LAUNCH(launch_unpack_velocity(Lv.ux, uf, Lv.nu, h->stream));
   if (relax) PM_LAUNCH(launch_relax<T>(u, static_cast<const T *>(Lv.uold), (T)h->opt.alpha, Lv.ndof, h->stream));
   PM_LAUNCH(launch_dirichlet<T>(u, rhs, Lv.nu, Lv.hb, Lv.ndir, h->stream));
+  return PM_OK;
+}
+
+template <typename T>
+pm_status smooth(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps) {
+  if (sweeps > 0 && Lv.packed() && std::fabs(1.0 - h->opt.alpha) <= 1e-3)
+    return patch_sweeps<T>(h, Lv, u, rhs, sweeps);
+  for (int s = 0; s < sweeps; ++s) PM_TRY(vanka_sweep<T>(h, Lv, u, rhs));
   return PM_OK;
 }
 
@@ -523,7 +621,7 @@ pm_status cycle(pm_handle *h, int i) {
   LevelDev &K = h->L[i - 1];
   T *d = static_cast<T *>(C.def);
   T *cu = static_cast<T *>(K.sol), *cf = static_cast<T *>(K.rhs);
-  for (int s = 0; s < h->opt.pre_smooth; ++s) PM_TRY(vanka_sweep<T>(h, C, u, f));
+  PM_TRY(smooth<T>(h, C, u, f, h->opt.pre_smooth));
   PM_LAUNCH(launch_dirichlet<T>(u, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
   PM_TRY(level_defect<T>(h, C, u, f, d));
   // DefectRestriction (u and p) + CorrectDefect + Reset
@@ -539,7 +637,7 @@ pm_status cycle(pm_handle *h, int i) {
   PM_LAUNCH(launch_dirichlet<T>(d, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
   PM_LAUNCH(launch_axpy<T>(u, (T)h->opt.beta, d, C.ndof, h->stream));
   PM_LAUNCH(launch_dirichlet<T>(u, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
-  for (int s = 0; s < h->opt.post_smooth; ++s) PM_TRY(vanka_sweep<T>(h, C, u, f));
+  PM_TRY(smooth<T>(h, C, u, f, h->opt.post_smooth));
   if (h->l_active &&
       (h->opt.learned_levels <= 0 || i >= (int)h->L.size() - h->opt.learned_levels))
     PM_TRY(learned_step<T>(h, C, u, f));
@@ -557,12 +655,141 @@ pm_status vcycle_core(pm_handle *h) {
   return cycle<T>(h, (int)h->L.size() - 1);
 }
 
+void drop_patch(pm_handle *h, LevelDev &Lv) {
+  for (const auto &m : Lv.patch_arrays(mixed(h) ? sizeof(float) : sizeof(double))) {
+    if (!m.p) continue;
+    h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), m.p));
+    h->patch_bytes -= m.bytes;
+    cudaFree(m.p);
+  }
+  Lv.pk_ids = Lv.pk_pattern = nullptr;
+  Lv.pk_flips = nullptr;
+  Lv.pk_patterns = Lv.pk_values = Lv.pk_u = Lv.pk_p = nullptr;
+  Lv.pk = -1;
+}
+
 void drop_graphs(pm_handle *h) {
   for (int k = 0; k < 2; ++k)
     if (h->vgraph_g[k]) {
       cudaGraphExecDestroy(h->vgraph_g[k]);
       h->vgraph_g[k] = nullptr;
     }
+}
+
+bool release_patches(pm_handle *h) {
+  bool any = false;
+  for (LevelDev &Lv : h->L) {
+    if (Lv.pk_values) any = true;
+  }
+  if (!any) return false;
+  cudaStreamSynchronize(h->stream);
+  drop_graphs(h);  // they launch the packed sweeps
+  for (LevelDev &Lv : h->L) drop_patch(h, Lv);
+  return true;
+}
+
+// Packed rows of one level: patch lists on the host, patterns and values on
+// the device.  *fits: the mesh and the CSR pattern have the layout's shape.
+template <typename T>
+pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
+  *fits = false;
+  std::vector<int> ids;
+  std::vector<unsigned char> flips;
+  if (!build_patches(Lv.ncells, Lv.h_udofs.data(), Lv.h_pdofs.data(), Lv.nu, Lv.np, Lv.colouring,
+                     ids, flips))
+    return PM_OK;
+  const size_t nc = (size_t)Lv.ncells;
+  unsigned char *val = nullptr, *u = nullptr, *p = nullptr, *pat = nullptr;
+  PM_TRY(upload(h, &Lv.pk_ids, ids.data(), ids.size()));
+  PM_TRY(upload(h, &Lv.pk_flips, flips.data(), flips.size()));
+  PM_TRY(dalloc(h, &Lv.pk_pattern, nc));
+  PM_TRY(dalloc(h, &u, (size_t)Lv.nu * 8 * sizeof(T)));
+  Lv.pk_u = u;
+  PM_TRY(dalloc(h, &p, (size_t)Lv.np * sizeof(T)));
+  Lv.pk_p = p;
+  PM_TRY(dalloc(h, &val, nc * kPatchValues * sizeof(T)));
+  Lv.pk_values = val;
+  // one pattern per hash value; the values array is the scratch of this step
+  unsigned long long *d_hash = reinterpret_cast<unsigned long long *>(val);
+  int *d_which = reinterpret_cast<int *>(d_hash + nc);
+  int *bad_d = h->status_d + 2, bad = 0;
+  const DevOp<T> op = Lv.op<T>();
+  auto check = [&]() -> pm_status {
+    if (cudaMemcpyAsync(&bad, bad_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream) !=
+        cudaSuccess)
+      return cuda_fail(h, "patch flag");
+    return sync(h, "patch check");
+  };
+  if (cudaMemsetAsync(bad_d, 0, sizeof(int), h->stream) != cudaSuccess)
+    return cuda_fail(h, "patch flag");
+  PM_LAUNCH(launch_patch_pattern<T>(0, Lv.pk_ids, op, Lv.ncells, nullptr, nullptr, nullptr, d_hash,
+                                    bad_d, h->stream));
+  std::vector<unsigned long long> hash(nc);
+  if (cudaMemcpyAsync(hash.data(), d_hash, nc * sizeof(hash[0]), cudaMemcpyDeviceToHost,
+                      h->stream) != cudaSuccess)
+    return cuda_fail(h, "patch hashes");
+  PM_TRY(check());
+  if (bad) return PM_OK;
+  std::unordered_map<unsigned long long, int> seen;
+  std::vector<int> which, pattern(nc);
+  for (size_t c = 0; c < nc; ++c) {
+    const auto it = seen.emplace(hash[c], (int)which.size());
+    if (it.second) which.push_back((int)c);
+    pattern[c] = it.first->second;
+  }
+  PM_TRY(dalloc(h, &pat, which.size() * kPatchPatternBytes));
+  Lv.pk_patterns = pat;
+  Lv.pk_npat = (long long)which.size();
+  if (cudaMemcpyAsync(d_which, which.data(), which.size() * sizeof(int), cudaMemcpyHostToDevice,
+                      h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(Lv.pk_pattern, pattern.data(), nc * sizeof(int), cudaMemcpyHostToDevice,
+                      h->stream) != cudaSuccess)
+    return cuda_fail(h, "patch patterns");
+  PM_LAUNCH(launch_patch_pattern<T>(1, Lv.pk_ids, op, (int)which.size(), d_which, pat, nullptr,
+                                    nullptr, bad_d, h->stream));
+  PM_LAUNCH(launch_patch_pattern<T>(2, Lv.pk_ids, op, Lv.ncells, nullptr, pat, Lv.pk_pattern,
+                                    nullptr, bad_d, h->stream));
+  PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), op, Lv.ncells, h->stream));
+  PM_TRY(check());
+  *fits = bad == 0;
+  return PM_OK;
+}
+
+// Packed rows of every level that can run from them: built once per level,
+// packed again when the matrix values are newer.  A level whose mesh does not
+// have the shape, or for which there is no memory, keeps the CSR kernels.
+template <typename T>
+pm_status ensure_patches(pm_handle *h) {
+  if (h->opt.residual_variant != 0) return PM_OK;  // a CSR kernel is asked for
+  for (size_t l = 1; l < h->L.size(); ++l) {
+    LevelDev &Lv = h->L[l];
+    if (Lv.pk < 0 || !Lv.schur() || Lv.ncells == 0 || (Lv.pk == 1 && !Lv.pk_stale)) continue;
+    if (Lv.pk == 1) {
+      PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), Lv.op<T>(), Lv.ncells, h->stream));
+      Lv.pk_stale = false;
+      continue;
+    }
+    const std::string err = h->err;
+    bool fits = false;
+    h->patch_alloc = true;
+    const pm_status st = build_patch<T>(h, Lv, &fits);
+    h->patch_alloc = false;
+    if (st != PM_OK && st != PM_OOM) return st;
+    if (st == PM_OOM || !fits) {
+      cudaStreamSynchronize(h->stream);
+      drop_patch(h, Lv);
+      h->err = err;
+      continue;
+    }
+    Lv.pk = 1;
+    Lv.pk_stale = false;
+    drop_graphs(h);
+  }
+  return PM_OK;
+}
+
+pm_status ensure_patches(pm_handle *h) {
+  return mixed(h) ? ensure_patches<float>(h) : ensure_patches<double>(h);
 }
 
 // One V-cycle; with a network attached and enabled the cycle includes the
@@ -603,6 +830,7 @@ pm_status run_vcycle_core(pm_handle *h) {
 // z = M v (FP64 in/out)
 pm_status precondition(pm_handle *h, double *z, const double *v) {
   LevelDev &F = h->L.back();
+  PM_TRY(ensure_patches(h));
   if (mixed(h))
     PM_LAUNCH((launch_convert<float, double>(static_cast<float *>(F.rhs), v, F.ndof, h->stream)));
   else if (cudaMemcpyAsync(F.rhs, v, sizeof(double) * F.ndof, cudaMemcpyDeviceToDevice,
@@ -1234,6 +1462,7 @@ pm_status factor_all(pm_handle *h) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, h->stream);
+  PM_TRY(ensure_patches(h));
   for (size_t l = 1; l < h->L.size(); ++l) {
     LevelDev &Lv = h->L[l];
     // block elimination in FP32 unless factor_fp32 = 0 (mixed only); the
@@ -1308,6 +1537,7 @@ int desc_blocks(const pm_level_desc *d) {
 }
 
 pm_status upload_values(pm_handle *h, LevelDev &Lv, const pm_level_desc *d, bool first) {
+  Lv.pk_stale = true;
   const int nblk = desc_blocks(d);
   if (nblk == 0) return fail(h, PM_BADARG, "A blocks: give all nine or only a[0]");
   if (first) Lv.structured = nblk == 1;
@@ -1767,6 +1997,7 @@ pm_status pm_setup(pm_handle *h) {
   PM_TRY(dalloc(h, &h->w, N));
   PM_TRY(dalloc(h, &h->xd, N));
   PM_TRY(dalloc(h, &h->bd, N));
+  PM_TRY(ensure_patches(h));
   PM_TRY(factor_all(h));
   for (size_t l = 1; l < h->L.size(); ++l) {
     if (mixed(h))
@@ -1939,16 +2170,17 @@ pm_status pm_cell_vanka(pm_handle *h, int level, double *u, const double *rhs, i
   PM_CHECK_LEVEL(h, level);
   if (level == 0) return fail(h, PM_BADARG, "the coarsest level is solved exactly");
   LevelDev &Lv = h->L[level];
+  PM_TRY(ensure_patches(h));
   PM_TRY(h2d(h, Lv.x64, u, Lv.ndof));
   PM_TRY(h2d(h, Lv.y64, rhs, Lv.ndof));
   if (mixed(h)) {
     float *uu = static_cast<float *>(Lv.sol), *ff = static_cast<float *>(Lv.rhs);
     PM_LAUNCH((launch_convert<float, double>(uu, Lv.x64, Lv.ndof, h->stream)));
     PM_LAUNCH((launch_convert<float, double>(ff, Lv.y64, Lv.ndof, h->stream)));
-    for (int s = 0; s < sweeps; ++s) PM_TRY(vanka_sweep<float>(h, Lv, uu, ff));
+    PM_TRY(smooth<float>(h, Lv, uu, ff, sweeps));
     PM_LAUNCH((launch_convert<double, float>(Lv.x64, uu, Lv.ndof, h->stream)));
   } else {
-    for (int s = 0; s < sweeps; ++s) PM_TRY(vanka_sweep<double>(h, Lv, Lv.x64, Lv.y64));
+    PM_TRY(smooth<double>(h, Lv, Lv.x64, Lv.y64, sweeps));
   }
   const pm_status st = d2h(h, u, Lv.x64, Lv.ndof);
   collect_profile(h);
@@ -2158,6 +2390,7 @@ static pm_status assemble_impl(pm_handle *h, int level, const double *d_cell_h,
   op.bt_scale = bt_scale;
   if (!sys) op.Aonly = op.Monly = nullptr;
   Lv.asm_theta = false;
+  Lv.pk_stale = true;
   PM_LAUNCH(launch_assemble_level(op, Lv.cells(), Lv.colour_cells, Lv.colouring.ptr.data(),
                                   (int)Lv.colouring.ptr.size() - 1, d_cell_h, d_conv, nu,
                                   h->stream));

@@ -196,6 +196,56 @@ constexpr int kSchurOffW = Schur<1>::offW;
 constexpr int kSchurOffS = Schur<1>::offS;
 constexpr int kSchurValues = Schur<1>::values;
 constexpr int kSchurStride = Schur<1>::stride;
+// ---- sweeps of one-block hexahedral levels from packed rows (pm_vanka_patch.cu)
+constexpr int kPatchNodes = 343;  // nodes of a cell and its 26 neighbours
+// Ints per cell: the patch's nodes in ascending order (node << 2 | changes
+// side per sweep << 1 | current copy; repeated to fill the list), their
+// count, the cell's own nodes (the same entries in local order), the mask of
+// own nodes that lie in this cell alone, and the first pressure DOF of the
+// cell and its 26 neighbours.
+constexpr int kPatchCount = 343, kPatchOwn = 344, kPatchSingle = 371, kPatchBase = 372;
+constexpr int kPatchIds = 400;
+constexpr int kPatchValues = 3904;  // A and BT entries of a cell, with 5.6 % of padding
+constexpr int kPatchPatternBytes = 8256;
+struct PatchPattern;
+template <typename T>
+struct PatchLevel {
+  int nu;
+  const PatchPattern *patterns;
+  const int *pattern;      // pattern of each cell
+  const int *ids;          // ncells x kPatchIds
+  const uint8_t *flips;    // per node: 1 when it changes copies from sweep to sweep
+  const T *values;         // ncells x kPatchValues
+  T *values_w;             // the same array, for the packing kernel
+  void *u;                 // two copies of the velocity, 4 values per node
+  T *p;
+};
+// the level's CSR values into the packed layout
+template <typename T>
+int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cudaStream_t s);
+// patterns of a level's cells: mode 0 hashes (n = ncells), 1 the patterns of
+// the cells which[0..n), 2 compare each cell (n = ncells) with its pattern;
+// *bad |= 1 when a row does not fit or a pattern differs
+template <typename T>
+int launch_patch_pattern(int mode, const int *ids, const DevOp<T> &op, int n, const int *which,
+                         void *patterns, const int *pattern, unsigned long long *hash, int *bad,
+                         cudaStream_t s);
+// a run of sweeps: begin (u into the copies), every colour of every sweep,
+// between two sweeps the Dirichlet nodes, end (the copies into u).  odd: the
+// sweep's number & 1; for end the number of sweeps & 1.  Every launch but the
+// first may start early and waits for its predecessor on the device.
+template <typename T>
+int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb, int np,
+                       cudaStream_t s);
+template <typename T>
+int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors,
+                        const T *rhs, T damp, int odd, cudaStream_t s);
+template <typename T>
+int launch_patch_between(const PatchLevel<T> &L, const T *rhs, int hb, cudaStream_t s);
+template <typename T>
+int launch_patch_end(const PatchLevel<T> &L, T *u, const T *rhs, int hb, int np, int odd,
+                     cudaStream_t s);
+
 // fp32: eliminate in FP32 (TF = float only; option factor_fp32), else FP64
 template <typename TF>
 int launch_schur_factor(const DevOp<double> &op, const DevCells &cells, TF *factors, int *status,

@@ -380,16 +380,23 @@ __global__ void __launch_bounds__(kApplyWarps * 32) k_schur_apply(
 // compared as values; a NaN counts as different)
 __global__ void __launch_bounds__(256) k_block_structure(DevOp<double> op, long long n,
                                                          int *flag) {
-  bool nz = false, differ = false;
+  // every value is loaded and compared without short-circuit branches: the
+  // version with || left whole levels of fully coupled blocks unflagged
+  unsigned bits = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    nz |= op.a[1][i] != 0.0 || op.a[2][i] != 0.0 || op.a[3][i] != 0.0 || op.a[5][i] != 0.0 ||
-          op.a[6][i] != 0.0 || op.a[7][i] != 0.0;
-    const double d = op.a[0][i];
-    differ |= !(op.a[4][i] == d) || !(op.a[8][i] == d);
+    double v[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = op.a[k][i];
+    unsigned nz = 0;
+#pragma unroll
+    for (int k = 1; k < 8; ++k)
+      if (k != 4) nz |= (unsigned)(v[k] != 0.0);
+    const unsigned differ = (unsigned)!(v[4] == v[0]) | (unsigned)!(v[8] == v[0]);
+    bits |= nz | (differ << 1);
   }
-  const int bits = (__any_sync(kFull, nz) ? 1 : 0) | (__any_sync(kFull, differ) ? 2 : 0);
-  if (bits && (threadIdx.x & 31) == 0) atomicOr(flag, bits);
+  bits = __reduce_or_sync(kFull, bits);
+  if (bits && (threadIdx.x & 31) == 0) atomicOr(flag, (int)bits);
 }
 
 inline int ok() { return cudaPeekAtLastError() == cudaSuccess ? 1 : -1; }
