@@ -35,7 +35,8 @@ GPU_CU = ["pm_api.cu", "pm_sparse.cu", "pm_vanka.cu", "pm_vanka_schur.cu", "pm_v
 GPU_CPP = ["pm_setup_host.cpp"]
 HOST_CPP = ["oseen_problem.cpp", "oseen_tet.cpp"]
 HEADERS = [INCLUDE / "pmgpu.h", CSRC / "pm_kernels.h", CSRC / "pm_setup_host.h",
-           CSRC / "oseen_problem.h", CSRC / "oseen_internal.h", CSRC / "pm_learned.h"]
+           CSRC / "oseen_problem.h", CSRC / "oseen_internal.h", CSRC / "pm_learned.h",
+           CSRC / "pm_bulk.cuh"]
 
 
 def nvcc_path() -> str:

@@ -93,7 +93,7 @@ struct LevelDev {
   // looked at yet, 1 in use, -1 not available (mesh shape, memory)
   int pk = 0;
   bool pk_stale = true;  // matrix values newer than the packed copy
-  int *pk_ids = nullptr, *pk_pattern = nullptr;
+  int *pk_ids = nullptr;
   uint8_t *pk_flips = nullptr;
   void *pk_patterns = nullptr, *pk_values = nullptr, *pk_u = nullptr, *pk_p = nullptr;
   long long pk_npat = 0;
@@ -104,12 +104,11 @@ struct LevelDev {
   };
   std::vector<PatchArray> patch_arrays(long long es) const {
     return {{pk_ids, (long long)ncells * kPatchIds * 4},
-            {pk_pattern, (long long)ncells * 4},
             {pk_flips, nu},
             {pk_patterns, pk_npat * kPatchPatternBytes},
             {pk_values, (long long)ncells * kPatchValues * es},
-            {pk_u, (long long)nu * 8 * es},
-            {pk_p, (long long)np * es}};
+            {pk_u, (long long)nu * 12 * es},
+            {pk_p, (long long)np * 2 * es}};
   }
   double *x64 = nullptr, *y64 = nullptr, *z64 = nullptr;
   // unique bytes of one Vanka sweep per cell, split by kernel (see pm_setup)
@@ -402,12 +401,13 @@ PatchLevel<T> patch_level(const pm_handle *h, const LevelDev &Lv) {
   PatchLevel<T> L;
   L.nu = Lv.nu;
   L.patterns = static_cast<const PatchPattern *>(Lv.pk_patterns);
-  L.pattern = Lv.pk_pattern;
   L.ids = Lv.pk_ids;
   L.flips = Lv.pk_flips;
   L.values = L.values_w = static_cast<T *>(Lv.pk_values);
   L.u = Lv.pk_u;
   L.p = static_cast<T *>(Lv.pk_p);
+  L.f = static_cast<T *>(Lv.pk_u) + (size_t)8 * Lv.nu;
+  L.fp = L.p + Lv.np;
   return L;
 }
 
@@ -426,8 +426,8 @@ pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweep
       const bool prof = h->prof && h->evused + 3 <= h->evpool.size();
       if (prof) cudaEventRecord(h->evpool[h->evused], h->stream);
       PM_LAUNCH(launch_patch_colour<T>(L, Lv.colour_cells + b, n,
-                                       static_cast<const T *>(Lv.factors), rhs,
-                                       (T)h->opt.smooth_damp, s & 1, h->stream));
+                                       static_cast<const T *>(Lv.factors), (T)h->opt.smooth_damp,
+                                       s & 1, h->sweep_err, h->num_sms, h->stream));
       if (prof) {  // residual and local solve are one launch: all of it is kernel 0
         cudaEventRecord(h->evpool[h->evused + 1], h->stream);
         cudaEventRecord(h->evpool[h->evused + 2], h->stream);
@@ -662,7 +662,7 @@ void drop_patch(pm_handle *h, LevelDev &Lv) {
     h->patch_bytes -= m.bytes;
     cudaFree(m.p);
   }
-  Lv.pk_ids = Lv.pk_pattern = nullptr;
+  Lv.pk_ids = nullptr;
   Lv.pk_flips = nullptr;
   Lv.pk_patterns = Lv.pk_values = Lv.pk_u = Lv.pk_p = nullptr;
   Lv.pk = -1;
@@ -699,19 +699,19 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
                      ids, flips))
     return PM_OK;
   const size_t nc = (size_t)Lv.ncells;
+  if (launch_patch_init() < 0) return cuda_fail(h, "packed sweeps");
   unsigned char *val = nullptr, *u = nullptr, *p = nullptr, *pat = nullptr;
   PM_TRY(upload(h, &Lv.pk_ids, ids.data(), ids.size()));
   PM_TRY(upload(h, &Lv.pk_flips, flips.data(), flips.size()));
-  PM_TRY(dalloc(h, &Lv.pk_pattern, nc));
-  PM_TRY(dalloc(h, &u, (size_t)Lv.nu * 8 * sizeof(T)));
+  PM_TRY(dalloc(h, &u, (size_t)Lv.nu * 12 * sizeof(T)));
   Lv.pk_u = u;
-  PM_TRY(dalloc(h, &p, (size_t)Lv.np * sizeof(T)));
+  PM_TRY(dalloc(h, &p, (size_t)Lv.np * 2 * sizeof(T)));
   Lv.pk_p = p;
   PM_TRY(dalloc(h, &val, nc * kPatchValues * sizeof(T)));
   Lv.pk_values = val;
   // one pattern per hash value; the values array is the scratch of this step
   unsigned long long *d_hash = reinterpret_cast<unsigned long long *>(val);
-  int *d_which = reinterpret_cast<int *>(d_hash + nc);
+  int *d_which = reinterpret_cast<int *>(d_hash + nc), *d_pattern = d_which + nc;
   int *bad_d = h->status_d + 2, bad = 0;
   const DevOp<T> op = Lv.op<T>();
   auto check = [&]() -> pm_status {
@@ -722,8 +722,8 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   };
   if (cudaMemsetAsync(bad_d, 0, sizeof(int), h->stream) != cudaSuccess)
     return cuda_fail(h, "patch flag");
-  PM_LAUNCH(launch_patch_pattern<T>(0, Lv.pk_ids, op, Lv.ncells, nullptr, nullptr, nullptr, d_hash,
-                                    bad_d, h->stream));
+  PM_LAUNCH(launch_patch_pattern<T>(0, Lv.pk_ids, op, Lv.ncells, nullptr, nullptr, d_hash, bad_d,
+                                    h->stream));
   std::vector<unsigned long long> hash(nc);
   if (cudaMemcpyAsync(hash.data(), d_hash, nc * sizeof(hash[0]), cudaMemcpyDeviceToHost,
                       h->stream) != cudaSuccess)
@@ -742,16 +742,32 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   Lv.pk_npat = (long long)which.size();
   if (cudaMemcpyAsync(d_which, which.data(), which.size() * sizeof(int), cudaMemcpyHostToDevice,
                       h->stream) != cudaSuccess ||
-      cudaMemcpyAsync(Lv.pk_pattern, pattern.data(), nc * sizeof(int), cudaMemcpyHostToDevice,
+      cudaMemcpyAsync(d_pattern, pattern.data(), nc * sizeof(int), cudaMemcpyHostToDevice,
                       h->stream) != cudaSuccess)
     return cuda_fail(h, "patch patterns");
+  PM_LAUNCH(launch_patch_assign(Lv.pk_ids, d_pattern, Lv.ncells, h->stream));
   PM_LAUNCH(launch_patch_pattern<T>(1, Lv.pk_ids, op, (int)which.size(), d_which, pat, nullptr,
-                                    nullptr, bad_d, h->stream));
-  PM_LAUNCH(launch_patch_pattern<T>(2, Lv.pk_ids, op, Lv.ncells, nullptr, pat, Lv.pk_pattern,
-                                    nullptr, bad_d, h->stream));
-  PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), op, Lv.ncells, h->stream));
+                                    bad_d, h->stream));
+  PM_LAUNCH(launch_patch_pattern<T>(2, Lv.pk_ids, op, Lv.ncells, nullptr, pat, nullptr, bad_d,
+                                    h->stream));
   PM_TRY(check());
-  *fits = bad == 0;
+  if (bad) return PM_OK;
+  // places of the nodes in shared memory; a level whose cells hardly share
+  // patterns keeps the list order
+  if (Lv.pk_npat <= 4096) {
+    std::vector<unsigned char> host((size_t)Lv.pk_npat * kPatchPatternBytes);
+    if (cudaMemcpyAsync(host.data(), pat, host.size(), cudaMemcpyDeviceToHost, h->stream) !=
+        cudaSuccess)
+      return cuda_fail(h, "patch patterns");
+    PM_TRY(sync(h, "patch patterns"));
+    patch_places(host.data(), Lv.pk_npat);
+    if (cudaMemcpyAsync(pat, host.data(), host.size(), cudaMemcpyHostToDevice, h->stream) !=
+        cudaSuccess)
+      return cuda_fail(h, "patch patterns");
+    PM_TRY(sync(h, "patch patterns"));
+  }
+  PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), op, Lv.ncells, h->stream));
+  *fits = true;
   return PM_OK;
 }
 

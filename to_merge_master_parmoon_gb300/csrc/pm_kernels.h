@@ -201,24 +201,26 @@ constexpr int kPatchNodes = 343;  // nodes of a cell and its 26 neighbours
 // Ints per cell: the patch's nodes in ascending order (node << 2 | changes
 // side per sweep << 1 | current copy; repeated to fill the list), their
 // count, the cell's own nodes (the same entries in local order), the mask of
-// own nodes that lie in this cell alone, and the first pressure DOF of the
-// cell and its 26 neighbours.
-constexpr int kPatchCount = 343, kPatchOwn = 344, kPatchSingle = 371, kPatchBase = 372;
+// own nodes that lie in this cell alone, the first pressure DOF of the cell
+// and its 26 neighbours, and the cell's pattern.
+constexpr int kPatchCount = 343, kPatchOwn = 344, kPatchSingle = 371, kPatchBase = 372,
+              kPatchPattern = 399;
 constexpr int kPatchIds = 400;
 constexpr int kPatchValues = 3904;  // A and BT entries of a cell, with 5.6 % of padding
-constexpr int kPatchPatternBytes = 8256;
+constexpr int kPatchPatternBytes = 8960;
 struct PatchPattern;
 template <typename T>
 struct PatchLevel {
   int nu;
   const PatchPattern *patterns;
-  const int *pattern;      // pattern of each cell
   const int *ids;          // ncells x kPatchIds
   const uint8_t *flips;    // per node: 1 when it changes copies from sweep to sweep
   const T *values;         // ncells x kPatchValues
   T *values_w;             // the same array, for the packing kernel
   void *u;                 // two copies of the velocity, 4 values per node
   T *p;
+  void *f;                 // right-hand side, 4 values per node
+  T *fp;                   // and its pressure part
 };
 // the level's CSR values into the packed layout
 template <typename T>
@@ -228,8 +230,10 @@ int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cu
 // *bad |= 1 when a row does not fit or a pattern differs
 template <typename T>
 int launch_patch_pattern(int mode, const int *ids, const DevOp<T> &op, int n, const int *which,
-                         void *patterns, const int *pattern, unsigned long long *hash, int *bad,
-                         cudaStream_t s);
+                         void *patterns, unsigned long long *hash, int *bad, cudaStream_t s);
+int launch_patch_assign(int *ids, const int *pattern, int ncells, cudaStream_t s);
+void patch_places(void *host_patterns, long long count);
+int launch_patch_init();  // shared-memory limit of the sweep kernels
 // a run of sweeps: begin (u into the copies), every colour of every sweep,
 // between two sweeps the Dirichlet nodes, end (the copies into u).  odd: the
 // sweep's number & 1; for end the number of sweeps & 1.  Every launch but the
@@ -239,7 +243,7 @@ int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb,
                        cudaStream_t s);
 template <typename T>
 int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors,
-                        const T *rhs, T damp, int odd, cudaStream_t s);
+                        T damp, int odd, int *err, int num_sms, cudaStream_t s);
 template <typename T>
 int launch_patch_between(const PatchLevel<T> &L, const T *rhs, int hb, cudaStream_t s);
 template <typename T>

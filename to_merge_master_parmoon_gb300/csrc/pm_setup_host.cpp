@@ -493,7 +493,7 @@ bool build_patches(int ncells, const int *udofs, const int *pdofs, int nu, int n
                    std::vector<unsigned char> &flips) {
   constexpr int NB = 26, NODES = 343, COUNT = 343, OWN = 344, SINGLE = 371, BASE = 372;
   constexpr int stride = kPatchIdsHost;
-  if (nu >= (1 << 29)) return false;
+  if (nu >= (1 << 29) || np % 4) return false;
   std::vector<unsigned char> seen((size_t)np, 0);
   for (int c = 0; c < ncells; ++c) {
     const int *p = pdofs + (size_t)c * 4;

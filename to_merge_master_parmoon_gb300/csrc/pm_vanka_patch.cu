@@ -24,10 +24,13 @@
 // entries; a butterfly over the lanes), and the block solve in the order of
 // k_schur_apply, so FP32 sweeps are equal to theirs bit for bit.
 //
-// Patch.  Each cell keeps the sorted list of its patch's nodes; where entry j
-// of row r finds its node in that list is a pattern of 16-bit positions that
-// cells with the same neighbourhood and numbering order share (one for all
-// inner cells of a uniform mesh).  Meshes whose cells have more than one
+// Patch.  Each cell keeps the sorted list of its patch's nodes; where the
+// nodes lie in shared memory and where entry j of row r finds its node is a
+// pattern that cells with the same neighbourhood and numbering order share
+// (one for all inner cells of a uniform mesh).  The places are chosen at
+// set-up (patch_places) so that the eight lanes of a row read eight different
+// 16-byte bank groups: in list order a row's runs of five nodes collided
+// pairwise.  Meshes whose cells have more than one
 // neighbour beyond a face, edge or vertex, or whose rows do not fit the lanes
 // (128 / 80 / 48 columns on vertex / edge / other rows) keep the CSR kernels.
 //
@@ -42,8 +45,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdint>
+#include <vector>
 
+#include "pm_bulk.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -51,7 +57,7 @@ namespace pm {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kPatchThreads = 256;  // warps 0-1 vertex rows, 2-4 edges, 5-6 the rest, 7 pressure
+constexpr int kPatchThreads = 256;  // warps 0-1 vertex rows, 2-4 edges, 5-6 the rest, 7 block solve
 constexpr int kRowLanes = 224;
 constexpr int kZeroSlot = kPatchNodes;  // a node that is zero: padding entries point to it
 constexpr int kZeroP = 27 * NP_LOC;
@@ -87,10 +93,11 @@ __device__ __forceinline__ int bt_pos(int li, int q, int c) {
 
 // Where the entries of a cell's rows find their nodes, pressures and B values.
 struct PatchPattern {
-  uint16_t slot[kRowLanes][16];  // A entry: position in the patch list
+  uint16_t slot[kRowLanes][16];  // A entry: 16 x place of its node in shared memory
   uint8_t bt[kRowLanes][4];      // BT entry: 4 * neighbour + mode
   uint8_t bj[32][4];             // B row lane / 8, entry lane % 8 + 8 q: own node
-  uint16_t own[32];              // own node: position in the patch list
+  uint16_t own[32];              // own node: 16 x its place
+  uint16_t place[kPatchIds - 48];  // patch list entry: its place
 };
 static_assert(sizeof(PatchPattern) == kPatchPatternBytes, "pattern size");
 
@@ -110,9 +117,6 @@ struct Node<float> {
   __device__ __forceinline__ void store(void *p, size_t i) const {
     reinterpret_cast<float4 *>(p)[i] = v;
   }
-  static __device__ __forceinline__ float *component(void *p, size_t i) {
-    return reinterpret_cast<float *>(p) + 4 * i;
-  }
 };
 template <>
 struct Node<double> {
@@ -125,9 +129,6 @@ struct Node<double> {
     double2 *q = reinterpret_cast<double2 *>(p) + 2 * i;
     q[0] = a;
     q[1] = b;
-  }
-  static __device__ __forceinline__ double *component(void *p, size_t i) {
-    return reinterpret_cast<double *>(p) + 4 * i;
   }
 };
 __device__ __forceinline__ Node<float> make_node(float x, float y, float z) {
@@ -159,8 +160,14 @@ struct Tri<float, N> {
     y = q.y;
     z = q.z;
   }
-  __device__ __forceinline__ float get(int i, int c) const {
-    return reinterpret_cast<const float *>(v)[4 * i + c];
+  __device__ __forceinline__ void at(unsigned off, float &x, float &y, float &z) const {
+    const float4 q = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(v) + off);
+    x = q.x;
+    y = q.y;
+    z = q.z;
+  }
+  __device__ __forceinline__ float &ref(int i, int c) {
+    return reinterpret_cast<float *>(v)[4 * i + c];
   }
   __device__ __forceinline__ void set(int i, float x, float y, float z) {
     v[i] = make_float4(x, y, z, 0.f);
@@ -176,8 +183,14 @@ struct Tri<double, N> {
     y = q.y;
     z = w[i];
   }
-  __device__ __forceinline__ double get(int i, int c) const {
-    return c < 2 ? reinterpret_cast<const double *>(v)[2 * i + c] : w[i];
+  __device__ __forceinline__ void at(unsigned off, double &x, double &y, double &z) const {
+    const double2 q = *reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(v) + off);
+    x = q.x;
+    y = q.y;
+    z = *reinterpret_cast<const double *>(reinterpret_cast<const char *>(w) + (off >> 1));
+  }
+  __device__ __forceinline__ double &ref(int i, int c) {
+    return c < 2 ? reinterpret_cast<double *>(v)[2 * i + c] : w[i];
   }
   __device__ __forceinline__ void set(int i, double x, double y, double z) {
     v[i] = make_double2(x, y);
@@ -185,38 +198,20 @@ struct Tri<double, N> {
   }
 };
 
-// four (two) consecutive values, read once
-__device__ __forceinline__ void ld4(const float *p, float &x, float &y, float &z, float &w) {
-  const float4 v = __ldcs(reinterpret_cast<const float4 *>(p));
-  x = v.x;
-  y = v.y;
-  z = v.z;
-  w = v.w;
-}
-__device__ __forceinline__ void ld4(const double *p, double &x, double &y, double &z, double &w) {
-  const double2 a = __ldcs(reinterpret_cast<const double2 *>(p)),
-                b = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
-  x = a.x;
-  y = a.y;
-  z = b.x;
-  w = b.y;
-}
-__device__ __forceinline__ void ld2(const float *p, float &x, float &y) {
-  const float2 v = __ldcs(reinterpret_cast<const float2 *>(p));
-  x = v.x;
-  y = v.y;
-}
-__device__ __forceinline__ void ld2(const double *p, double &x, double &y) {
-  const double2 v = __ldcs(reinterpret_cast<const double2 *>(p));
-  x = v.x;
-  y = v.y;
-}
-
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   return v;
+}
+
+// named barriers of a CTA
+enum { kBarRows = 1, kBarFull = 2, kBarFree = 4 };  // kBarFull, kBarFree: two each
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 // the previous kernel of the stream has finished and its writes are visible
@@ -228,235 +223,667 @@ __device__ __forceinline__ void start_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// a0 b0 + a1 b1 + a2 b2, contracted in FP32 as the compiler does in
+// k_schur_apply and in the pressure rows of the row-group kernel
 template <typename T>
-struct PatchSmem {
-  Tri<T, kPatchNodes + 1> u;
-  __align__(16) T r[3][28];  // local residual by component
-  T p[28][NP_LOC];           // pressures of the cell and its neighbours, then zeros
-  T y[3][32];
-  T rp[NP_LOC], t[NP_LOC];
-};
+__device__ __forceinline__ T dot3(T a0, T b0, T a1, T b1, T a2, T b2) {
+  if constexpr (sizeof(T) == 4)
+    return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+  else
+    return a0 * b0 + a1 * b1 + a2 * b2;
+}
 
-// FP32: bound by the packed values from HBM on large levels, by the chain
-// gather -> sums -> solve -> update on small ones.  FP64: by the FP64 pipe.
 template <typename T>
-__global__ void __launch_bounds__(kPatchThreads, sizeof(T) == 4 ? 3 : 2) k_patch_sweep(
-    PatchLevel<T> L, const int *__restrict__ list, const T *__restrict__ factors,
-    const T *__restrict__ rhs, T damp, int odd) {
-  using S1 = Schur<1>;
-  __shared__ PatchSmem<T> sm;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, sub = lane >> 3, sl = lane & 7;
-  const int nu = L.nu;
-  start_next();
-  const int cell = __ldg(list + blockIdx.x);
+__device__ __forceinline__ void lds4(const T *p, T (&o)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  } else {
+    const double2 a = reinterpret_cast<const double2 *>(p)[0],
+                  b = reinterpret_cast<const double2 *>(p)[1];
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void lds2(const T *p, T &x, T &y) {
+  if constexpr (sizeof(T) == 4) {
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    x = v.x;
+    y = v.y;
+  } else {
+    const double2 v = *reinterpret_cast<const double2 *>(p);
+    x = v.x;
+    y = v.y;
+  }
+}
 
-  // ---- everything that the previous colour does not change
-  const int *ids = L.ids + (size_t)cell * kPatchIds;
-  const PatchPattern &pat = L.patterns[__ldg(L.pattern + cell)];
-  const int id0 = __ldg(ids + t);
-  const int id1 = t + kPatchThreads < kPatchNodes ? __ldg(ids + t + kPatchThreads) : 0;
-  const int pb = t < 27 ? __ldg(ids + kPatchBase + t) : 0;
-  const T *V = L.values + (size_t)cell * kPatchValues;
-  const T *F = factors + (size_t)cell * S1::stride;
-  const bool vtx = warp < 2, edge = warp >= 2 && warp < 5, rest = warp == 5 || warp == 6;
-  // Values a thread keeps, by the work of its warp (one array, so that the
-  // warps' different lists share registers):
-  //   vertex, edge rows: A entries 0..15, BT entries 16 + 4 c + q, D 28..30
-  //   other rows:        A entries 0..5, BT entries 6 + c
-  //   pressure rows:     B entries 4 c + q
-  //   warps 5..7:        A^{-1} row 12..38, W 39..42, S^{-1} row 43..46
-  T R[47];
-  uint4 s0 = {0, 0, 0, 0}, s1 = {0, 0, 0, 0};
-  unsigned bts = 0;
-  if (vtx) {
-    const T *p = V + 4 * t;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ld4(p + q * 256, R[4 * q], R[4 * q + 1], R[4 * q + 2], R[4 * q + 3]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      ld4(p + kOffTV + c * 256, R[16 + 4 * c], R[17 + 4 * c], R[18 + 4 * c], R[19 + 4 * c]);
-  } else if (edge) {
-    const int li = t - 64;
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      ld4(V + kOffE + (q * 96 + li) * 4, R[4 * q], R[4 * q + 1], R[4 * q + 2], R[4 * q + 3]);
-    ld2(V + kOffE2 + li * 2, R[8], R[9]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) ld2(V + kOffTE + (c * 96 + li) * 2, R[16 + 4 * c], R[17 + 4 * c]);
-  } else if (rest) {
-    const int li = t - 160;
-    ld4(V + kOffR + li * 4, R[0], R[1], R[2], R[3]);
-    ld2(V + kOffR2 + li * 2, R[4], R[5]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) R[6 + c] = __ldcs(V + kOffTR + c * 64 + li);
-  }
-  if (warp < 7) {
-    s0 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[t]));
-    if (warp < 5) s1 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[t]) + 1);
-    bts = __ldg(reinterpret_cast<const unsigned *>(pat.bt[t]));
-  } else {  // B rows: the D block of the factors in the order of the CSR row
-    bts = __ldg(reinterpret_cast<const unsigned *>(pat.bj[lane]));
-    unsigned o[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = (bts >> (8 * q)) & 0xff;
-      o[q] = __ldg(&pat.own[j]);
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        R[4 * c + q] = j < NU_LOC ? __ldg(F + S1::offD + (sub * 3 + c) * NU_LOC + j) : T(0);
-    }
-    s0.x = o[0] | (o[1] << 16);
-    s0.y = o[2] | (o[3] << 16);
-  }
-  // right-hand side: lane 0..2 of a row its component, lane 0 of a B row
-  const int k = warp * 4 + sub;  // row in c_rows order
-  const int row = c_rows[k < 27 ? k : 27];
-  T f = T(0);
-  if (k < NU_LOC && sl < 3) f = __ldcg(rhs + (size_t)sl * nu + (__ldg(ids + kPatchOwn + row) >> 2));
-  if (warp == 7 && sl == 0) f = __ldcg(rhs + (size_t)3 * nu + __ldg(ids + kPatchBase) + sub);
-  // block solve: warps 5..7 one component each, warps 0..3 one row of D each
-  const bool solver = warp >= 5;
-  const int comp = warp - 5;
-  const bool in = lane < NU_LOC;
-  if (solver) {
-#pragma unroll
-    for (int j = 0; j < NU_LOC; ++j) R[12 + j] = in ? __ldcs(F + j * NU_LOC + lane) : T(0);
-#pragma unroll
-    for (int m = 0; m < NP_LOC; ++m) {
-      R[39 + m] = in ? __ldcs(F + S1::offW + (m * 3 + comp) * NU_LOC + lane) : T(0);
-      R[43 + m] = lane < NP_LOC ? __ldg(F + S1::offS + m * NP_LOC + lane) : T(0);  // S^{-1}[lane][m]
-    }
-  } else if (warp < NP_LOC) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      R[28 + c] = in ? __ldcs(F + S1::offD + (warp * 3 + c) * NU_LOC + lane) : T(0);
-  }
-
-  // ---- current values of the patch
-  wait_previous();
-  {
-    auto at = [&](int e) {  // the copy that holds node e >> 2 at this colour's turn
-      return (size_t)((e ^ ((e >> 1) & odd)) & 1) * nu + (e >> 2);
-    };
+// Sum of one row's entries for one lane of its eight: entries q of lane li in
+// the order of the row-group kernel.  VAL: the cell's packed values; u, p: the
+// patch; s0, s1, bts: places of the lane's nodes and pressures.
+template <typename T, typename U>
+__device__ __forceinline__ void row_sum(int group, int li, const T *V, const U &u, const T *p,
+                                        const uint4 &s0, const uint4 &s1, unsigned bts, T &c0,
+                                        T &c1, T &c2) {
+  c0 = c1 = c2 = T(0);
+  auto a_entry = [&](unsigned off, T v) {
     T x, y, z;
-    const Node<T> n0 = Node<T>::load(L.u, at(id0));
-    if (t + kPatchThreads < kPatchNodes) {
-      const Node<T> n1 = Node<T>::load(L.u, at(id1));
-      comps(n1, x, y, z);
-      sm.u.set(t + kPatchThreads, x, y, z);
-    }
-    if (t < 27) {
+    u.at(off, x, y, z);
+    c0 += v * x;
+    c1 += v * y;
+    c2 += v * z;
+  };
+  auto a_four = [&](unsigned lo, unsigned hi, const T *q) {
+    T v[4];
+    lds4(q, v);
+    a_entry(lo & 0xffff, v[0]);
+    a_entry(lo >> 16, v[1]);
+    a_entry(hi & 0xffff, v[2]);
+    a_entry(hi >> 16, v[3]);
+  };
+  auto a_two = [&](unsigned o, const T *q) {
+    T v0, v1;
+    lds2(q, v0, v1);
+    a_entry(o & 0xffff, v0);
+    a_entry(o >> 16, v1);
+  };
+  auto bt_entry = [&](int q, T v0, T v1, T v2) {
+    const T pc = p[(bts >> (8 * q)) & 0xff];
+    c0 += v0 * pc;
+    c1 += v1 * pc;
+    c2 += v2 * pc;
+  };
+  if (group < 2) {  // vertex rows
+    V += 4 * li;
+    a_four(s0.x, s0.y, V);
+    a_four(s0.z, s0.w, V + 256);
+    T g0[4], g1[4], g2[4];
+    lds4(V + kOffTV, g0);
+    lds4(V + kOffTV + 256, g1);
+    lds4(V + kOffTV + 512, g2);
 #pragma unroll
-      for (int m = 0; m < NP_LOC; ++m) sm.p[t][m] = __ldcg(L.p + pb + m);
-    }
-    comps(n0, x, y, z);
-    sm.u.set(t, x, y, z);
-    if (t == kPatchThreads - 1) {
-      sm.u.set(kZeroSlot, T(0), T(0), T(0));
+    for (int q = 0; q < 4; ++q) bt_entry(q, g0[q], g1[q], g2[q]);
+    a_four(s1.x, s1.y, V + 512);
+    a_four(s1.z, s1.w, V + 768);
+  } else if (group < 5) {  // edge rows
+    li -= 64;
+    a_four(s0.x, s0.y, V + kOffE + 4 * li);
+    a_four(s0.z, s0.w, V + kOffE + 4 * (96 + li));
+    T g0[2], g1[2], g2[2];
+    lds2(V + kOffTE + 2 * li, g0[0], g0[1]);
+    lds2(V + kOffTE + 2 * li + 192, g1[0], g1[1]);
+    lds2(V + kOffTE + 2 * li + 384, g2[0], g2[1]);
+    bt_entry(0, g0[0], g1[0], g2[0]);
+    bt_entry(1, g0[1], g1[1], g2[1]);
+    a_two(s1.x, V + kOffE2 + 2 * li);
+  } else {  // face rows and the centre
+    li -= 160;
+    a_four(s0.x, s0.y, V + kOffR + 4 * li);
+    a_two(s0.z, V + kOffR2 + 2 * li);
+    bt_entry(0, V[kOffTR + li], V[kOffTR + 64 + li], V[kOffTR + 128 + li]);
+  }
+}
+
+// Pressure rows of a cell: lanes 8 k .. 8 k + 7 return the sum of row k; bj,
+// o01, o23: the row's own nodes and their places (D in the order of the CSR
+// row)
+template <typename T, typename U>
+__device__ __forceinline__ T pressure_sum(int sub, const T *fac, const U &u, unsigned bj,
+                                          unsigned o01, unsigned o23) {
+  T c = 0;
 #pragma unroll
-      for (int m = 0; m < NP_LOC; ++m) sm.p[27][m] = T(0);
+  for (int q = 0; q < 4; ++q) {
+    const int jn = (bj >> (8 * q)) & 0xff;
+    const bool live = jn < NU_LOC;
+    const T *D = fac + Schur<1>::offD + sub * 3 * NU_LOC + (live ? jn : 0);
+    T g0, g1, g2;
+    u.at(((q < 2 ? o01 : o23) >> (16 * (q & 1))) & 0xffff, g0, g1, g2);
+    const T d0 = live ? D[0] : T(0), d1 = live ? D[NU_LOC] : T(0),
+            d2 = live ? D[2 * NU_LOC] : T(0);
+    c += dot3(d0, g0, d1, g1, d2, g2);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+  return c;
+}
+template <typename P>
+__device__ __forceinline__ void pressure_pattern(const P &pat, int lane, unsigned &bj,
+                                                 unsigned &o01, unsigned &o23) {
+  bj = __ldg(reinterpret_cast<const unsigned *>(pat.bj[lane]));
+  unsigned o[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o[q] = __ldg(&pat.own[(bj >> (8 * q)) & 0xff]);
+  o01 = o[0] | (o[1] << 16);
+  o23 = o[2] | (o[3] << 16);
+}
+
+// copy of a patch entry's node that is current at this colour's turn
+__device__ __forceinline__ size_t node_at(int e, int odd, int nu) {
+  return (size_t)((e ^ ((e >> 1) & odd)) & 1) * nu + (e >> 2);
+}
+
+// 16 bytes global -> shared, asynchronous, through L2
+__device__ __forceinline__ void async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// bounded wait for a copy that is to be left behind
+__device__ __forceinline__ void drain(uint64_t *bar, int phase) {
+  for (long long it = 0; it < kMaxPolls; ++it)
+    if (mbar_test_wait(bar, phase & 1)) break;
+}
+
+// ------------------------------------------------------------------ FP32 ---
+struct Smem32 {
+  float values[2][kPatchValues];        // packed rows of this cell and the next
+  float fac[2][Schur<1>::stride];       // factors of this cell and the next
+  int ids[4][kPatchIds];                // patch lists, up to three cells ahead
+  Tri<float, kPatchNodes + 1> u[3];     // current values of a patch, then a zero
+  float4 p[3][28];                      // pressures of a cell and its neighbours, then zeros
+  float4 f[3][28];                      // right-hand side: own nodes, then the pressure part
+  Tri<float, NU_LOC> r[2];              // velocity part of the local residual
+  float rp[2][NP_LOC];
+  uint64_t vbar[2], fbar[2], ibar[4];
+};
+constexpr int kCtas32 = 3;  // resident CTAs per SM (67 KB of shared memory each)
+
+// Persistent CTAs, each walking the colour's cells with a stride.  Warps 0..6
+// form a cell's local residual; warp 7 solves the cell before it, writes its
+// update and starts the bulk copies: packed rows (15.6 KB) and factors
+// (5.6 KB) two cells ahead, patch lists four ahead.  The gathers of current
+// values, which no cell of this colour changes, are 16-byte asynchronous
+// copies into shared memory two cells ahead: one cell ahead (in registers or
+// in a second buffer) left their latency exposed.
+// Bound by HBM and by shared-memory wavefronts on large levels, by the chain
+// gather -> sums -> solve -> update on small ones.
+__global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
+    PatchLevel<float> L, const int *__restrict__ list, int n, const float *__restrict__ factors,
+    float damp, int odd, int *err) {
+  using S1 = Schur<1>;
+  extern __shared__ __align__(16) unsigned char raw[];
+  Smem32 &sm = *reinterpret_cast<Smem32 *>(raw);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, sub = lane >> 3, sl = lane & 7;
+  const int nu = L.nu, G = gridDim.x, first = blockIdx.x;
+  const int count = (n - first + G - 1) / G;
+  start_next();
+  if (t == 0) {
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.vbar[b], 1);
+      mbar_init(&sm.fbar[b], 1);
+    }
+    for (int b = 0; b < 4; ++b) mbar_init(&sm.ibar[b], 1);
+    fence_mbar_init();
+    for (int b = 0; b < 3; ++b) {
+      sm.u[b].set(kZeroSlot, 0.f, 0.f, 0.f);
+      sm.p[b][27] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   __syncthreads();
+  // a wait that runs out marks the launch as failed; the warp goes on without
+  // touching global memory through a patch list that did not arrive
+  long long polls = kMaxPolls;
+  auto arrived = [&](uint64_t *bar, int phase) {
+    if (mbar_wait(bar, phase & 1, polls)) return true;
+    polls = 1;
+    if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
+    return false;
+  };
 
-  // ---- local residual
-  {
-    const unsigned sw[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-    T c0 = 0, c1 = 0, c2 = 0;
-    const T *ps = &sm.p[0][0];
-    auto a_entry = [&](int q) {
-      T x, y, z;
-      sm.u.get((sw[q >> 1] >> (16 * (q & 1))) & 0xffff, x, y, z);
-      c0 += R[q] * x;
-      c1 += R[q] * y;
-      c2 += R[q] * z;
+  if (warp == 7) {
+    // ------------------------------------------------ copies and block solve
+    int nv = 0, nf = 0, ni = 0;  // lane 0: copies started of each kind
+    auto cell_of = [&](int c) { return __ldg(list + first + (size_t)c * G); };
+    auto bring_values = [&](int c, int cell) {
+      bulk_load(sm.values[c & 1], L.values + (size_t)cell * kPatchValues, sizeof(sm.values[0]),
+                &sm.vbar[c & 1]);
+      nv = c + 1;
     };
-    auto bt_entry = [&](int q, int at, int stride) {
-      const T pc = ps[(bts >> (8 * q)) & 0xff];
-      c0 += R[at] * pc;
-      c1 += R[at + stride] * pc;
-      c2 += R[at + 2 * stride] * pc;
+    auto bring_fac = [&](int c, int cell) {
+      bulk_load(sm.fac[c & 1], factors + (size_t)cell * S1::stride, sizeof(sm.fac[0]),
+                &sm.fbar[c & 1]);
+      nf = c + 1;
     };
-    if (vtx) {
+    auto bring_ids = [&](int c, int cell) {
+      bulk_load(sm.ids[c & 3], L.ids + (size_t)cell * kPatchIds, sizeof(sm.ids[0]),
+                &sm.ibar[c & 3]);
+      ni = c + 1;
+    };
+    int a2 = 0, a3 = 0, a4 = 0;  // cells j + 2, j + 3 and j + 4
+    if (lane == 0) {
+      const int c0 = cell_of(0);
+      bring_ids(0, c0);
+      bring_values(0, c0);
+      bring_fac(0, c0);
+      if (count > 1) {
+        const int c1 = cell_of(1);
+        bring_ids(1, c1);
+        bring_values(1, c1);
+        bring_fac(1, c1);
+      }
+      if (count > 2) bring_ids(2, a2 = cell_of(2));
+      if (count > 3) bring_ids(3, a3 = cell_of(3));
+      if (count > 4) a4 = cell_of(4);
+    }
+    const bool in = lane < NU_LOC;
+    bool alive = true;
+    wait_previous();
+    for (int j = 0; j < count; ++j) {
+      const int b = j & 1;
+      const int *ids = sm.ids[j & 3];
+      alive = arrived(&sm.ibar[j & 3], j >> 2) && alive;
+      Node<float> old = {};
+      float pold = 0.f;
+      size_t where = 0;
+      if (alive) {
+        const int me = ids[kPatchOwn + (in ? lane : 0)];
+        old = Node<float>::load(L.u, node_at(me, odd, nu));
+        // into the other copy, unless the node belongs to this cell alone
+        const bool single = ((unsigned)ids[kPatchSingle] >> lane) & 1;
+        where = node_at(single ? me : me ^ 1, odd, nu);
+        if (lane < NP_LOC) pold = __ldcg(L.p + ids[kPatchBase] + lane);
+      }
+      alive = arrived(&sm.fbar[b], j >> 1) && alive;
+      const float *F = sm.fac[b] + (in ? lane : 0);
+      bar_sync(kBarFull + b, kPatchThreads);  // the residual is there
+      if (alive && lane == 0 && j + 2 < count) bring_values(j + 2, a2);
+      // y_c = A^{-1} r_c
+      float y0 = 0, y1 = 0, y2 = 0;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a_entry(q);
+      for (int q = 0; q < NU_LOC; ++q) {
+        float x, y, z;
+        sm.r[b].get(q, x, y, z);
+        const float a = F[q * NU_LOC];
+        y0 += a * x;
+        y1 += a * y;
+        y2 += a * z;
+      }
+      if (!in) y0 = y1 = y2 = 0.f;
+      // t = r_p - D y, p = S^{-1} t, x = y - W p
+      float s[NP_LOC], p[NP_LOC];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) bt_entry(q, 16 + q, 4);
+      for (int k = 0; k < NP_LOC; ++k) {
+        const float *D = F + S1::offD + 3 * NU_LOC * k;
+        s[k] = dot3(in ? D[0] : 0.f, y0, in ? D[NU_LOC] : 0.f, y1, in ? D[2 * NU_LOC] : 0.f, y2);
+      }
 #pragma unroll
-      for (int q = 8; q < 16; ++q) a_entry(q);
-    } else if (edge) {
+      for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a_entry(q);
+        for (int k = 0; k < NP_LOC; ++k) s[k] += __shfl_xor_sync(kFull, s[k], o);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) bt_entry(q, 16 + q, 4);
+      for (int k = 0; k < NP_LOC; ++k) {
+        s[k] = sm.rp[b][k] - s[k];
+        p[k] = 0.f;
+      }
 #pragma unroll
-      for (int q = 8; q < 10; ++q) a_entry(q);
-    } else if (rest) {
+      for (int m = 0; m < NP_LOC; ++m)
 #pragma unroll
-      for (int q = 0; q < 6; ++q) a_entry(q);
-      bt_entry(0, 6, 1);
-    } else {
+        for (int k = 0; k < NP_LOC; ++k) p[k] += sm.fac[b][S1::offS + m * NP_LOC + k] * s[m];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        T g0, g1, g2;
-        sm.u.get((sw[q >> 1] >> (16 * (q & 1))) & 0xffff, g0, g1, g2);
-        c0 += R[q] * g0 + R[4 + q] * g1 + R[8 + q] * g2;
+      for (int k = 0; k < NP_LOC; ++k) {
+        const float *W = F + S1::offW + 3 * NU_LOC * k;
+        y0 -= W[0] * p[k];
+        y1 -= W[NU_LOC] * p[k];
+        y2 -= W[2 * NU_LOC] * p[k];
+      }
+      if (alive) {
+        if (in) {
+          float x, y, z;
+          comps(old, x, y, z);
+          x += damp * y0;
+          y += damp * y1;
+          z += damp * y2;
+          make_node(x, y, z).store(L.u, where);
+        }
+        if (lane < NP_LOC) {
+          const float pl = lane == 0 ? p[0] : (lane == 1 ? p[1] : (lane == 2 ? p[2] : p[3]));
+          pold += damp * pl;
+          L.p[ids[kPatchBase] + lane] = pold;
+        }
+      }
+      __syncwarp();  // factors and patch list have been read
+      if (alive && lane == 0) {
+        if (j + 2 < count) bring_fac(j + 2, a2);
+        if (j + 4 < count) bring_ids(j + 4, a4);
+        a2 = a3;
+        a3 = a4;
+        if (j + 5 < count) a4 = cell_of(j + 5);
+      }
+      if (j + 2 < count) bar_arrive(kBarFree + b, kPatchThreads);
+    }
+    if (!alive && lane == 0) {  // copies still in flight
+      for (int c = nv > 2 ? nv - 2 : 0; c < nv; ++c) drain(&sm.vbar[c & 1], c >> 1);
+      for (int c = nf > 2 ? nf - 2 : 0; c < nf; ++c) drain(&sm.fbar[c & 1], c >> 1);
+      for (int c = ni > 4 ? ni - 4 : 0; c < ni; ++c) drain(&sm.ibar[c & 3], c >> 2);
+    }
+    return;
+  }
+
+  // ------------------------------------------------------------ residuals
+  const bool last = warp == 6;
+  const int k = warp * 4 + sub;  // row in c_rows order; the spare group of warp 6 repeats the centre
+  const int row = c_rows[k];
+  bool alive = true;
+  int pid = -1;
+  uint4 s0 = {0, 0, 0, 0}, s1 = {0, 0, 0, 0};
+  unsigned bts = 0, bj = 0, o01 = 0, o23 = 0;
+  auto pattern = [&](int id) {  // where the lane's entries lie in the patch
+    if (id == pid) return;      // most cells of a level share one
+    pid = id;
+    const PatchPattern &pat = L.patterns[id];
+    s0 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[t]));
+    bts = __ldg(reinterpret_cast<const unsigned *>(pat.bt[t]));
+    if (warp < 5) s1 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[t]) + 1);
+    if (last) pressure_pattern(pat, lane, bj, o01, o23);
+  };
+  // start the gathers of cell c (one group of copies a cell, empty or not)
+  int gpid = -1;  // pattern of the places below
+  unsigned pl = 0;
+  auto gather = [&](int c) {
+    if (c < count) {
+      alive = arrived(&sm.ibar[c & 3], c >> 2) && alive;
+      if (alive) {
+        const int *ids = sm.ids[c & 3];
+        const int g = c % 3;
+        if (ids[kPatchPattern] != gpid) {
+          gpid = ids[kPatchPattern];
+          const PatchPattern &pat = L.patterns[gpid];
+          pl = __ldg(&pat.place[t]);
+          if (t + kRowLanes < kPatchNodes) pl |= (unsigned)__ldg(&pat.place[t + kRowLanes]) << 16;
+        }
+        const float4 *u4 = static_cast<const float4 *>(L.u);
+        async16(&sm.u[g].v[pl & 0xffff], u4 + node_at(ids[t], odd, nu));
+        if (t + kRowLanes < kPatchNodes)
+          async16(&sm.u[g].v[pl >> 16], u4 + node_at(ids[t + kRowLanes], odd, nu));
+        if (t < 27)
+          async16(&sm.p[g][t], L.p + ids[kPatchBase + t]);
+        else if (t < 55)  // own nodes of the right-hand side, then its pressures
+          async16(&sm.f[g][t - 27],
+                  t < 54 ? static_cast<const float4 *>(L.f) + (ids[kPatchOwn + t - 27] >> 2)
+                         : reinterpret_cast<const float4 *>(L.fp + ids[kPatchBase]));
       }
     }
+    async_commit();
+  };
+  if (arrived(&sm.ibar[0], 0)) pattern(sm.ids[0][kPatchPattern]);
+  // everything up to here does not depend on the previous launch
+  wait_previous();
+  gather(0);
+  gather(1);
+  for (int j = 0; j < count; ++j) {
+    const int b = j & 1, g = j % 3;
+    async_wait<1>();                  // this thread's copies of cell j
+    bar_sync(kBarRows, kRowLanes);    // everybody's; and cell j - 1 has been read
+    gather(j + 2);
+    if (alive) pattern(sm.ids[j & 3][kPatchPattern]);
+    alive = arrived(&sm.vbar[b], j >> 1) && alive;
+    float c0, c1, c2;
+    row_sum(warp, t, sm.values[b], sm.u[g], &sm.p[g][0].x, s0, s1, bts, c0, c1, c2);
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
       c0 += __shfl_xor_sync(kFull, c0, o);
-      if (warp < 7) {
-        c1 += __shfl_xor_sync(kFull, c1, o);
-        c2 += __shfl_xor_sync(kFull, c2, o);
+      c1 += __shfl_xor_sync(kFull, c1, o);
+      c2 += __shfl_xor_sync(kFull, c2, o);
+    }
+    float cp = 0.f;
+    if (last) {
+      alive = arrived(&sm.fbar[b], j >> 1) && alive;
+      cp = pressure_sum(sub, sm.fac[b], sm.u[g], bj, o01, o23);
+    }
+    if (j >= 2) bar_sync(kBarFree + b, kPatchThreads);  // this buffer's cell before is solved
+    if (k < NU_LOC && sl < 3)
+      sm.r[b].ref(row, sl) =
+          reinterpret_cast<const float *>(&sm.f[g][row])[sl] - (sl == 0 ? c0 : (sl == 1 ? c1 : c2));
+    if (last && sl == 0) sm.rp[b][sub] = reinterpret_cast<const float *>(&sm.f[g][27])[sub] - cp;
+    bar_arrive(kBarFull + b, kPatchThreads);
+  }
+}
+
+// ------------------------------------------------------------------ FP64 ---
+struct Smem64 {
+  double values[2][kPatchValues];
+  double fac[2][Schur<1>::stride];
+  int ids[3][kPatchIds];
+  Tri<double, kPatchNodes + 1> u;
+  __align__(16) double p[28][NP_LOC];
+  Tri<double, 28> r;
+  double yp[3][7 * NU_LOC];  // partial A^{-1} r
+  double y[3][32];
+  double rp[NP_LOC], t[NP_LOC];
+  uint64_t vbar[2], fbar[2], ibar[3];
+};
+constexpr int kCtas64 = 2;  // resident CTAs per SM (106 KB of shared memory each)
+
+// FP64: the pipe takes half a lane per cycle in each quarter of the SM, so a
+// warp's FMA occupies its quarter for 64 cycles and every phase is spread
+// over the quarters (warp % 4): vertex rows on quarters 0 and 1, edges on 2,
+// 3 and 2, the other rows on 0 and 3, pressure rows on 1; the block solve on
+// all warps instead of one.  Two stages of bulk copies as in FP32.
+__global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
+    PatchLevel<double> L, const int *__restrict__ list, int n, const double *__restrict__ factors,
+    double damp, int odd, int *err) {
+  using S1 = Schur<1>;
+  extern __shared__ __align__(16) unsigned char raw[];
+  Smem64 &sm = *reinterpret_cast<Smem64 *>(raw);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, sub = lane >> 3, sl = lane & 7;
+  const int nu = L.nu, G = gridDim.x, first = blockIdx.x;
+  const int count = (n - first + G - 1) / G;
+  start_next();
+  if (t == 0) {
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.vbar[b], 1);
+      mbar_init(&sm.fbar[b], 1);
+    }
+    for (int b = 0; b < 3; ++b) mbar_init(&sm.ibar[b], 1);
+    fence_mbar_init();
+    sm.u.set(kZeroSlot, 0.0, 0.0, 0.0);
+    for (int m = 0; m < NP_LOC; ++m) sm.p[27][m] = 0.0;
+    sm.r.set(27, 0.0, 0.0, 0.0);
+  }
+  __syncthreads();
+  long long polls = kMaxPolls;
+  auto arrived = [&](uint64_t *bar, int phase) {
+    if (mbar_wait(bar, phase & 1, polls)) return true;
+    polls = 1;
+    if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
+    return false;
+  };
+  auto cell_of = [&](int c) { return __ldg(list + first + (size_t)c * G); };
+  auto bring = [&](int c, int cell) {  // thread 0: values and factors of the CTA's cell c
+    bulk_load(sm.values[c & 1], L.values + (size_t)cell * kPatchValues, sizeof(sm.values[0]),
+              &sm.vbar[c & 1]);
+    bulk_load(sm.fac[c & 1], factors + (size_t)cell * S1::stride, sizeof(sm.fac[0]),
+              &sm.fbar[c & 1]);
+  };
+  auto bring_ids = [&](int c, int cell) {
+    bulk_load(sm.ids[c % 3], L.ids + (size_t)cell * kPatchIds, sizeof(sm.ids[0]), &sm.ibar[c % 3]);
+  };
+  int a2 = 0, a3 = 0, issued = 0, issued_ids = 0;  // thread 0
+  if (t == 0) {
+    for (int c = 0; c < 2 && c < count; ++c) {
+      const int cell = cell_of(c);
+      bring_ids(c, cell);
+      bring(c, cell);
+    }
+    if (count > 2) bring_ids(2, a2 = cell_of(2));
+    if (count > 3) a3 = cell_of(3);
+    issued = count < 2 ? count : 2;
+    issued_ids = count < 3 ? count : 3;
+  }
+  // row group of a warp: 0, 1 vertices, 2..4 edges, 5, 6 the rest, 7 pressure rows
+  const int group = warp < 4 ? warp : (warp == 4 ? 5 : (warp == 5 ? 7 : (warp == 6 ? 4 : 6)));
+  const int k = group * 4 + sub, li = 32 * group + lane;
+  const int row = c_rows[k < 27 ? k : 27];
+  const bool in = lane < NU_LOC;
+  // current values and right-hand side of one cell, on their way
+  Node<double> n0 = {}, n1 = {};
+  double pv = 0.0, f = 0.0;
+  auto gather_u = [&](const int *ids) {
+    n0 = Node<double>::load(L.u, node_at(ids[t], odd, nu));
+    if (t + kPatchThreads < kPatchNodes)
+      n1 = Node<double>::load(L.u, node_at(ids[t + kPatchThreads], odd, nu));
+    if (t < 27 * NP_LOC) pv = __ldcg(L.p + ids[kPatchBase + (t >> 2)] + (t & 3));
+    if (k < NU_LOC && sl < 3)
+      f = __ldcg(static_cast<const double *>(L.f) + 4 * (size_t)(ids[kPatchOwn + row] >> 2) + sl);
+    if (group == 7 && sl == 0) f = __ldcg(L.fp + ids[kPatchBase] + sub);
+  };
+  uint4 s0 = {0, 0, 0, 0}, s1 = {0, 0, 0, 0};
+  unsigned bts = 0, bj = 0, o01 = 0, o23 = 0, pl = 0, mine = 0;
+  int pid = -1;
+  auto pattern = [&](int id) {
+    if (id == pid) return;
+    pid = id;
+    const PatchPattern &pat = L.patterns[id];
+    if (group < 7) {
+      s0 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[li]));
+      if (group < 5) s1 = __ldg(reinterpret_cast<const uint4 *>(pat.slot[li]) + 1);
+      bts = __ldg(reinterpret_cast<const unsigned *>(pat.bt[li]));
+    } else {
+      pressure_pattern(pat, lane, bj, o01, o23);
+    }
+    pl = __ldg(&pat.place[t]);
+    if (t + kPatchThreads < kPatchNodes)
+      pl |= (unsigned)__ldg(&pat.place[t + kPatchThreads]) << 16;
+    mine = __ldg(&pat.own[lane]);
+  };
+  bool alive = arrived(&sm.ibar[0], 0);
+  if (alive) pattern(sm.ids[0][kPatchPattern]);
+  wait_previous();
+  if (alive) gather_u(sm.ids[0]);
+  int ib = 0, ip = 0;
+  for (int j = 0; j < count; ++j) {
+    const int b = j & 1;
+    const int *ids = sm.ids[ib];
+    const int ibn = ib == 2 ? 0 : ib + 1, ipn = ib == 2 ? ip ^ 1 : ip;
+    {
+      double x, y, z;
+      comps(n0, x, y, z);
+      sm.u.set(pl & 0xffff, x, y, z);
+      if (t + kPatchThreads < kPatchNodes) {
+        comps(n1, x, y, z);
+        sm.u.set(pl >> 16, x, y, z);
+      }
+      if (t < 27 * NP_LOC) (&sm.p[0][0])[t] = pv;
+    }
+    const double fi = f;
+    __syncthreads();
+    int next_pid = pid;
+    if (j + 1 < count) {
+      alive = arrived(&sm.ibar[ibn], ipn) && alive;
+      if (alive) {
+        gather_u(sm.ids[ibn]);
+        next_pid = sm.ids[ibn][kPatchPattern];
       }
     }
-    if (k < NU_LOC && sl < 3) sm.r[sl][row] = f - (sl == 0 ? c0 : (sl == 1 ? c1 : c2));
-    if (warp == 7 && sl == 0) sm.rp[sub] = f - c0;
-  }
-  __syncthreads();
-
-  // ---- y = A^{-1} r, one component per warp
-  T y = 0;
-  if (solver) {
-#pragma unroll
-    for (int j = 0; j < NU_LOC; ++j) y += R[12 + j] * sm.r[comp][j];
-    sm.y[comp][lane] = y;
-  }
-  __syncthreads();
-
-  // ---- t = r_p - D y, p = S^{-1} t, x = y - W p
-  if (warp < NP_LOC) {
-    const T s = warp_sum(R[28] * sm.y[0][lane] + R[29] * sm.y[1][lane] + R[30] * sm.y[2][lane]);
-    if (lane == 0) sm.t[warp] = sm.rp[warp] - s;
-  }
-  __syncthreads();
-  if (solver) {
-    T pk = 0;
-#pragma unroll
-    for (int m = 0; m < NP_LOC; ++m) pk += R[43 + m] * sm.t[m];
-#pragma unroll
-    for (int m = 0; m < NP_LOC; ++m) y -= R[39 + m] * __shfl_sync(kFull, pk, m);
-    if (in) {
-      const int me = __ldg(ids + kPatchOwn + lane);
-      const unsigned single = (unsigned)__ldg(ids + kPatchSingle);
-      // into the other copy, unless the node belongs to this cell alone
-      const int copy = (me ^ ((me >> 1) & odd)) & 1;
-      const int w = ((single >> lane) & 1) ? copy : copy ^ 1;
-      T v = sm.u.get(__ldg(&pat.own[lane]), comp);
-      v += damp * y;
-      Node<T>::component(L.u, (size_t)w * nu + (me >> 2))[comp] = v;
+    alive = arrived(&sm.vbar[b], j >> 1) && alive;
+    alive = arrived(&sm.fbar[b], j >> 1) && alive;
+    if (group < 7) {
+      double c0, c1, c2;
+      row_sum(group, li, sm.values[b], sm.u, &sm.p[0][0], s0, s1, bts, c0, c1, c2);
+      // six FP64 additions instead of nine: lanes 0..3 go on with component
+      // 1, lanes 4..7 with component 2
+      c0 += __shfl_xor_sync(kFull, c0, 4);
+      const double o12 = __shfl_xor_sync(kFull, (sl & 4) ? c1 : c2, 4);
+      double d = ((sl & 4) ? c2 : c1) + o12;
+      c0 += __shfl_xor_sync(kFull, c0, 2);
+      d += __shfl_xor_sync(kFull, d, 2);
+      c0 += __shfl_xor_sync(kFull, c0, 1);
+      d += __shfl_xor_sync(kFull, d, 1);
+      const double d2 = __shfl_xor_sync(kFull, d, 6);
+      if (k < NU_LOC && sl < 3) sm.r.ref(row, sl) = fi - (sl == 0 ? c0 : (sl == 1 ? d : d2));
+    } else {
+      const double c = pressure_sum(sub, sm.fac[b], sm.u, bj, o01, o23);
+      if (sl == 0) sm.rp[sub] = fi - c;
     }
-    if (warp == 7 && lane < NP_LOC) {
-      T v = sm.p[0][lane];
-      v += damp * pk;
-      L.p[__ldg(ids + kPatchBase) + lane] = v;
+    __syncthreads();
+    const double *F = sm.fac[b];
+    if (t >= 64 && t - 64 < 7 * NU_LOC) {  // y = A^{-1} r: four columns per thread
+      const int q = t - 64, gq = q / NU_LOC, i = q - gq * NU_LOC;
+      double c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int col = 4 * gq + m;
+        double x, y, z;
+        sm.r.get(col, x, y, z);
+        const double a = col < NU_LOC ? F[col * NU_LOC + i] : 0.0;
+        c0 += a * x;
+        c1 += a * y;
+        c2 += a * z;
+      }
+      sm.yp[0][q] = c0;
+      sm.yp[1][q] = c1;
+      sm.yp[2][q] = c2;
     }
+    __syncthreads();
+    double y = 0;
+    if (warp < 3) {  // one component per warp
+      if (in) {
+#pragma unroll
+        for (int q = 0; q < 7; ++q) y += sm.yp[warp][q * NU_LOC + lane];
+      }
+      sm.y[warp][lane] = y;
+    }
+    __syncthreads();
+    if (warp >= 4) {  // t = r_p - D y, one pressure per warp
+      const double *D = F + S1::offD + (warp - 4) * 3 * NU_LOC + (in ? lane : 0);
+      const double s = warp_sum(in ? D[0] * sm.y[0][lane] + D[NU_LOC] * sm.y[1][lane] +
+                                         D[2 * NU_LOC] * sm.y[2][lane]
+                                   : 0.0);
+      if (lane == 0) sm.t[warp - 4] = sm.rp[warp - 4] - s;
+    }
+    __syncthreads();
+    if (warp < 3) {  // p = S^{-1} t, x = y - W p, update of one component
+      double pk = 0;
+      if (lane < NP_LOC) {
+#pragma unroll
+        for (int m = 0; m < NP_LOC; ++m) pk += F[S1::offS + m * NP_LOC + lane] * sm.t[m];
+      }
+      const double *W = F + S1::offW + warp * NU_LOC + (in ? lane : 0);
+#pragma unroll
+      for (int m = 0; m < NP_LOC; ++m) y -= W[m * 3 * NU_LOC] * __shfl_sync(kFull, pk, m);
+      if (alive) {
+        if (in) {
+          const int me = ids[kPatchOwn + lane];
+          // into the other copy, unless the node belongs to this cell alone
+          const bool single = ((unsigned)ids[kPatchSingle] >> lane) & 1;
+          double v = sm.u.ref(mine >> 4, warp);
+          v += damp * y;
+          static_cast<double *>(L.u)[4 * node_at(single ? me : me ^ 1, odd, nu) + warp] = v;
+        }
+        if (warp == 2 && lane < NP_LOC) {
+          double v = sm.p[0][lane];
+          v += damp * pk;
+          L.p[ids[kPatchBase] + lane] = v;
+        }
+      }
+    }
+    __syncthreads();  // the stage and the gathered values have been read
+    if (alive && t == 0) {
+      if (j + 2 < count) bring(j + 2, a2), issued = j + 3;
+      if (j + 3 < count) bring_ids(j + 3, a3), issued_ids = j + 4;
+      a2 = a3;
+      if (j + 4 < count) a3 = cell_of(j + 4);
+    }
+    pattern(next_pid);
+    ib = ibn;
+    ip = ipn;
+  }
+  if (!alive && t == 0) {  // copies still in flight
+    for (int c = issued > 2 ? issued - 2 : 0; c < issued; ++c) {
+      drain(&sm.vbar[c & 1], c >> 1);
+      drain(&sm.fbar[c & 1], c >> 1);
+    }
+    for (int c = issued_ids > 3 ? issued_ids - 3 : 0; c < issued_ids; ++c)
+      drain(&sm.ibar[c % 3], c / 3);
   }
 }
 
 // u -> the copies (both), u on the Dirichlet nodes taken from the right-hand
-// side; p -> its copy
+// side; p -> its copy; the right-hand side with its components side by side
 template <typename T>
 __global__ void k_patch_pack_u(PatchLevel<T> L, const T *__restrict__ u, const T *__restrict__ rhs,
                                int hb, int np) {
@@ -468,8 +895,12 @@ __global__ void k_patch_pack_u(PatchLevel<T> L, const T *__restrict__ u, const T
       const Node<T> v = make_node(s[i], s[(size_t)nu + i], s[(size_t)2 * nu + i]);
       v.store(L.u, i);
       v.store(L.u, (size_t)nu + i);
+      make_node(rhs[i], rhs[(size_t)nu + i], rhs[(size_t)2 * nu + i]).store(L.f, i);
     }
-    if (i < np) L.p[i] = u[(size_t)3 * nu + i];
+    if (i < np) {
+      L.p[i] = u[(size_t)3 * nu + i];
+      L.fp[i] = rhs[(size_t)3 * nu + i];
+    }
   }
 }
 
@@ -543,6 +974,11 @@ __global__ void __launch_bounds__(256) k_patch_pack(PatchLevel<T> L, DevOp<T> op
     reinterpret_cast<float4 *>(V)[i] = reinterpret_cast<const float4 *>(stage)[i];
 }
 
+__global__ void k_patch_assign(int *ids, const int *pattern, int ncells) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < ncells) ids[(size_t)c * kPatchIds + kPatchPattern] = pattern[c];
+}
+
 // Pattern of a cell from the CSR patterns and its patch list (once per level,
 // at set-up).  MODE 0: a hash of the pattern into hash[cell]; 1: the pattern
 // of cell which[blockIdx.x] into patterns[blockIdx.x]; 2: compare with the
@@ -551,7 +987,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_patch_pattern(
     const int *ids_all, const int *a_rowptr, const int *a_col, const int *b_rowptr,
     const int *b_col, const int *bt_rowptr, const int *bt_col, int nact, const int *which,
-    PatchPattern *patterns, const int *pattern, unsigned long long *hash, int *bad) {
+    PatchPattern *patterns, unsigned long long *hash, int *bad) {
   __shared__ __align__(16) PatchPattern pt;
   __shared__ int node[kPatchNodes], own[NU_LOC], base[27];
   __shared__ unsigned long long h;
@@ -565,10 +1001,11 @@ __global__ void __launch_bounds__(256) k_patch_pattern(
     base[t] = ids[kPatchBase + t];
   }
   if (t == 0) h = 0;
-  for (int i = t; i < kRowLanes * 16; i += 256) (&pt.slot[0][0])[i] = (uint16_t)kZeroSlot;
+  for (int i = t; i < kRowLanes * 16; i += 256) (&pt.slot[0][0])[i] = (uint16_t)(16 * kZeroSlot);
   for (int i = t; i < kRowLanes * 4; i += 256) (&pt.bt[0][0])[i] = (uint8_t)kZeroP;
   if (t < 128) (&pt.bj[0][0])[t] = (uint8_t)NU_LOC;
-  if (t < 32) pt.own[t] = (uint16_t)kZeroSlot;
+  if (t < 32) pt.own[t] = (uint16_t)(16 * kZeroSlot);
+  for (int i = t; i < kPatchIds - 48; i += 256) pt.place[i] = (uint16_t)i;
   __syncthreads();
   auto find = [&](int id) {
     int lo = 0, hi = n;
@@ -587,7 +1024,7 @@ __global__ void __launch_bounds__(256) k_patch_pattern(
     if (s < 0)
       miss = true;
     else
-      pt.own[t] = (uint16_t)s;
+      pt.own[t] = (uint16_t)(16 * s);
   }
   for (int k = warp; k < NU_LOC; k += 8) {
     const int r = own[c_rows[k]];
@@ -598,7 +1035,7 @@ __global__ void __launch_bounds__(256) k_patch_pattern(
       if (s < 0)
         miss = true;
       else
-        pt.slot[8 * k + (j & 7)][j >> 3] = (uint16_t)s;
+        pt.slot[8 * k + (j & 7)][j >> 3] = (uint16_t)(16 * s);
     }
     if (r >= nact) continue;
     const int ts = bt_rowptr[r], mt = bt_rowptr[r + 1] - ts;
@@ -650,7 +1087,7 @@ __global__ void __launch_bounds__(256) k_patch_pattern(
       reinterpret_cast<unsigned long long *>(patterns + blockIdx.x)[i] = w[i];
   } else {
     const unsigned long long *v =
-        reinterpret_cast<const unsigned long long *>(patterns + pattern[cell]);
+        reinterpret_cast<const unsigned long long *>(patterns + ids[kPatchPattern]);
     bool differ = false;
     for (int i = t; i < words; i += 256) differ |= v[i] != w[i];
     if (differ) atomicOr(bad, 1);
@@ -662,11 +1099,12 @@ inline int ok() { return cudaPeekAtLastError() == cudaSuccess ? 1 : -1; }
 // launch that may start while the previous kernel of the stream still runs
 // (the kernel waits for it with griddepcontrol.wait)
 template <typename... Args>
-int launch_chained(void (*kernel)(Args...), int grid, int block, cudaStream_t s,
+int launch_chained(void (*kernel)(Args...), int grid, int block, size_t smem, cudaStream_t s,
                    const Args &...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -693,13 +1131,12 @@ int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cu
 
 template <typename T>
 int launch_patch_pattern(int mode, const int *ids, const DevOp<T> &op, int n, const int *which,
-                         void *patterns, const int *pattern, unsigned long long *hash, int *bad,
-                         cudaStream_t s) {
+                         void *patterns, unsigned long long *hash, int *bad, cudaStream_t s) {
   if (n <= 0) return 0;
   PatchPattern *p = static_cast<PatchPattern *>(patterns);
   auto run = [&](auto kernel) {
     kernel<<<n, 256, 0, s>>>(ids, op.a_rowptr, op.a_col, op.b_rowptr, op.b_col, op.bt_rowptr,
-                             op.bt_col, op.nact, which, p, pattern, hash, bad);
+                             op.bt_col, op.nact, which, p, hash, bad);
   };
   if (mode == 0)
     run(k_patch_pattern<0>);
@@ -710,6 +1147,103 @@ int launch_patch_pattern(int mode, const int *ids, const DevOp<T> &op, int n, co
   return ok();
 }
 
+// Places of a pattern's nodes: greedy over the nodes in list order, each into
+// the bank group (place % 8) where the fewest lanes of a row's octets meet,
+// then a pass of improving exchanges (1.7 ms; 533 -> 394 wavefronts for the
+// 288 octets of an inner cell, more passes 386); place kZeroSlot stays the zero's.
+void patch_places(void *patterns, long long count) {
+  PatchPattern *P = static_cast<PatchPattern *>(patterns);
+#pragma omp parallel for schedule(dynamic)
+  for (long long c = 0; c < count; ++c) {
+    PatchPattern &pt = P[c];
+    constexpr int N = kPatchNodes, OCT = 28 * 16;
+    std::vector<std::vector<int>> octets(N);  // octets (row, entry number) that read a node
+    for (int r = 0; r < 28; ++r)
+      for (int q = 0; q < 16; ++q)
+        for (int l = 0; l < 8; ++l) {
+          const int node = pt.slot[8 * r + l][q] / 16;
+          if (node < N) octets[node].push_back(16 * r + q);
+        }
+    std::vector<int> group(N, -1), used(8, 0);
+    std::vector<std::array<uint8_t, 8>> cnt(OCT);
+    for (auto &o : cnt) o.fill(0);
+    const int room[8] = {43, 43, 43, 43, 43, 43, 43, 42};  // places of a group (343 in all)
+    auto cost = [&](int node, int g) {
+      int s = 0;
+      for (int o : octets[node]) s += cnt[o][g];
+      return s;
+    };
+    auto put = [&](int node, int g, int d) {
+      for (int o : octets[node]) cnt[o][g] = (uint8_t)(cnt[o][g] + d);
+      used[g] += d;
+    };
+    int at = 0;
+    for (int n = 0; n < N; ++n) {
+      int best = -1, bc = 0;
+      for (int q = 0; q < 8; ++q) {
+        const int g = (at + q) & 7;
+        if (used[g] >= room[g]) continue;
+        const int k = cost(n, g);
+        if (best < 0 || k < bc) {
+          best = g;
+          bc = k;
+        }
+      }
+      group[n] = best;
+      put(n, best, 1);
+      at = best + 1;
+    }
+    for (int n = 0; n < N; ++n) {
+      const int g = group[n];
+      put(n, g, -1);
+      const int own = cost(n, g);
+      int gain = 0, with = -1;
+      for (int m = 0; own > 0 && m < N; ++m) {
+        const int h = group[m];
+        if (m == n || h == g) continue;
+        put(m, h, -1);
+        const int before = own + cost(m, h), after = cost(n, h) + cost(m, g);
+        put(m, h, 1);
+        if (before - after > gain) {
+          gain = before - after;
+          with = m;
+        }
+      }
+      if (with >= 0) {
+        put(with, group[with], -1);
+        group[n] = group[with];
+        group[with] = g;
+        put(with, g, 1);
+      }
+      put(n, group[n], 1);
+    }
+    int next[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint16_t place[N + 1];
+    for (int n = 0; n < N; ++n) place[n] = (uint16_t)(8 * next[group[n]]++ + group[n]);
+    place[N] = (uint16_t)N;
+    for (auto &lane : pt.slot)
+      for (uint16_t &e : lane) e = (uint16_t)(16 * place[e / 16]);
+    for (uint16_t &e : pt.own) e = (uint16_t)(16 * place[e / 16]);
+    for (int n = 0; n <= N; ++n) pt.place[n] = place[n];
+  }
+}
+
+int launch_patch_assign(int *ids, const int *pattern, int ncells, cudaStream_t s) {
+  if (ncells <= 0) return 0;
+  k_patch_assign<<<(ncells + 255) / 256, 256, 0, s>>>(ids, pattern, ncells);
+  return ok();
+}
+
+int launch_patch_init() {
+  auto set = [](auto kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
+           cudaSuccess;
+  };
+  return set(k_patch_sweep32, sizeof(Smem32)) && set(k_patch_sweep64, sizeof(Smem64))
+             ? 0
+             : -1;
+}
+
 template <typename T>
 int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb, int np,
                        cudaStream_t s) {
@@ -718,36 +1252,41 @@ int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb,
 }
 
 template <typename T>
-int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors,
-                        const T *rhs, T damp, int odd, cudaStream_t s) {
+int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors, T damp,
+                        int odd, int *err, int num_sms, cudaStream_t s) {
   if (n <= 0) return 0;
-  return launch_chained<PatchLevel<T>, const int *, const T *, const T *, T, int>(
-      k_patch_sweep<T>, n, kPatchThreads, s, L, list, factors, rhs, damp, odd);
+  if constexpr (sizeof(T) == 4)
+    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *>(
+        k_patch_sweep32, std::min(n, kCtas32 * num_sms), kPatchThreads, sizeof(Smem32), s, L, list,
+        n, factors, damp, odd, err);
+  else
+    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *>(
+        k_patch_sweep64, std::min(n, kCtas64 * num_sms), kPatchThreads, sizeof(Smem64), s, L, list,
+        n, factors, damp, odd, err);
 }
 
 template <typename T>
 int launch_patch_between(const PatchLevel<T> &L, const T *rhs, int hb, cudaStream_t s) {
   if (hb >= L.nu) return 0;
   return launch_chained<PatchLevel<T>, const T *, int>(k_patch_dirichlet<T>, node_grid(L.nu - hb),
-                                                       256, s, L, rhs, hb);
+                                                       256, 0, s, L, rhs, hb);
 }
 
 template <typename T>
 int launch_patch_end(const PatchLevel<T> &L, T *u, const T *rhs, int hb, int np, int odd,
                      cudaStream_t s) {
   return launch_chained<PatchLevel<T>, T *, const T *, int, int, int>(
-      k_patch_unpack_u<T>, node_grid(std::max(L.nu, np)), 256, s, L, u, rhs, hb, np, odd);
+      k_patch_unpack_u<T>, node_grid(std::max(L.nu, np)), 256, 0, s, L, u, rhs, hb, np, odd);
 }
 
 #define PM_PINST(T)                                                                               \
   template int launch_patch_pack<T>(const PatchLevel<T> &, const DevOp<T> &, int, cudaStream_t);  \
   template int launch_patch_pattern<T>(int, const int *, const DevOp<T> &, int, const int *,      \
-                                       void *, const int *, unsigned long long *, int *,          \
-                                       cudaStream_t);                                             \
+                                       void *, unsigned long long *, int *, cudaStream_t);        \
   template int launch_patch_begin<T>(const PatchLevel<T> &, const T *, const T *, int, int,       \
                                      cudaStream_t);                                               \
   template int launch_patch_colour<T>(const PatchLevel<T> &, const int *, int, const T *,         \
-                                      const T *, T, int, cudaStream_t);                           \
+                                      T, int, int *, int, cudaStream_t);                          \
   template int launch_patch_between<T>(const PatchLevel<T> &, const T *, int, cudaStream_t);      \
   template int launch_patch_end<T>(const PatchLevel<T> &, T *, const T *, int, int, int,          \
                                    cudaStream_t);

@@ -20,6 +20,7 @@
 
 #include <cstdint>
 
+#include "pm_bulk.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -31,55 +32,6 @@ constexpr int kTmaWarps = 3;
 constexpr int kCellBytes = kFacStride * (int)sizeof(float);  // 28,912
 static_assert(kCellBytes % 16 == 0, "bulk copies move multiples of 16 bytes");
 constexpr size_t kTmaSmem = (size_t)kTmaWarps * 2 * kCellBytes;  // 173,472
-constexpr long long kMaxPolls = 1ll << 22;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
-               : "memory");
-}
-
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// one thread: arm the barrier for `bytes` and start the copy global -> shared
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
-                                          uint64_t *bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Bounded wait by the whole warp (at most `polls` non-blocking tests); true
-// when the phase completed.  The result is warp-uniform (every lane has
-// observed the completion itself, so every lane's later shared-memory reads
-// are ordered after the copy).
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long long polls) {
-  for (long long it = 0; it < polls; ++it)
-    if (__all_sync(kFull, mbar_test_wait(bar, parity))) return true;
-  return false;
-}
 
 __device__ __forceinline__ void scatter_cell(int i, float v, const int *ud, const int *pd, int nu,
                                              float *u) {
