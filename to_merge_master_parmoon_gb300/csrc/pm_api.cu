@@ -75,6 +75,7 @@ struct LevelDev {
   int nl = NU_LOC;                // velocity nodes per cell (27 Q2, 15 P2+bubble tetrahedra)
   HostCsr h_pu, h_pp;             // handed-over prolongation from the next coarser level
   bool has_colour = false;
+  int *rows = nullptr;  // order of the velocity rows in defects and mat-vecs
   int *a_rowptr = nullptr, *a_col = nullptr, *b_rowptr = nullptr, *b_col = nullptr;
   int *bt_rowptr = nullptr, *bt_col = nullptr;
   double *a64[9] = {}, *b64[3] = {}, *bt64[3] = {};
@@ -155,6 +156,7 @@ DevOp<double> LevelDev::op<double>() const {
   o.diag = diag == 1;
   o.np = np;
   o.nact = nact;
+  o.rows = rows;
   o.a_rowptr = a_rowptr;
   o.a_col = a_col;
   for (int k = 0; k < 9; ++k) o.a[k] = a64[k];
@@ -177,6 +179,7 @@ DevOp<float> LevelDev::op<float>() const {
   o.diag = diag == 1;
   o.np = np;
   o.nact = nact;
+  o.rows = rows;
   o.a_rowptr = a_rowptr;
   o.a_col = a_col;
   for (int k = 0; k < 9; ++k) o.a[k] = a32[k];
@@ -412,12 +415,16 @@ PatchLevel<T> patch_level(const pm_handle *h, const LevelDev &Lv) {
 }
 
 // `sweeps` sweeps from the packed rows (one launch per colour), with the
-// Dirichlet nodes set before, between and after them as vanka_sweep does
+// Dirichlet nodes set before, between and after them as vanka_sweep does.
+// zero_start: u is zero on entry, whatever it holds; zero_end: zero on the
+// Dirichlet nodes at the end
 template <typename T>
-pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps) {
+pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps,
+                       bool zero_start = false, bool zero_end = false) {
   const PatchLevel<T> L = patch_level<T>(h, Lv);
   const int ncol = (int)Lv.colouring.ptr.size() - 1;
-  PM_LAUNCH(launch_patch_begin<T>(L, u, rhs, Lv.hb, Lv.np, h->stream));
+  PM_LAUNCH(launch_patch_begin<T>(L, zero_start ? (const T *)nullptr : u, rhs, Lv.hb, Lv.np,
+                                  h->stream));
   for (int s = 0; s < sweeps; ++s) {
     if (s > 0) PM_LAUNCH(launch_patch_between<T>(L, rhs, Lv.hb, h->stream));
     for (int k = 0; k < ncol; ++k) {
@@ -437,7 +444,8 @@ pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweep
       }
     }
   }
-  PM_LAUNCH(launch_patch_end<T>(L, u, rhs, Lv.hb, Lv.np, sweeps & 1, h->stream));
+  PM_LAUNCH(launch_patch_end<T>(L, u, zero_end ? (const T *)nullptr : rhs, Lv.hb, Lv.np,
+                                sweeps & 1, h->stream));
   return PM_OK;
 }
 
@@ -526,11 +534,19 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
   return PM_OK;
 }
 
+// zero_start / zero_end as for patch_sweeps
 template <typename T>
-pm_status smooth(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps) {
+pm_status smooth(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweeps,
+                 bool zero_start = false, bool zero_end = false) {
   if (sweeps > 0 && Lv.packed() && std::fabs(1.0 - h->opt.alpha) <= 1e-3)
-    return patch_sweeps<T>(h, Lv, u, rhs, sweeps);
+    return patch_sweeps<T>(h, Lv, u, rhs, sweeps, zero_start, zero_end);
+  if (zero_start) {
+    PM_LAUNCH(launch_fill<T>(u, T(0), Lv.ndof, h->stream));
+    PM_LAUNCH(launch_dirichlet<T>(u, rhs, Lv.nu, Lv.hb, Lv.ndir, h->stream));
+  }
   for (int s = 0; s < sweeps; ++s) PM_TRY(vanka_sweep<T>(h, Lv, u, rhs));
+  if (zero_end)
+    PM_LAUNCH(launch_dirichlet<T>(u, (const T *)nullptr, Lv.nu, Lv.hb, Lv.ndir, h->stream));
   return PM_OK;
 }
 
@@ -610,33 +626,38 @@ pm_status learned_step(pm_handle *h, LevelDev &C, T *u, const T *f) {
   return PM_OK;
 }
 
-// TNSE_MultiGrid::Cycle (V-cycle, cell Vanka, coarse SolveExact)
+// TNSE_MultiGrid::Cycle (V-cycle, cell Vanka, coarse SolveExact) from a zero
+// start with the Dirichlet nodes set (CorrectNodes, SetDirichletNodes).
+// Between the sweeps a level takes five launches: defect, the mean of its
+// pressure, restriction, projection, prolongation with the update; fifteen
+// with one kernel per step took a tenth of a V-cycle on small problems.
 template <typename T>
 pm_status cycle(pm_handle *h, int i) {
   LevelDev &C = h->L[i];
   T *u = static_cast<T *>(C.sol), *f = static_cast<T *>(C.rhs);
-  // CorrectNodes + SetDirichletNodes
-  PM_LAUNCH(launch_dirichlet<T>(u, f, C.nu, C.hb, C.ndir, h->stream));
   if (i == 0) return coarse_solve<T>(h, C, f, u);
   LevelDev &K = h->L[i - 1];
   T *d = static_cast<T *>(C.def);
   T *cu = static_cast<T *>(K.sol), *cf = static_cast<T *>(K.rhs);
-  PM_TRY(smooth<T>(h, C, u, f, h->opt.pre_smooth));
-  PM_LAUNCH(launch_dirichlet<T>(u, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
-  PM_TRY(level_defect<T>(h, C, u, f, d));
-  // DefectRestriction (u and p) + CorrectDefect + Reset
-  PM_LAUNCH(launch_csr_apply<T>(C.Ru.view<T>(), 3, d, C.nu, cf, K.nu, h->stream));
-  PM_LAUNCH(launch_csr_apply<T>(C.Rp.view<T>(), 1, d + 3 * C.nu, C.np, cf + 3 * K.nu, K.np, h->stream));
-  PM_LAUNCH(launch_zero_nonactive<T>(cf, K.nu, K.nact, h->stream));
+  PM_TRY(smooth<T>(h, C, u, f, h->opt.pre_smooth, true, true));
+  PM_LAUNCH(launch_coupled<T>(C.op<T>(), u, f, d, true, true, h->stream));
+  // L2_0 of the defect's pressure: its mean is removed in the restriction;
+  // stacked systems project each system's block in place
+  const double *mean = nullptr;
+  if (h->nsys > 1) {
+    PM_TRY(l20<T>(h, d + 3 * C.nu, C.np));
+  } else if (h->opt.project_pressure) {
+    double *m = h->partials + 8 * 152;
+    PM_LAUNCH(launch_l20_mean<T>(d + 3 * C.nu, C.np, h->partials, h->counter, m, h->stream));
+    mean = m;
+  }
+  // DefectRestriction (u and p) + CorrectDefect
+  PM_LAUNCH(launch_restrict<T>(C.Ru.view<T>(), C.Rp.view<T>(), d, cf, K.nact, mean, h->stream));
   PM_TRY(l20<T>(h, cf + 3 * K.nu, K.np));
-  PM_LAUNCH(launch_fill<T>(cu, T(0), K.ndof, h->stream));
   PM_TRY(cycle<T>(h, i - 1));
   // Prolongate, CorrectNodes(defect), Update, CorrectNodes(u)
-  PM_LAUNCH(launch_csr_apply<T>(C.Pu.view<T>(), 3, cu, K.nu, d, C.nu, h->stream));
-  PM_LAUNCH(launch_csr_apply<T>(C.Pp.view<T>(), 1, cu + 3 * K.nu, K.np, d + 3 * C.nu, C.np, h->stream));
-  PM_LAUNCH(launch_dirichlet<T>(d, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
-  PM_LAUNCH(launch_axpy<T>(u, (T)h->opt.beta, d, C.ndof, h->stream));
-  PM_LAUNCH(launch_dirichlet<T>(u, (const T *)nullptr, C.nu, C.hb, C.ndir, h->stream));
+  PM_LAUNCH(launch_prolongate<T>(C.Pu.view<T>(), C.Pp.view<T>(), cu, u, C.hb, (T)h->opt.beta,
+                                 h->stream));
   PM_TRY(smooth<T>(h, C, u, f, h->opt.post_smooth));
   if (h->l_active &&
       (h->opt.learned_levels <= 0 || i >= (int)h->L.size() - h->opt.learned_levels))
@@ -644,14 +665,9 @@ pm_status cycle(pm_handle *h, int i) {
   return PM_OK;
 }
 
-// TMultiGridIte::Iterate body after rhs is in place: zero start,
-// SetDirichletNodes, one cycle.
+// TMultiGridIte::Iterate body after rhs is in place
 template <typename T>
 pm_status vcycle_core(pm_handle *h) {
-  LevelDev &F = h->L.back();
-  PM_LAUNCH(launch_fill<T>(static_cast<T *>(F.sol), T(0), F.ndof, h->stream));
-  PM_LAUNCH(launch_dirichlet<T>(static_cast<T *>(F.sol), static_cast<const T *>(F.rhs), F.nu, F.hb,
-                                F.ndir, h->stream));
   return cycle<T>(h, (int)h->L.size() - 1);
 }
 
@@ -1838,6 +1854,9 @@ pm_status pm_add_level(pm_handle *h, const pm_level_desc *d) {
   Lv.pattern_key = pattern_fingerprint(d);
   Lv.has_colour = d->cell_colour != nullptr;
   if (Lv.has_colour) Lv.h_colour.assign(d->cell_colour, d->cell_colour + Lv.ncells);
+  std::vector<int> order;
+  row_order(d->a_rowptr, Lv.nu, order);
+  PM_TRY(upload(h, &Lv.rows, order.data(), order.size()));
   PM_TRY(upload(h, &Lv.a_rowptr, d->a_rowptr, (size_t)Lv.nu + 1));
   PM_TRY(upload_padded(h, &Lv.a_col, d->a_col, (size_t)Lv.a_nnz));
   PM_TRY(upload(h, &Lv.b_rowptr, d->b_rowptr, (size_t)Lv.np + 1));

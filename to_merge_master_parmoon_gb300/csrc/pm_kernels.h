@@ -46,6 +46,7 @@ struct DevOp {
   // upload); the sweeps read only ad[0..2] = A11, A22, A33.  (A nine-block
   // level whose diagonal blocks are also identical runs with structured = 1.)
   int diag;
+  const int *rows;  // order in which defects and mat-vecs take the velocity rows (or nullptr)
   const int *a_rowptr, *a_col;
   const T *a[9];
   const T *ad[3];
@@ -89,6 +90,18 @@ int launch_csr_apply(const DevCsr<T> &m, int ncomp, const T *x, int x_stride, T 
 // reset to zero by the last block.
 template <typename T>
 int launch_l20_project(T *p, int np, double *scratch, unsigned int *counter, cudaStream_t s);
+// the mean alone, left in *mean
+template <typename T>
+int launch_l20_mean(const T *p, int np, double *scratch, unsigned int *counter, double *mean,
+                    cudaStream_t s);
+// cf = R d (velocity and pressure; zero on velocity rows >= nact), with *mean
+// removed from d's pressure when given; u += beta P cu, zero on rows >= hb
+template <typename T>
+int launch_restrict(const DevCsr<T> &ru, const DevCsr<T> &rp, const T *d, T *cf, int nact,
+                    const double *mean, cudaStream_t s);
+template <typename T>
+int launch_prolongate(const DevCsr<T> &pu, const DevCsr<T> &pp, const T *cu, T *u, int hb, T beta,
+                      cudaStream_t s);
 int launch_dot(const double *a, const double *b, int n, double *partials, unsigned int *counter,
                double *result, cudaStream_t s);
 // w -= h[k_axpy]*v_axpy (if v_axpy), then result = <w, v_dot> (if v_dot) or
@@ -113,8 +126,6 @@ int launch_axpy(T *y, T a, const T *x, int n, cudaStream_t s);
 template <typename T>
 int launch_dirichlet(T *u, const T *src, int nu, int hb, int ndir, cudaStream_t s);
 // zero velocity rows >= nact of the three components
-template <typename T>
-int launch_zero_nonactive(T *v, int nu, int nact, cudaStream_t s);
 // u = uold + alpha (u - uold)
 template <typename T>
 int launch_relax(T *u, const T *uold, T alpha, int n, cudaStream_t s);
@@ -235,9 +246,10 @@ int launch_patch_assign(int *ids, const int *pattern, int ncells, cudaStream_t s
 void patch_places(void *host_patterns, long long count);
 int launch_patch_init();  // shared-memory limit of the sweep kernels
 // a run of sweeps: begin (u into the copies), every colour of every sweep,
-// between two sweeps the Dirichlet nodes, end (the copies into u).  odd: the
-// sweep's number & 1; for end the number of sweeps & 1.  Every launch but the
-// first may start early and waits for its predecessor on the device.
+// between two sweeps the Dirichlet nodes, end (the copies into u).  begin
+// without u starts from zero, end without rhs leaves zero on the Dirichlet
+// nodes.  odd: the
+// sweep's number & 1; for end the number of sweeps & 1.
 template <typename T>
 int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb, int np,
                        cudaStream_t s);
@@ -316,7 +328,7 @@ int launch_dense_lu(double *a, int n, int *ipiv, int *status, cudaStream_t s);
 // x = A^{-1} b with the factors (one CTA); b[first_p] = 0 when project.
 int launch_dense_solve(const double *lu, const int *ipiv, int n, const double *b, double *x,
                        int pin_row, cudaStream_t s);
-// A^{-1} (column-major) from the LU factors, one CTA per column.
+// A^{-1} (row-major) from the LU factors, one CTA per column.
 int launch_dense_inverse(const double *lu, const int *ipiv, int n, double *inv, cudaStream_t s);
 // x = A^{-1} b in FP64 arithmetic (b[pin_row] = 0 when pin_row >= 0).
 template <typename TB, typename TX>

@@ -488,6 +488,22 @@ bool stack_levels(const pm_level_desc *d, int G, const StackSizes &coarse, Stack
   return true;
 }
 
+void row_order(const int *rowptr, int rows, std::vector<int> &order) {
+  constexpr int kWindow = 4096, kClasses = 32;
+  order.resize((size_t)rows);
+#pragma omp parallel for schedule(static)
+  for (int w = 0; w < rows; w += kWindow) {
+    const int e = std::min(rows, w + kWindow);
+    int at[kClasses + 1] = {0};
+    auto cls = [&](int i) {  // longest first
+      return kClasses - 1 - std::min(kClasses - 1, (rowptr[i + 1] - rowptr[i] + 15) / 16);
+    };
+    for (int i = w; i < e; ++i) ++at[cls(i) + 1];
+    for (int c = 0; c < kClasses; ++c) at[c + 1] += at[c];
+    for (int i = w; i < e; ++i) order[(size_t)(w + at[cls(i)]++)] = i;
+  }
+}
+
 bool build_patches(int ncells, const int *udofs, const int *pdofs, int nu, int np,
                    const Colouring &col, std::vector<int> &ids,
                    std::vector<unsigned char> &flips) {

@@ -72,6 +72,10 @@ bool build_patches(int ncells, const int *udofs, const int *pdofs, int nu, int n
                    std::vector<unsigned char> &flips);
 constexpr int kPatchIdsHost = 400;  // kPatchIds
 
+// Rows of a CSR pattern by descending length class (16 entries) within
+// windows of 4096 rows, in their order otherwise.
+void row_order(const int *rowptr, int rows, std::vector<int> &order);
+
 // G level descriptors of one mesh (equal sizes, nnz and local DOF counts;
 // values and patterns may differ) stacked into one block-diagonal level:
 // velocity DOF i of system s goes to s*na + i if i < na (na = n_active),

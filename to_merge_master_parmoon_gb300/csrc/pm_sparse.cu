@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "pm_chain.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -140,21 +141,126 @@ __device__ __forceinline__ void rows8_sum(const int *__restrict__ col, const T *
   }
 }
 
+// Sums of the three components over the 8 lanes of a row, in lane 0.  FP32: a
+// butterfly each.  FP64, whose pipe takes half a lane per cycle and quarter
+// SM: six additions instead of nine, lanes 0..3 going on with component 1 and
+// lanes 4..7 with component 2.
+template <typename T>
+__device__ __forceinline__ void row_reduce(T (&s)[3]) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] = group_sum<8>(s[c]);
+  } else {
+    const bool high = threadIdx.x & 4;
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 4);
+    T d = (high ? s[2] : s[1]) + __shfl_xor_sync(0xffffffffu, high ? s[1] : s[2], 4);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    s[1] = d;
+    s[2] = __shfl_xor_sync(0xffffffffu, d, 4);
+  }
+}
+
+// Pressure rows q - B u (or B u), 16 lanes per row: entry j of a row belongs
+// to lane j % 16, a butterfly adds the lanes.  FP32: one row per 16 lanes.
+// FP64: four, whose butterflies share their additions (the lanes take a row
+// each as the strides shrink: 5 instead of 16 for eight rows of a warp, the
+// same sums), since the FP64 pipe bounds the kernel.
+template <typename T>
+constexpr int pressure_rows_per_group() {
+  return sizeof(T) == 4 ? 1 : 4;
+}
+template <typename T>
+__device__ __forceinline__ T pressure_part(const DevOp<T> &op, int i, int lane,
+                                           const T *__restrict__ u1, const T *__restrict__ u2,
+                                           const T *__restrict__ u3) {
+  T s = 0;
+  const int rs = op.b_rowptr[i], re = op.b_rowptr[i + 1];
+  for (int j = rs + lane; j < re; j += 16) {
+    const int c = __ldg(op.b_col + j);
+    if constexpr (sizeof(T) == 4) {
+      s += ld_stream(op.b[0] + j) * __ldg(u1 + c) + ld_stream(op.b[1] + j) * __ldg(u2 + c) +
+           ld_stream(op.b[2] + j) * __ldg(u3 + c);
+    } else {
+      s = __dadd_rn(s, __fma_rn(ld_stream(op.b[2] + j), __ldg(u3 + c),
+                                __fma_rn(ld_stream(op.b[0] + j), __ldg(u1 + c),
+                                         __dmul_rn(ld_stream(op.b[1] + j), __ldg(u2 + c)))));
+    }
+  }
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ void pressure_rows(const DevOp<T> &op, long long group,
+                                              const T *__restrict__ x, const T *__restrict__ b,
+                                              T *__restrict__ r, int defect) {
+  const int lane = threadIdx.x & 15, nu = op.nu;
+  const T *u1 = x, *u2 = x + nu, *u3 = x + 2 * nu;
+  long long row;
+  T s;
+  bool write;
+  if constexpr (sizeof(T) == 4) {
+    row = group;
+    s = row < op.np ? pressure_part<T>(op, (int)row, lane, u1, u2, u3) : T(0);
+    s = group_sum<16>(s);
+    write = lane == 0;
+  } else {
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long i = 4 * group + q;
+      v[q] = i < op.np ? pressure_part<T>(op, (int)i, lane, u1, u2, u3) : T(0);
+    }
+    const bool h8 = lane & 8, h4 = lane & 4;
+    const T a = (h8 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, h8 ? v[0] : v[1], 8);
+    const T c = (h8 ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, h8 ? v[2] : v[3], 8);
+    s = (h4 ? c : a) + __shfl_xor_sync(0xffffffffu, h4 ? a : c, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    row = 4 * group + (h8 ? 1 : 0) + (h4 ? 2 : 0);
+    write = (lane & 3) == 0;
+  }
+  if (write && row < op.np) r[3 * (size_t)nu + row] = defect ? b[3 * (size_t)nu + row] - s : s;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_pressure(DevOp<T> op, const T *__restrict__ x,
+                                                     const T *__restrict__ b, T *__restrict__ r,
+                                                     int defect) {
+  wait_previous();
+  start_next();
+  pressure_rows<T>(op, ((long long)blockIdx.x * kBlock + threadIdx.x) >> 4, x, b, r, defect);
+}
+
+// Coupled defect or mat-vec: blocks 0 .. vblocks - 1 the velocity rows, the
+// others the pressure rows.  FP64 takes the velocity rows in the level's row
+// order (op.rows: by stencil size within windows), so that the four rows of a
+// warp are equally long: in the order of the numbering a warp held vertex and
+// edge rows side by side and held the FP64 pipe as long as its longest (64^3:
+// 1.53 -> 1.29 ms).  FP32, bound by its gathers, loses locality by it (0.42
+// -> 0.51 ms) and keeps the numbering.
 // KIND 0: nine A blocks; 1: one A block for the three components; 2: the
 // three diagonal blocks only (A12..A32 zero on the level)
 template <typename T, int VEC, int KIND, int UR>
-__global__ void __launch_bounds__(kBlock) k_coupled_velocity8(DevOp<T> op, const T *__restrict__ x,
-                                                              const T *__restrict__ b,
-                                                              T *__restrict__ r, int defect,
-                                                              int zero_nonactive) {
+__global__ void __launch_bounds__(kBlock) k_coupled(DevOp<T> op, const T *__restrict__ x,
+                                                    const T *__restrict__ b, T *__restrict__ r,
+                                                    int defect, int zero_nonactive, int vblocks) {
   // BT rows (at most 32 entries on hexahedra): one load round trip
   constexpr int URB = (16 / (int)sizeof(T)) / VEC > 1 ? (16 / (int)sizeof(T)) / VEC : 1;
+  wait_previous();
+  start_next();
+  if ((int)blockIdx.x >= vblocks) {
+    pressure_rows<T>(op, ((long long)(blockIdx.x - vblocks) * kBlock + threadIdx.x) >> 4, x, b, r,
+                     defect);
+    return;
+  }
   // no early return before the group shuffles: every lane of the warp joins
   const int sl = threadIdx.x & 7;
   const long long row = ((long long)blockIdx.x * kBlock + threadIdx.x) >> 3;
   const int nu = op.nu;
   const bool valid = row < nu;
-  const int i = valid ? (int)row : 0;
+  const int i = valid ? (sizeof(T) == 8 && op.rows ? __ldg(op.rows + row) : (int)row) : 0;
   const bool skip = !valid || (zero_nonactive && i >= op.nact);
   const T *u1 = x, *u2 = x + nu, *u3 = x + 2 * nu, *p = x + 3 * nu;
   T s[3] = {T(0), T(0), T(0)};
@@ -169,8 +275,7 @@ __global__ void __launch_bounds__(kBlock) k_coupled_velocity8(DevOp<T> op, const
       rows8_sum<T, VEC, 3, URB>(op.bt_col, op.bt, op.bt_rowptr[i], op.bt_rowptr[i + 1], sl, p, p,
                                 p, s);
   }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) s[c] = group_sum<8>(s[c]);
+  row_reduce<T>(s);
   if (valid && sl == 0) {
     if (skip) {
       r[i] = r[nu + i] = r[2 * nu + i] = T(0);
@@ -184,30 +289,6 @@ __global__ void __launch_bounds__(kBlock) k_coupled_velocity8(DevOp<T> op, const
       r[2 * nu + i] = s[2];
     }
   }
-}
-
-// Pressure rows q - B u (or B u): G lanes per row.
-template <typename T, int G>
-__global__ void __launch_bounds__(kBlock) k_coupled_pressure(DevOp<T> op, const T *__restrict__ x,
-                                                             const T *__restrict__ b,
-                                                             T *__restrict__ r, int defect) {
-  const int lane = threadIdx.x & (G - 1);
-  const long long row = ((long long)blockIdx.x * kBlock + threadIdx.x) / G;
-  const bool valid = row < op.np;
-  const int nu = op.nu;
-  const int i = valid ? (int)row : 0;
-  const T *u1 = x, *u2 = x + nu, *u3 = x + 2 * nu;
-  T s = 0;
-  if (valid) {
-    const int rs = op.b_rowptr[i], re = op.b_rowptr[i + 1];
-    for (int j = rs + lane; j < re; j += G) {
-      const int c = __ldg(op.b_col + j);
-      s += ld_stream(op.b[0] + j) * __ldg(u1 + c) + ld_stream(op.b[1] + j) * __ldg(u2 + c) +
-           ld_stream(op.b[2] + j) * __ldg(u3 + c);
-    }
-  }
-  s = group_sum<G>(s);
-  if (valid && lane == 0) r[3 * nu + i] = defect ? b[3 * nu + i] - s : s;
 }
 
 // y_k = M x_k for NC components (transfers): G lanes per row.
@@ -236,6 +317,97 @@ __global__ void __launch_bounds__(kBlock) k_csr_apply(DevCsr<T> m, const T *__re
     T t = group_sum<G>(s[k]);
     if (valid && lane == 0) y[(size_t)k * y_stride + i] = t;
   }
+}
+
+// One row of a transfer for NC components by G lanes, as k_csr_apply; `mean`
+// (or nullptr) is subtracted from the constant pressure modes (every fourth
+// entry) of x as k_l20_sub does.
+template <typename T, int G, int NC>
+__device__ __forceinline__ void csr_row(const DevCsr<T> &m, int i, bool valid,
+                                        const T *__restrict__ x, int x_stride, bool sub, T mean,
+                                        T (&s)[NC]) {
+  const int lane = threadIdx.x & (G - 1);
+#pragma unroll
+  for (int k = 0; k < NC; ++k) s[k] = 0;
+  if (valid) {
+    const int rs = m.rowptr[i], re = m.rowptr[i + 1];
+    for (int j = rs + lane; j < re; j += G) {
+      const int c = __ldg(m.col + j);
+      const T v = __ldg(m.val + j);
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        T xv = __ldg(x + (size_t)k * x_stride + c);
+        if (sub && (c & 3) == 0) xv -= mean;
+        s[k] += v * xv;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NC; ++k) s[k] = group_sum<G>(s[k]);
+}
+
+// DefectRestriction of both parts and CorrectDefect in one launch: cf = R d,
+// zero on the non-active velocity rows; the mean of d's pressure is removed
+// on the way (mean: device scalar or nullptr).
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_restrict(DevCsr<T> ru, DevCsr<T> rp,
+                                                     const T *__restrict__ d, T *__restrict__ cf,
+                                                     int nact, const double *mean, int vblocks) {
+  wait_previous();
+  start_next();
+  const bool lead = (threadIdx.x & 7) == 0;
+  if ((int)blockIdx.x < vblocks) {
+    const long long row = ((long long)blockIdx.x * kBlock + threadIdx.x) >> 3;
+    const bool valid = row < ru.rows;
+    const int i = valid ? (int)row : 0;
+    T s[3];
+    csr_row<T, 8, 3>(ru, i, valid && i < nact, d, ru.cols, false, T(0), s);
+    if (valid && lead) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) cf[(size_t)k * ru.rows + i] = i < nact ? s[k] : T(0);
+    }
+    return;
+  }
+  const long long row = ((long long)(blockIdx.x - vblocks) * kBlock + threadIdx.x) >> 3;
+  const bool valid = row < rp.rows;
+  T s[1];
+  csr_row<T, 8, 1>(rp, valid ? (int)row : 0, valid, d + (size_t)3 * ru.cols, 0, mean != nullptr,
+                   mean ? (T)*mean : T(0), s);
+  if (valid && lead) cf[(size_t)3 * ru.rows + row] = s[0];
+}
+
+// Prolongate of both parts and Update in one launch: u += beta P cu on the
+// active velocity rows and the pressure, u = 0 on the Dirichlet rows (from hb)
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_prolongate(DevCsr<T> pu, DevCsr<T> pp,
+                                                       const T *__restrict__ cu, T *__restrict__ u,
+                                                       int hb, T beta, int vblocks) {
+  wait_previous();
+  start_next();
+  const bool lead = (threadIdx.x & 7) == 0;
+  if ((int)blockIdx.x < vblocks) {
+    const long long row = ((long long)blockIdx.x * kBlock + threadIdx.x) >> 3;
+    const bool valid = row < pu.rows;
+    const int i = valid ? (int)row : 0;
+    T s[3];
+    csr_row<T, 8, 3>(pu, i, valid && i < hb, cu, pu.cols, false, T(0), s);
+    if (valid && lead) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        T *v = u + (size_t)k * pu.rows + i;
+        if (i < hb)
+          *v += beta * s[k];
+        else
+          *v = T(0);
+      }
+    }
+    return;
+  }
+  const long long row = ((long long)(blockIdx.x - vblocks) * kBlock + threadIdx.x) >> 3;
+  const bool valid = row < pp.rows;
+  T s[1];
+  csr_row<T, 8, 1>(pp, valid ? (int)row : 0, valid, cu + (size_t)3 * pu.cols, 0, false, T(0), s);
+  if (valid && lead) u[(size_t)3 * pu.rows + row] += beta * s[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -280,9 +452,32 @@ __device__ __forceinline__ void final_reduce(const double *partials, int n, doub
   }
 }
 
+// mean of the constant modes of a short vector by one block, subtracted from
+// them (sub) and left in *mean
+template <typename T>
+__global__ void __launch_bounds__(1024) k_l20_small(T *__restrict__ p, int np, double *mean,
+                                                    int sub) {
+  __shared__ double sh[32];
+  wait_previous();
+  start_next();
+  double s = 0;
+  for (int i = threadIdx.x * 4; i < np; i += 4096) s += (double)p[i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = warp_sum(sh[threadIdx.x & 31]) * (4.0 / (double)np);
+  if (threadIdx.x == 0) *mean = s;
+  if (!sub) return;
+  const T m = (T)s;
+  for (int i = threadIdx.x * 4; i < np; i += 4096) p[i] -= m;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_l20_sum(const T *__restrict__ p, int np,
-                                                    double *partials, unsigned int *counter) {
+                                                    double *partials, unsigned int *counter,
+                                                    double *mean) {
+  wait_previous();
+  start_next();
   double s = 0;
   for (int i = (blockIdx.x * kBlock + threadIdx.x) * 4; i < np; i += gridDim.x * kBlock * 4)
     s += (double)p[i];
@@ -290,12 +485,14 @@ __global__ void __launch_bounds__(kBlock) k_l20_sum(const T *__restrict__ p, int
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
   if (last_block_done(counter)) {
     // mean of the constant modes: s / np * 4 (IntoL20Vector3D, case -11)
-    final_reduce(partials, gridDim.x, partials + gridDim.x, counter, 4.0 / (double)np, false);
+    final_reduce(partials, gridDim.x, mean, counter, 4.0 / (double)np, false);
   }
 }
 
 template <typename T>
 __global__ void k_l20_sub(T *p, int np, const double *mean) {
+  wait_previous();
+  start_next();
   const T m = (T)(*mean);
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4; i < np; i += gridDim.x * blockDim.x * 4)
     p[i] -= m;
@@ -376,14 +573,6 @@ __global__ void k_dirichlet(T *u, const T *src, int nu, int hb, int ndir) {
   if (t >= 3 * ndir) return;
   const int c = t / ndir, i = hb + t % ndir;
   u[(size_t)c * nu + i] = src ? src[(size_t)c * nu + i] : T(0);
-}
-
-template <typename T>
-__global__ void k_zero_nonactive(T *v, int nu, int nact) {
-  const int m = nu - nact;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * m) return;
-  v[(size_t)(t / m) * nu + nact + t % m] = T(0);
 }
 
 template <typename T>
@@ -476,33 +665,56 @@ inline int ok() { return cudaPeekAtLastError() == cudaSuccess ? 1 : -1; }
 template <typename T>
 int launch_coupled(const DevOp<T> &op, const T *x, const T *b, T *r, bool defect,
                    bool zero_nonactive, cudaStream_t s) {
-  constexpr int GP = 16;
   constexpr int VEC = sizeof(T) == 4 ? 4 : 2;
-  const unsigned gv = grid_for((long long)op.nu * 8);
+  const int vb = grid_for((long long)op.nu * 8),
+            pb = grid_for((op.np + pressure_rows_per_group<T>() - 1LL) /
+                          pressure_rows_per_group<T>() * 16);
+  // One launch for both parts where launches count; from kSplitRows rows on
+  // the pressure rows run faster in a kernel of their own, with its smaller
+  // register count (64^3: the merged launch cost 0.5 ms per FP64 mat-vec)
+  constexpr int kSplitRows = 100000;
+  const bool split = op.nu >= kSplitRows;
+  if ((long long)vb + pb > 2147483647LL) return -1;
+  auto run = [&](auto kernel) {
+    int n = launch_chained<DevOp<T>, const T *, const T *, T *, int, int, int>(
+        kernel, dim3((unsigned)(split ? vb : vb + pb)), kBlock, 0, s, op, x, b, r, defect ? 1 : 0,
+        zero_nonactive ? 1 : 0, vb);
+    if (n < 0 || !split) return n;
+    n = launch_chained<DevOp<T>, const T *, const T *, T *, int>(
+        k_pressure<T>, dim3((unsigned)pb), kBlock, 0, s, op, x, b, r, defect ? 1 : 0);
+    return n < 0 ? -1 : 2;
+  };
   if (op.structured) {
     // FP32: scalar entries, the 8 lanes of a row gathering consecutive
     // columns (fewer cache lines per gather instruction than vectors of 4)
     if constexpr (sizeof(T) == 4)
-      k_coupled_velocity8<T, 1, 1, 8><<<gv, kBlock, 0, s>>>(op, x, b, r, defect ? 1 : 0,
-                                                           zero_nonactive ? 1 : 0);
+      return run(k_coupled<T, 1, 1, 8>);
     else
-      k_coupled_velocity8<T, VEC, 1, 2><<<gv, kBlock, 0, s>>>(op, x, b, r, defect ? 1 : 0,
-                                                             zero_nonactive ? 1 : 0);
-  } else if (op.diag) {
-    if constexpr (sizeof(T) == 4)
-      k_coupled_velocity8<T, 1, 2, 8><<<gv, kBlock, 0, s>>>(op, x, b, r, defect ? 1 : 0,
-                                                           zero_nonactive ? 1 : 0);
-    else
-      k_coupled_velocity8<T, VEC, 2, 2><<<gv, kBlock, 0, s>>>(op, x, b, r, defect ? 1 : 0,
-                                                             zero_nonactive ? 1 : 0);
-  } else {
-    k_coupled_velocity8<T, VEC, 0, 1><<<gv, kBlock, 0, s>>>(op, x, b, r, defect ? 1 : 0,
-                                                           zero_nonactive ? 1 : 0);
+      return run(k_coupled<T, VEC, 1, 2>);
   }
-  if (ok() < 0) return -1;
-  k_coupled_pressure<T, GP><<<grid_for((long long)op.np * GP), kBlock, 0, s>>>(op, x, b, r,
-                                                                               defect ? 1 : 0);
-  return ok() < 0 ? -1 : 2;
+  if (op.diag) {
+    if constexpr (sizeof(T) == 4)
+      return run(k_coupled<T, 1, 2, 8>);
+    else
+      return run(k_coupled<T, VEC, 2, 2>);
+  }
+  return run(k_coupled<T, VEC, 0, 1>);
+}
+
+template <typename T>
+int launch_restrict(const DevCsr<T> &ru, const DevCsr<T> &rp, const T *d, T *cf, int nact,
+                    const double *mean, cudaStream_t s) {
+  const int vb = grid_for((long long)ru.rows * 8), pb = grid_for((long long)rp.rows * 8);
+  return launch_chained<DevCsr<T>, DevCsr<T>, const T *, T *, int, const double *, int>(
+      k_restrict<T>, dim3((unsigned)(vb + pb)), kBlock, 0, s, ru, rp, d, cf, nact, mean, vb);
+}
+
+template <typename T>
+int launch_prolongate(const DevCsr<T> &pu, const DevCsr<T> &pp, const T *cu, T *u, int hb, T beta,
+                      cudaStream_t s) {
+  const int vb = grid_for((long long)pu.rows * 8), pb = grid_for((long long)pp.rows * 8);
+  return launch_chained<DevCsr<T>, DevCsr<T>, const T *, T *, int, T, int>(
+      k_prolongate<T>, dim3((unsigned)(vb + pb)), kBlock, 0, s, pu, pp, cu, u, hb, beta, vb);
 }
 
 template <typename T>
@@ -519,13 +731,32 @@ int launch_csr_apply(const DevCsr<T> &m, int ncomp, const T *x, int x_stride, T 
   return ok() < 0 ? -1 : 1;
 }
 
+// One block for up to 2,048 cells (4 us instead of 6 + 3 for sum and
+// subtraction over the whole GPU; 9 us at 8,192), else a grid-wide sum.
+constexpr int kL20Small = 4 * 2048;
+template <typename T>
+int launch_l20_mean(const T *p, int np, double *scratch, unsigned int *counter, double *mean,
+                    cudaStream_t s) {
+  if (np <= kL20Small)
+    return launch_chained<T *, int, double *, int>(k_l20_small<T>, dim3(1), 1024, 0, s,
+                                                   const_cast<T *>(p), np, mean, 0);
+  return launch_chained<const T *, int, double *, unsigned int *, double *>(
+      k_l20_sum<T>, dim3(2 * 152), kBlock, 0, s, p, np, scratch, counter, mean);
+}
+
 template <typename T>
 int launch_l20_project(T *p, int np, double *scratch, unsigned int *counter, cudaStream_t s) {
   const int nb = 2 * 152;
-  k_l20_sum<T><<<nb, kBlock, 0, s>>>(p, np, scratch, counter);
-  if (ok() < 0) return -1;
-  k_l20_sub<T><<<stride_grid(np / 4 + 1), kBlock, 0, s>>>(p, np, scratch + nb);
-  return ok() < 0 ? -1 : 2;
+  double *mean = scratch + nb;
+  if (np <= kL20Small)
+    return launch_chained<T *, int, double *, int>(k_l20_small<T>, dim3(1), 1024, 0, s, p, np,
+                                                   mean, 1);
+  if (launch_l20_mean<T>(p, np, scratch, counter, mean, s) < 0) return -1;
+  return launch_chained<T *, int, const double *>(k_l20_sub<T>,
+                                                  dim3((unsigned)stride_grid(np / 4 + 1)), kBlock,
+                                                  0, s, p, np, mean) < 0
+             ? -1
+             : 2;
 }
 
 int launch_dot(const double *a, const double *b, int n, double *partials, unsigned int *counter,
@@ -577,12 +808,6 @@ int launch_dirichlet(T *u, const T *src, int nu, int hb, int ndir, cudaStream_t 
   return ok() < 0 ? -1 : 1;
 }
 template <typename T>
-int launch_zero_nonactive(T *v, int nu, int nact, cudaStream_t s) {
-  if (nu <= nact) return 0;
-  k_zero_nonactive<T><<<grid_for(3LL * (nu - nact)), kBlock, 0, s>>>(v, nu, nact);
-  return ok() < 0 ? -1 : 1;
-}
-template <typename T>
 int launch_relax(T *u, const T *uold, T alpha, int n, cudaStream_t s) {
   k_relax<T><<<stride_grid(n), kBlock, 0, s>>>(u, uold, alpha, n);
   return ok() < 0 ? -1 : 1;
@@ -627,10 +852,15 @@ int launch_check_finite(const double *x, int n, int *flag, cudaStream_t s) {
   template int launch_csr_apply<T>(const DevCsr<T> &, int, const T *, int, T *, int,              \
                                    cudaStream_t);                                                 \
   template int launch_l20_project<T>(T *, int, double *, unsigned int *, cudaStream_t);           \
+  template int launch_l20_mean<T>(const T *, int, double *, unsigned int *, double *,             \
+                                  cudaStream_t);                                                  \
+  template int launch_restrict<T>(const DevCsr<T> &, const DevCsr<T> &, const T *, T *, int,      \
+                                  const double *, cudaStream_t);                                  \
+  template int launch_prolongate<T>(const DevCsr<T> &, const DevCsr<T> &, const T *, T *, int, T, \
+                                    cudaStream_t);                                                \
   template int launch_fill<T>(T *, T, int, cudaStream_t);                                         \
   template int launch_axpy<T>(T *, T, const T *, int, cudaStream_t);                              \
   template int launch_dirichlet<T>(T *, const T *, int, int, int, cudaStream_t);                  \
-  template int launch_zero_nonactive<T>(T *, int, int, cudaStream_t);                             \
   template int launch_relax<T>(T *, const T *, T, int, cudaStream_t);
 PM_INST(double)
 PM_INST(float)

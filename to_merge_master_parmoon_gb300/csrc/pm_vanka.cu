@@ -1375,7 +1375,8 @@ __global__ void __launch_bounds__(kDenseSolveThreads) k_dense_solve(const double
 }
 
 // Column j of A^{-1} from the LU factors (P A = L U): one CTA per column,
-// forward and back substitution of P e_j with barriers per step.  Runs once
+// forward and back substitution of P e_j with barriers per step, written to
+// column j of the row-major inverse.  Runs once
 // per factorisation; every coarse solve is then one GEMV.
 constexpr int kInvThreads = 256;
 __global__ void __launch_bounds__(kInvThreads) k_dense_inverse(const double *lu, const int *ipiv,
@@ -1408,26 +1409,32 @@ __global__ void __launch_bounds__(kInvThreads) k_dense_inverse(const double *lu,
       for (int i = tid; i < k; i += kInvThreads) xs[i] -= lu[(size_t)k * N + i] * xk;
     __syncthreads();
   }
-  for (int i = tid; i < N; i += kInvThreads) inv[(size_t)j * N + i] = xs[i];
+  for (int i = tid; i < N; i += kInvThreads) inv[(size_t)i * N + j] = xs[i];  // row-major
 }
 
-// x = A^{-1} b (A^{-1} column-major), b[pin_row] = 0 when pin_row >= 0
+// x = A^{-1} b (A^{-1} row-major), b[pin_row] = 0 when pin_row >= 0.  One warp
+// per row: N = 407 (a 2^3 coarsest level) gives 407 warps with all of a row's
+// loads in flight.  With one thread per row and the columns walked in turn
+// the launch took 84 us at N = 407 and 199 us at N = 992.
+constexpr int kGemvWarps = 4;
 template <typename TB, typename TX>
-__global__ void k_dense_gemv(const double *__restrict__ inv, int N, const TB *__restrict__ b,
-                             TX *__restrict__ x, int pin_row) {
-  extern __shared__ double bs[];
-  for (int i = threadIdx.x; i < N; i += blockDim.x) bs[i] = (i == pin_row) ? 0.0 : (double)b[i];
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
+__global__ void __launch_bounds__(kGemvWarps * 32) k_dense_gemv(const double *__restrict__ inv,
+                                                               int N, const TB *__restrict__ b,
+                                                               TX *__restrict__ x, int pin_row) {
+  const int i = blockIdx.x * kGemvWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= N) return;  // whole warp
+  const double *row = inv + (size_t)i * N;
   double s0 = 0.0, s1 = 0.0;
-  int j = 0;
-  for (; j + 1 < N; j += 2) {
-    s0 += inv[(size_t)j * N + i] * bs[j];
-    s1 += inv[(size_t)(j + 1) * N + i] * bs[j + 1];
+#pragma unroll 8
+  for (int j = lane; j < N; j += 64) {
+    s0 += row[j] * (j == pin_row ? 0.0 : (double)b[j]);
+    const int k = j + 32;
+    if (k < N) s1 += row[k] * (k == pin_row ? 0.0 : (double)b[k]);
   }
-  if (j < N) s0 += inv[(size_t)j * N + i] * bs[j];
-  x[i] = (TX)(s0 + s1);
+  s0 += s1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(kFull, s0, o);
+  if (lane == 0) x[i] = (TX)s0;
 }
 
 inline int ok() { return cudaPeekAtLastError() == cudaSuccess ? 1 : -1; }
@@ -1614,10 +1621,8 @@ int launch_dense_inverse(const double *lu, const int *ipiv, int n, double *inv, 
 
 template <typename TB, typename TX>
 int launch_dense_gemv(const double *inv, int n, const TB *b, TX *x, int pin_row, cudaStream_t s) {
-  const size_t sm = sizeof(double) * n;
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_dense_gemv<TB, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_dense_gemv<TB, TX><<<(n + 127) / 128, 128, sm, s>>>(inv, n, b, x, pin_row);
+  k_dense_gemv<TB, TX><<<(n + kGemvWarps - 1) / kGemvWarps, kGemvWarps * 32, 0, s>>>(inv, n, b, x,
+                                                                                    pin_row);
   return ok() < 0 ? -1 : 1;
 }
 template int launch_dense_gemv<double, double>(const double *, int, const double *, double *, int,

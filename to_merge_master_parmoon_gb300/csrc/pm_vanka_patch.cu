@@ -50,6 +50,7 @@
 #include <vector>
 
 #include "pm_bulk.cuh"
+#include "pm_chain.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -212,15 +213,6 @@ __device__ __forceinline__ void bar_sync(int id, int threads) {
 }
 __device__ __forceinline__ void bar_arrive(int id, int threads) {
   asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// the previous kernel of the stream has finished and its writes are visible
-__device__ __forceinline__ void wait_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-// the next kernel of the stream may start (it waits before it reads results)
-__device__ __forceinline__ void start_next() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // a0 b0 + a1 b1 + a2 b2, contracted in FP32 as the compiler does in
@@ -882,24 +874,37 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
   }
 }
 
+// node i of a vector [v1|v2|v3], read from L2 (the kernel before updates u in
+// place)
+template <typename T>
+__device__ __forceinline__ Node<T> node_of(const T *v, int i, int nu) {
+  return make_node(__ldcg(v + i), __ldcg(v + (size_t)nu + i), __ldcg(v + (size_t)2 * nu + i));
+}
+
 // u -> the copies (both), u on the Dirichlet nodes taken from the right-hand
 // side; p -> its copy; the right-hand side with its components side by side
+// (u = nullptr: zero).  The first kernel of a run of sweeps lets the next one
+// start only after it has waited itself: what the sweeps read before they
+// wait (packed rows, factors, patch lists) was complete then.
 template <typename T>
-__global__ void k_patch_pack_u(PatchLevel<T> L, const T *__restrict__ u, const T *__restrict__ rhs,
-                               int hb, int np) {
+__global__ void k_patch_begin(PatchLevel<T> L, const T *__restrict__ u, const T *__restrict__ rhs,
+                              int hb, int np) {
   const int nu = L.nu, n = nu > np ? nu : np;
+  wait_previous();
   start_next();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (i < nu) {
-      const T *s = i < hb ? u : rhs;
-      const Node<T> v = make_node(s[i], s[(size_t)nu + i], s[(size_t)2 * nu + i]);
+      const Node<T> f = node_of(rhs, i, nu);
+      Node<T> v = f;
+      if (i < hb)
+        v = u ? node_of(u, i, nu) : make_node(T(0), T(0), T(0));
       v.store(L.u, i);
       v.store(L.u, (size_t)nu + i);
-      make_node(rhs[i], rhs[(size_t)nu + i], rhs[(size_t)2 * nu + i]).store(L.f, i);
+      f.store(L.f, i);
     }
     if (i < np) {
-      L.p[i] = u[(size_t)3 * nu + i];
-      L.fp[i] = rhs[(size_t)3 * nu + i];
+      L.p[i] = u ? __ldcg(u + (size_t)3 * nu + i) : T(0);
+      L.fp[i] = __ldcg(rhs + (size_t)3 * nu + i);
     }
   }
 }
@@ -917,10 +922,11 @@ __global__ void k_patch_dirichlet(PatchLevel<T> L, const T *__restrict__ rhs, in
   }
 }
 
-// the current copies -> u (Dirichlet nodes from the right-hand side) and p
+// the current copies -> u (Dirichlet nodes from the right-hand side, or zero
+// without one) and p
 template <typename T>
-__global__ void k_patch_unpack_u(PatchLevel<T> L, T *__restrict__ u, const T *__restrict__ rhs,
-                                 int hb, int np, int odd) {
+__global__ void k_patch_end(PatchLevel<T> L, T *__restrict__ u, const T *__restrict__ rhs, int hb,
+                            int np, int odd) {
   const int nu = L.nu, n = nu > np ? nu : np;
   start_next();
   wait_previous();
@@ -931,9 +937,9 @@ __global__ void k_patch_unpack_u(PatchLevel<T> L, T *__restrict__ u, const T *__
         const int copy = odd & L.flips[i];
         comps(Node<T>::load(L.u, (size_t)copy * nu + i), x, y, z);
       } else {
-        x = rhs[i];
-        y = rhs[(size_t)nu + i];
-        z = rhs[(size_t)2 * nu + i];
+        x = rhs ? rhs[i] : T(0);
+        y = rhs ? rhs[(size_t)nu + i] : T(0);
+        z = rhs ? rhs[(size_t)2 * nu + i] : T(0);
       }
       u[i] = x;
       u[(size_t)nu + i] = y;
@@ -1096,24 +1102,6 @@ __global__ void __launch_bounds__(256) k_patch_pattern(
 
 inline int ok() { return cudaPeekAtLastError() == cudaSuccess ? 1 : -1; }
 
-// launch that may start while the previous kernel of the stream still runs
-// (the kernel waits for it with griddepcontrol.wait)
-template <typename... Args>
-int launch_chained(void (*kernel)(Args...), int grid, int block, size_t smem, cudaStream_t s,
-                   const Args &...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? 1 : -1;
-}
-
 int node_grid(int n) {
   const int g = (n + 255) / 256;
   return g < 1 ? 1 : (g > 8 * 152 ? 8 * 152 : g);
@@ -1247,8 +1235,8 @@ int launch_patch_init() {
 template <typename T>
 int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb, int np,
                        cudaStream_t s) {
-  k_patch_pack_u<T><<<node_grid(std::max(L.nu, np)), 256, 0, s>>>(L, u, rhs, hb, np);
-  return ok();
+  return launch_chained<PatchLevel<T>, const T *, const T *, int, int>(
+      k_patch_begin<T>, node_grid(std::max(L.nu, np)), 256, 0, s, L, u, rhs, hb, np);
 }
 
 template <typename T>
@@ -1276,7 +1264,7 @@ template <typename T>
 int launch_patch_end(const PatchLevel<T> &L, T *u, const T *rhs, int hb, int np, int odd,
                      cudaStream_t s) {
   return launch_chained<PatchLevel<T>, T *, const T *, int, int, int>(
-      k_patch_unpack_u<T>, node_grid(std::max(L.nu, np)), 256, 0, s, L, u, rhs, hb, np, odd);
+      k_patch_end<T>, node_grid(std::max(L.nu, np)), 256, 0, s, L, u, rhs, hb, np, odd);
 }
 
 #define PM_PINST(T)                                                                               \
