@@ -76,6 +76,7 @@ struct LevelDev {
   HostCsr h_pu, h_pp;             // handed-over prolongation from the next coarser level
   bool has_colour = false;
   int *rows = nullptr;  // order of the velocity rows in defects and mat-vecs
+  int max_row = 0;      // longest row of A, B and BT
   int *a_rowptr = nullptr, *a_col = nullptr, *b_rowptr = nullptr, *b_col = nullptr;
   int *bt_rowptr = nullptr, *bt_col = nullptr;
   double *a64[9] = {}, *b64[3] = {}, *bt64[3] = {};
@@ -492,7 +493,8 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
                                           static_cast<float *>(Lv.dbuf), h->stream));
     else
       PM_LAUNCH(launch_vanka_residual<T>(op, cells, Lv.colour_cells + b, n, u, rhs,
-                                         static_cast<T *>(Lv.dbuf), Lv.res_variant, h->stream));
+                                         static_cast<T *>(Lv.dbuf), Lv.res_variant, Lv.max_row,
+                                         h->stream));
     if (e1) cudaEventRecord(e1, h->stream);
     if (aos)
       PM_LAUNCH(launch_schur_apply_aos(cells, Lv.nu, Lv.colour_cells + b, n,
@@ -518,7 +520,7 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
       PM_LAUNCH(launch_vanka_apply<T>(cells, Lv.nu, Lv.colour_cells + b, n,
                                       static_cast<const T *>(Lv.factors), Lv.perm, use_inverse(h),
                                       static_cast<const T *>(Lv.dbuf), damp, u,
-                                      Lv.apply_variant == 0, h->stream));
+                                      Lv.apply_variant == 0, h->sweep_err, h->num_sms, h->stream));
     if (e2) {
       cudaEventRecord(e2, h->stream);
       // algorithmic bytes of this colour: the level's unique Vanka-sweep
@@ -1432,7 +1434,8 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
     for (int v = 0; v < 2 && st == PM_OK; ++v)
       st = time_it([&] {
         return launch_vanka_residual<T>(op, Lv.cells(), list, nb, u,
-                                        static_cast<const T *>(Lv.rhs), rb, v, h->stream);
+                                        static_cast<const T *>(Lv.rhs), rb, v, Lv.max_row,
+                                        h->stream);
       }, t[v]);
     Lv.res_variant = t[1] < t[0] ? 1 : 0;  // kernel index: 0 row groups, 1 stream
   }
@@ -1453,7 +1456,7 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
       } else {
         st = time_it([&] {
           return launch_vanka_apply<T>(Lv.cells(), Lv.nu, list, nb, F, Lv.perm, false, rb, T(1), u,
-                                       v == 0, h->stream);
+                                       v == 0, h->sweep_err, h->num_sms, h->stream);
         }, t[v]);
       }
     }
@@ -1854,6 +1857,12 @@ pm_status pm_add_level(pm_handle *h, const pm_level_desc *d) {
   Lv.pattern_key = pattern_fingerprint(d);
   Lv.has_colour = d->cell_colour != nullptr;
   if (Lv.has_colour) Lv.h_colour.assign(d->cell_colour, d->cell_colour + Lv.ncells);
+  auto longest = [&](const int *rp, int n) {
+    for (int i = 0; i < n; ++i) Lv.max_row = std::max(Lv.max_row, rp[i + 1] - rp[i]);
+  };
+  longest(d->a_rowptr, Lv.nu);
+  longest(d->b_rowptr, Lv.np);
+  longest(d->bt_rowptr, Lv.nu);
   std::vector<int> order;
   row_order(d->a_rowptr, Lv.nu, order);
   PM_TRY(upload(h, &Lv.rows, order.data(), order.size()));

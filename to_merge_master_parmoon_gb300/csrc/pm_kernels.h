@@ -160,7 +160,8 @@ int launch_vanka_factor(const DevOp<double> &op, const DevCells &cells, TF *fact
 // segmented sums.  Same result up to summation order.
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, cudaStream_t s);
+                          const T *u, const T *rhs, T *rbuf, int variant, int max_row,
+                          cudaStream_t s);
 // The same (row groups) on an FP32 one-block hexahedral level with the
 // velocity read from its interleaved copy ux (node d: ux[d].x/y/z) and the
 // pressure from u; -1 for any other level.
@@ -173,7 +174,7 @@ int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, con
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf,
-                       T damp, T *u, bool pairs, cudaStream_t s);
+                       T damp, T *u, bool pairs, int *err, int num_sms, cudaStream_t s);
 
 // Error bits of bounded device waits (sweep kernels, `err` arguments)
 constexpr int PM_ERR_BULK_TIMEOUT = 1;
