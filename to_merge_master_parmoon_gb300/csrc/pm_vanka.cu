@@ -19,6 +19,8 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "pm_bulk.cuh"
+#include "pm_chain.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -542,6 +544,25 @@ __constant__ unsigned char c_row_order[NU_LOC] = {0, 2, 6, 8, 18, 20, 24, 26, 1,
                                                   15, 17, 19, 21, 23, 25, 4, 10, 12, 14, 16, 22,
                                                   13};
 
+// a0 b0 + a1 b1 + a2 b2; FP32 in the contraction the compiler chooses for
+// that expression, spelled out so that every kernel with it agrees
+template <typename T>
+__device__ __forceinline__ T dot3(T a0, T b0, T a1, T b1, T a2, T b2) {
+  if constexpr (sizeof(T) == 4)
+    return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+  else
+    return a0 * b0 + a1 * b1 + a2 * b2;
+}
+// gathered vector entries: through L1, or (CG) from L2 in launches that start
+// before the kernel that writes the vector has finished
+template <bool CG, typename T>
+__device__ __forceinline__ T ld_x(const T *p) {
+  if constexpr (CG)
+    return __ldcg(p);
+  else
+    return __ldg(p);
+}
+
 // NV = 9 (nine A blocks), 1 (one A block), 3 with gather3 (a B row: one
 // output) or without (a BT row: gather p, three outputs); DIAG (NV = 3):
 // the diagonal blocks A11, A22, A33, value k times x_k into s[k].  AOS
@@ -571,7 +592,7 @@ __device__ __forceinline__ void rg_load(const int *__restrict__ col, const T *co
 }
 
 // the products of the loaded entries in [rs, re): gathers and FMAs
-template <typename T, int VEC, int NV, int UR, bool DIAG, bool AOS>
+template <typename T, int VEC, int NV, int UR, bool DIAG, bool AOS, bool CG = false>
 __device__ __forceinline__ void rg_accum(const int (&ci)[UR][VEC], const T (&v)[UR][NV][VEC],
                                          int g, int rs, int re, const T *__restrict__ x0,
                                          const T *__restrict__ x1, const T *__restrict__ x2,
@@ -593,9 +614,9 @@ __device__ __forceinline__ void rg_accum(const int (&ci)[UR][VEC], const T (&v)[
             g1 = g4.y;
             g2 = g4.z;
           } else {
-            g0 = __ldg(x0 + c);
-            g1 = __ldg(x1 + c);
-            g2 = __ldg(x2 + c);
+            g0 = ld_x<CG>(x0 + c);
+            g1 = ld_x<CG>(x1 + c);
+            g2 = ld_x<CG>(x2 + c);
           }
           if constexpr (DIAG) {
             s[0] += v[q][0][m] * g0;
@@ -610,10 +631,10 @@ __device__ __forceinline__ void rg_accum(const int (&ci)[UR][VEC], const T (&v)[
             s[1] += v[q][3][m] * g0 + v[q][4][m] * g1 + v[q][5][m] * g2;
             s[2] += v[q][6][m] * g0 + v[q][7][m] * g1 + v[q][8][m] * g2;
           } else {  // B row: one output
-            s[0] += v[q][0][m] * g0 + v[q][1][m] * g1 + v[q][2][m] * g2;
+            s[0] += dot3(v[q][0][m], g0, v[q][1][m], g1, v[q][2][m], g2);
           }
         } else {  // BT row: gather p, three outputs
-          const T pc = __ldg(x0 + c);
+          const T pc = ld_x<CG>(x0 + c);
           s[0] += v[q][0][m] * pc;
           if constexpr (NV >= 3) {
             s[1] += v[q][1][m] * pc;
@@ -625,7 +646,8 @@ __device__ __forceinline__ void rg_accum(const int (&ci)[UR][VEC], const T (&v)[
   }
 }
 
-template <typename T, int VEC, int NV, int UR, bool DIAG = false, bool AOS = false>
+template <typename T, int VEC, int NV, int UR, bool DIAG = false, bool AOS = false,
+          bool CG = false>
 __device__ __forceinline__ void row_group_sum(const int *__restrict__ col, const T *const *vals,
                                               int rs, int re, int sl, const T *__restrict__ x0,
                                               const T *__restrict__ x1, const T *__restrict__ x2,
@@ -634,7 +656,7 @@ __device__ __forceinline__ void row_group_sum(const int *__restrict__ col, const
     int ci[UR][VEC];
     T v[UR][NV][VEC];
     rg_load<T, VEC, NV, UR>(col, vals, g, re, ci, v);
-    rg_accum<T, VEC, NV, UR, DIAG, AOS>(ci, v, g, rs, re, x0, x1, x2, gather3, s);
+    rg_accum<T, VEC, NV, UR, DIAG, AOS, CG>(ci, v, g, rs, re, x0, x1, x2, gather3, s);
   }
 }
 
@@ -765,6 +787,205 @@ __global__ void __launch_bounds__(kResWarps * 32) k_vanka_residual_rows(
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) s[0] += __shfl_xor_sync(kFull, s[0], o);
     if (sl == 0) R[3 * NU_LOC + sub] = fp - s[0];
+  }
+}
+
+// The row-group residual with one CTA per cell and one row step per warp
+// (the last warp: the pressure rows), for colours that do not fill the GPU:
+// with one warp per cell the row steps' loads follow one another (31 us per
+// launch of any size on tetrahedra).  Each row is summed as by
+// k_vanka_residual_rows.  Matrix data are loaded before the launch waits.
+template <typename T, int VEC, int KIND, int URA, int NU>
+__global__ void __launch_bounds__(((NU + 3) / 4 + 1) * 32) k_vanka_residual_split(
+    DevOp<T> op, DevCells cells, const int *__restrict__ list, const T *__restrict__ u,
+    const T *__restrict__ rhs, T *__restrict__ rbuf) {
+  constexpr int NU_LOC = NU, kRStride = Elem<NU>::r_stride, kSteps = (NU + 3) / 4;
+  constexpr int URB = (16 / (int)sizeof(T)) / VEC > 1 ? (16 / (int)sizeof(T)) / VEC : 1;
+  constexpr int NV = KIND == 2 ? 3 : (KIND == 1 ? 1 : 9);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane >> 3, sl = lane & 7;
+  start_next();
+  const int slot = blockIdx.x, cell = __ldg(list + slot), nu = op.nu;
+  const T *u1 = u, *u2 = u + nu, *u3 = u + 2 * nu, *p = u + 3 * nu;
+  T *R = rbuf + (size_t)slot * kRStride;
+  T s[3] = {T(0), T(0), T(0)};
+  if (warp == kSteps) {
+    const int q = __ldg(cells.pdofs + (size_t)cell * NP_LOC + sub);
+    const int brs = __ldg(op.b_rowptr + q), bre = __ldg(op.b_rowptr + q + 1);
+    const T fp = __ldcg(rhs + (size_t)3 * nu + q);
+    wait_previous();
+    row_group_sum<T, VEC, 3, URB, false, false, true>(op.b_col, op.b, brs, bre, sl, u1, u2, u3, true, s);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s[0] += __shfl_xor_sync(kFull, s[0], o);
+    if (sl == 0) R[3 * NU_LOC + sub] = fp - s[0];
+    return;
+  }
+  const int k = warp * 4 + sub;
+  const bool valid = k < NU_LOC;
+  const int a = valid ? (NU == 27 ? (int)c_row_order[k] : k) : 0;
+  const int r = __ldg(cells.udofs + (size_t)cell * NU_LOC + a);
+  const int ars = __ldg(op.a_rowptr + r), are = valid ? __ldg(op.a_rowptr + r + 1) : ars;
+  int trs = 0, tre = 0;
+  if (valid && r < op.nact) {
+    trs = __ldg(op.bt_rowptr + r);
+    tre = __ldg(op.bt_rowptr + r + 1);
+  }
+  const T f = sl < 3 ? __ldcg(rhs + (size_t)sl * nu + r) : T(0);
+  const T *const *avals = KIND == 2 ? op.ad : op.a;
+  // first chunks of both parts
+  const int ga = ars / VEC + sl, gt = trs / VEC + sl;
+  int ci[URA][VEC], cj[URB][VEC];
+  T v[URA][NV][VEC], w[URB][3][VEC];
+  rg_load<T, VEC, NV, URA>(op.a_col, avals, ga, are, ci, v);
+  rg_load<T, VEC, 3, URB>(op.bt_col, op.bt, gt, tre, cj, w);
+  wait_previous();
+  rg_accum<T, VEC, NV, URA, KIND == 2, false, true>(ci, v, ga, ars, are, u1, u2, u3, true, s);
+  const int ra = (ars / VEC + 8 * URA) * VEC, rt = (trs / VEC + 8 * URB) * VEC;
+  if (ra < are)
+    row_group_sum<T, VEC, NV, URA, KIND == 2, false, true>(op.a_col, avals, ra, are, sl, u1, u2, u3, true, s);
+  rg_accum<T, VEC, 3, URB, false, false, true>(cj, w, gt, trs, tre, p, p, p, false, s);
+  if (rt < tre)
+    row_group_sum<T, VEC, 3, URB, false, false, true>(op.bt_col, op.bt, rt, tre, sl, p, p, p,
+                                                      false, s);
+  __syncwarp();
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(kFull, s[c], o);
+  }
+  if (valid && sl < 3) R[sl * NU_LOC + a] = f - (sl == 0 ? s[0] : (sl == 1 ? s[1] : s[2]));
+}
+
+// The flattened-stream residual with one CTA of eight warps per cell, for
+// colours that do not fill the GPU: the stream's blocks of 32 groups are
+// shared out over the warps and the blocks' row sums added in the order of
+// k_vanka_residual (a row of at most 32 groups meets at most two blocks).
+constexpr int kWideWarps = 8;
+constexpr int kWideBlocks = 2;  // blocks a row may meet, per part
+template <typename T, int MODE, int VEC>
+__device__ __forceinline__ void wide_rows(const SegTab &t, int nseg, int total, int base,
+                                          const int *__restrict__ col, const T *const *vals,
+                                          const T *__restrict__ x0, const T *__restrict__ x1,
+                                          const T *__restrict__ x2, T *part, int lane) {
+  constexpr int NV = MODE == 0 ? 9 : 3, NO = MODE == 2 ? 1 : 3;
+  const int g = base + lane;
+  int seg = -1;
+  long long gq = 0;
+  if (g < total) {
+    seg = find_seg(t.off, nseg, g);
+    gq = (long long)t.qs[seg] + (g - t.off[seg]);
+  }
+  T s[NO];
+#pragma unroll
+  for (int k = 0; k < NO; ++k) s[k] = T(0);
+  if (seg >= 0) {
+    int ci[VEC];
+    T v[NV][VEC];
+    VecLd<T, VEC>::idx(col + gq * VEC, ci);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) VecLd<T, VEC>::val(vals[k] + gq * VEC, v[k]);
+    const long long e0 = gq * VEC;
+    const int lo = t.rs[seg], hi = t.re[seg];
+#pragma unroll
+    for (int m = 0; m < VEC; ++m) {
+      const long long e = e0 + m;
+      if (e >= lo && e < hi) {
+        const int c = ci[m];
+        if constexpr (MODE == 1) {
+          const T g0 = __ldcg(x0 + c);
+          s[0] += v[0][m] * g0;
+          s[1 % NO] += v[1][m] * g0;
+          s[2 % NO] += v[2][m] * g0;
+        } else {
+          const T g0 = __ldcg(x0 + c), g1 = __ldcg(x1 + c), g2 = __ldcg(x2 + c);
+          s[0] += dot3(v[0][m], g0, v[1][m], g1, v[2][m], g2);
+          if constexpr (MODE == 0) {
+            s[1 % NO] += dot3(v[3][m], g0, v[4][m], g1, v[5][m], g2);
+            s[2 % NO] += dot3(v[6][m], g0, v[7][m], g1, v[8][m], g2);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int so = __shfl_down_sync(kFull, seg, o);
+#pragma unroll
+    for (int k = 0; k < NO; ++k) {
+      const T w = __shfl_down_sync(kFull, s[k], o);
+      if (lane + o < 32 && so == seg) s[k] += w;
+    }
+  }
+  const int sp = __shfl_up_sync(kFull, seg, 1);
+  if (seg >= 0 && (lane == 0 || sp != seg)) {
+    const int block = base / 32 - t.off[seg] / 32;  // 0 or 1
+#pragma unroll
+    for (int k = 0; k < NO; ++k) part[(block * NO + k) * 32 + seg] = s[k];
+  }
+}
+
+template <typename T, int VEC>
+__global__ void __launch_bounds__(kWideWarps * 32) k_vanka_residual_wide(
+    DevOp<T> op, DevCells cells, const int *__restrict__ list, const T *__restrict__ u,
+    const T *__restrict__ rhs, T *__restrict__ rbuf) {
+  __shared__ int s_tab[3][4][32], s_total[3];
+  __shared__ T s_part[2][kWideBlocks * 3 * 32], s_p[kWideBlocks * 32];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  start_next();
+  const int slot = blockIdx.x, cell = __ldg(list + slot), nu = op.nu;
+  const T *u1 = u, *u2 = u + nu, *u3 = u + 2 * nu, *p = u + 3 * nu;
+  for (int i = t; i < kWideBlocks * 3 * 32; i += kWideWarps * 32) {
+    s_part[0][i] = T(0);
+    s_part[1][i] = T(0);
+    if (i < kWideBlocks * 32) s_p[i] = T(0);
+  }
+  auto tab = [&](int k) { return SegTab{s_tab[k][0], s_tab[k][1], s_tab[k][2], s_tab[k][3]}; };
+  const bool vu = lane < NU_LOC, vp = lane < NP_LOC;
+  int my = 0;
+  if (warp < 2 && vu) my = __ldg(cells.udofs + (size_t)cell * NU_LOC + lane);
+  if (warp == 2 && vp) my = __ldg(cells.pdofs + (size_t)cell * NP_LOC + lane);
+  if (warp < 3) {
+    const int *rp = warp == 0 ? op.a_rowptr : (warp == 1 ? op.bt_rowptr : op.b_rowptr);
+    const bool on = warp == 0 ? vu : (warp == 1 ? vu && my < op.nact : vp);
+    const int n = seg_setup<VEC>(tab(warp), lane, on, on ? __ldg(rp + my) : 0,
+                                 on ? __ldg(rp + my + 1) : 0);
+    if (lane == 0) s_total[warp] = n;
+  }
+  // right-hand side of local entry t
+  T f = T(0);
+  int at = 0;
+  if (t < NLOC) {
+    const int c = t / NU_LOC;
+    at = c < 3 ? c * nu + __ldg(cells.udofs + (size_t)cell * NU_LOC + t - c * NU_LOC)
+               : 3 * nu + __ldg(cells.pdofs + (size_t)cell * NP_LOC + t - 3 * NU_LOC);
+    f = __ldcg(rhs + at);
+  }
+  __syncthreads();
+  wait_previous();
+  const int na = (s_total[0] + 31) / 32, nt = (s_total[1] + 31) / 32, nb = (s_total[2] + 31) / 32;
+  for (int k = warp; k < na + nt + nb; k += kWideWarps) {
+    if (k < na)
+      wide_rows<T, 0, VEC>(tab(0), NU_LOC, s_total[0], 32 * k, op.a_col, op.a, u1, u2, u3,
+                           s_part[0], lane);
+    else if (k < na + nt)
+      wide_rows<T, 1, VEC>(tab(1), NU_LOC, s_total[1], 32 * (k - na), op.bt_col, op.bt, p, p, p,
+                           s_part[1], lane);
+    else
+      wide_rows<T, 2, VEC>(tab(2), NP_LOC, s_total[2], 32 * (k - na - nt), op.b_col, op.b, u1, u2,
+                           u3, s_p, lane);
+  }
+  __syncthreads();
+  if (t < NLOC) {
+    T s = T(0);
+    const int c = t / NU_LOC, a = t - c * NU_LOC;
+    if (c < 3) {
+#pragma unroll
+      for (int q = 0; q < 2 * kWideBlocks; ++q)
+        s += s_part[q / kWideBlocks][((q % kWideBlocks) * 3 + c) * 32 + a];
+    } else {
+#pragma unroll
+      for (int q = 0; q < kWideBlocks; ++q) s += s_p[q * 32 + a];
+    }
+    rbuf[(size_t)slot * kRStride + t] = f - s;
   }
 }
 
@@ -1035,6 +1256,96 @@ __global__ void __launch_bounds__(WARPS * 32) k_vanka_apply2(
       const int r = hl + 16 * q;
       if (r < NLOC) scatter_local<T, NU>(r, damp * y[q], ud, pd, nu, u);
     }
+  }
+}
+
+// LU apply for colours that do not fill the GPU: one warp per cell, the whole
+// factor block (28.9 KB FP32 hexahedra, 9.6 KB tetrahedra) brought to shared
+// memory by one bulk copy before the launch waits for the residual, so that
+// the substitution's steps wait for shared memory only.  Loading columns from
+// global memory on the way took 11 us (tetrahedra) and 25 us per launch of
+// any size.  Same operations in the same order as k_vanka_apply.
+template <typename T, int NU>
+__global__ void __launch_bounds__(32) k_vanka_apply_staged(
+    DevCells cells, int nu, const int *__restrict__ list, const T *__restrict__ F,
+    const uint8_t *__restrict__ perm, const T *__restrict__ rbuf, T damp, T *__restrict__ u,
+    int *err) {
+  constexpr int NU_LOC = NU, NLOC = Elem<NU>::nloc, kFacStride = Elem<NU>::fac_stride,
+                kRStride = Elem<NU>::r_stride, SL = (NLOC + 31) / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const T *Fs = reinterpret_cast<const T *>(smem_raw);
+  __shared__ uint64_t bar;
+  const int lane = threadIdx.x;
+  start_next();
+  const int cell = __ldg(list + blockIdx.x);
+  if (lane == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+    bulk_load(smem_raw, F + (size_t)cell * kFacStride, kFacStride * (uint32_t)sizeof(T), &bar);
+  }
+  __syncwarp();
+  const uint8_t *pc = perm + (size_t)cell * NLOC;
+  int pr[SL], dof[SL];
+#pragma unroll
+  for (int q = 0; q < SL; ++q) {
+    const int i = lane + 32 * q;
+    pr[q] = i < NLOC ? __ldg(pc + i) : 0;
+    const int c = i / NU_LOC;
+    dof[q] = i < 3 * NU_LOC
+                 ? c * nu + __ldg(cells.udofs + (size_t)cell * NU_LOC + i - c * NU_LOC)
+                 : (i < NLOC ? 3 * nu + __ldg(cells.pdofs + (size_t)cell * NP_LOC + i - 3 * NU_LOC)
+                             : 0);
+  }
+  const bool there = mbar_wait(&bar, 0, kMaxPolls);
+  if (!there) {
+    if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
+    mbar_wait(&bar, 0, kMaxPolls);  // the copy still in flight (bounded)
+  }
+  wait_previous();
+  if (!there) return;
+  const T *R = rbuf + (size_t)blockIdx.x * kRStride;
+  T y[SL], o[SL];
+#pragma unroll
+  for (int q = 0; q < SL; ++q) {
+    y[q] = lane + 32 * q < NLOC ? __ldcg(R + pr[q]) : T(0);
+    o[q] = lane + 32 * q < NLOC ? __ldcg(u + dof[q]) : T(0);
+  }
+  // forward substitution with the unit lower factor
+#pragma unroll
+  for (int jb = 0; jb < SL; ++jb) {
+    const int je = jb == SL - 1 ? NLOC - 1 : 32 * jb + 32;
+#pragma unroll 4
+    for (int j = 32 * jb; j < je; ++j) {
+      const T *col = Fs + j * NLOC;
+      const T yj = __shfl_sync(kFull, y[jb], j & 31);
+#pragma unroll
+      for (int q = 0; q < SL; ++q) {
+        const int i = lane + 32 * q;
+        const T l = (i > j && i < NLOC) ? col[i] : T(0);
+        y[q] -= l * yj;
+      }
+    }
+  }
+  // back substitution with U (diagonal stores 1/U_jj)
+#pragma unroll
+  for (int jb = SL - 1; jb >= 0; --jb) {
+    const int jt = jb == SL - 1 ? NLOC - 1 : 32 * jb + 31;
+#pragma unroll 4
+    for (int j = jt; j >= 32 * jb; --j) {
+      const T *col = Fs + j * NLOC;
+      if (lane == (j & 31)) y[jb] *= col[j];
+      const T xj = __shfl_sync(kFull, y[jb], j & 31);
+#pragma unroll
+      for (int q = 0; q < SL; ++q) {
+        const int i = lane + 32 * q;
+        if (i < j) y[q] -= col[i] * xj;
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < SL; ++q) {
+    o[q] += damp * y[q];
+    if (lane + 32 * q < NLOC) u[dof[q]] = o[q];
   }
 }
 
@@ -1476,13 +1787,43 @@ int launch_vanka_factor(const DevOp<double> &op, const DevCells &cells, TF *fact
   return -1;  // the inverse is stored in FP32 only
 }
 
+// Cells of a colour up to which the residual runs with one CTA per cell.
+constexpr int kSplitCells = 2048;
+
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, cudaStream_t s) {
+                          const T *u, const T *rhs, T *rbuf, int variant, int max_row,
+                          cudaStream_t s) {
   if (ncol <= 0) return 0;
   constexpr int VEC = sizeof(T) == 4 ? 4 : 2;
   constexpr int U = sizeof(T) == 4 ? 1 : 2;
   const int grid = (ncol + kResWarps - 1) / kResWarps;
+  // one CTA per cell where the colour would leave the GPU idle
+  if (ncol <= kSplitCells) {
+    auto split = [&](auto kernel, int steps) {
+      return launch_chained<DevOp<T>, DevCells, const int *, const T *, const T *, T *>(
+          kernel, dim3((unsigned)ncol), (steps + 1) * 32, 0, s, op, cells, cell_list, u, rhs, rbuf);
+    };
+    if (cells.nl == NU_TET) {
+      if (op.structured) return split(k_vanka_residual_split<T, VEC, 1, 2, NU_TET>, 4);
+      if (op.diag) return split(k_vanka_residual_split<T, VEC, 2, 2, NU_TET>, 4);
+      return split(k_vanka_residual_split<T, VEC, 0, 1, NU_TET>, 4);
+    }
+    if (cells.nl == NU_LOC && variant == 0) {
+      if constexpr (sizeof(T) == 4) {
+        if (op.structured) return split(k_vanka_residual_split<T, 1, 1, 16, NU_LOC>, 7);
+        if (op.diag) return split(k_vanka_residual_split<T, 1, 2, 8, NU_LOC>, 7);
+      } else {
+        if (op.structured) return split(k_vanka_residual_split<T, VEC, 1, 2, NU_LOC>, 7);
+        if (op.diag) return split(k_vanka_residual_split<T, VEC, 2, 2, NU_LOC>, 7);
+      }
+      return split(k_vanka_residual_split<T, VEC, 0, 1, NU_LOC>, 7);
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (cells.nl == NU_LOC && !op.structured && !op.diag && max_row + VEC - 1 <= 32 * VEC)
+        return split(k_vanka_residual_wide<T, VEC>, kWideWarps - 1);
+    }
+  }
   if (cells.nl == NU_TET) {  // tetrahedra: the row-group kernel
     if (op.structured)
       k_vanka_residual_rows<T, VEC, 1, 2, NU_TET><<<grid, kResWarps * 32, 0, s>>>(
@@ -1544,8 +1885,26 @@ int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, con
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf, T damp,
-                       T *u, bool pairs, cudaStream_t s) {
+                       T *u, bool pairs, int *err, int num_sms, cudaStream_t s) {
   if (ncol <= 0) return 0;
+  if (!inverse && (cells.nl == NU_TET || cells.nl == NU_LOC)) {
+    // one wave of CTAs that hold a cell's factors each
+    auto staged = [&](auto kernel, int stride) {
+      const size_t sm = (size_t)stride * sizeof(T);
+      const int per_sm = std::min(24, (int)(220 * 1024 / (sm + 2048)));
+      if (ncol > per_sm * num_sms) return 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
+          cudaSuccess)
+        return -1;
+      return launch_chained<DevCells, int, const int *, const T *, const uint8_t *, const T *, T,
+                            T *, int *>(kernel, dim3((unsigned)ncol), 32, sm, s, cells, nu,
+                                        cell_list, factors, perm, rbuf, damp, u, err);
+    };
+    const int n = cells.nl == NU_TET
+                      ? staged(k_vanka_apply_staged<T, NU_TET>, Elem<NU_TET>::fac_stride)
+                      : staged(k_vanka_apply_staged<T, NU_LOC>, Elem<NU_LOC>::fac_stride);
+    if (n != 0) return n;
+  }
   const int grid = (ncol + kApplyWarps - 1) / kApplyWarps;
   constexpr int W = sizeof(T) == 4 ? 8 : 4;  // FP64 holds twice the registers
   const int g2 = (ncol + 2 * W - 1) / (2 * W);
@@ -1645,9 +2004,10 @@ template int launch_vanka_factor<float>(const DevOp<double> &, const DevCells &,
                                         uint8_t *, bool, bool, int *, cudaStream_t);
 #define PM_VINST(T)                                                                                 \
   template int launch_vanka_residual<T>(const DevOp<T> &, const DevCells &, const int *, int,      \
-                                        const T *, const T *, T *, int, cudaStream_t);             \
+                                        const T *, const T *, T *, int, int, cudaStream_t);        \
   template int launch_vanka_apply<T>(const DevCells &, int, const int *, int, const T *,           \
-                                     const uint8_t *, bool, const T *, T, T *, bool, cudaStream_t);
+                                     const uint8_t *, bool, const T *, T, T *, bool, int *, int,   \
+                                     cudaStream_t);
 PM_VINST(double)
 PM_VINST(float)
 #undef PM_VINST
