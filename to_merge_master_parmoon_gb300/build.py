@@ -36,7 +36,8 @@ GPU_CPP = ["pm_setup_host.cpp"]
 HOST_CPP = ["oseen_problem.cpp", "oseen_tet.cpp"]
 HEADERS = [INCLUDE / "pmgpu.h", CSRC / "pm_kernels.h", CSRC / "pm_setup_host.h",
            CSRC / "oseen_problem.h", CSRC / "oseen_internal.h", CSRC / "pm_learned.h",
-           CSRC / "pm_bulk.cuh", CSRC / "pm_chain.cuh"]
+           CSRC / "pm_bulk.cuh", CSRC / "pm_chain.cuh",
+           CSRC / "pm_fp.cuh"]
 
 
 def nvcc_path() -> str:

@@ -14,6 +14,7 @@
 // all taken from the state before the colour (CellVanka_GPU semantics,
 // src/FE/NSE_CellVanka.cu:2181-2365), so step 2 runs after step 1 of the
 // whole colour in a separate launch.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,6 +22,7 @@
 
 #include "pm_bulk.cuh"
 #include "pm_chain.cuh"
+#include "pm_fp.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -153,19 +155,22 @@ __global__ void __launch_bounds__(kFactorThreads) k_vanka_factor(DevOp<double> o
   // freshly updated entries.
   // pivot of column k (rows k..): first maximal |a|, with its signed value
   auto pivot_search = [&](int k) {
-    TC best = TC(-1), bv = TC(0);
+    typedef typename KeyOf<TC>::type Key;
+    Key best = Key(-1);
+    TC bv = TC(0);
     int bi = k;
     for (int i = k + lane; i < NLOC; i += 32) {
       const TC v = S[k * NLOC + i];
-      if (fabs(v) > best) {
-        best = fabs(v);
+      const Key key = abs_key(v);
+      if (key > best) {
+        best = key;
         bv = v;
         bi = i;
       }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const TC ob = __shfl_xor_sync(kFull, best, o);
+      const Key ob = __shfl_xor_sync(kFull, best, o);
       const TC ov = __shfl_xor_sync(kFull, bv, o);
       const int oi = __shfl_xor_sync(kFull, bi, o);
       if (ob > best || (ob == best && oi < bi)) {
@@ -178,8 +183,8 @@ __global__ void __launch_bounds__(kFactorThreads) k_vanka_factor(DevOp<double> o
       piv_row = bi;
       piv_val = bv;
       piv_d0 = S[k * NLOC + k];  // lane 0 holds row k (its own entry)
-      piv_rcp = bv != TC(0) ? TC(1) / bv : TC(0);
-      if (bv == TC(0)) singular = 1;
+      piv_rcp = nonzero(bv) ? TC(1) / bv : TC(0);
+      if (!nonzero(bv)) singular = 1;
     }
   };
   if (warp == 0) pivot_search(0);
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(kFactorThreads) k_vanka_factor(DevOp<double> o
       }
     // column k after the interchange: pv on the diagonal, row p holds the
     // old diagonal d0; below the diagonal scaled by 1 / pivot
-    const TC sc = rp != TC(0) ? rp : TC(1);
+    const TC sc = nonzero(rp) ? rp : TC(1);
     for (int i = k + 1 + tid; i < NLOC; i += kFactorThreads)
       S[k * NLOC + i] = (i == p ? d0 : S[k * NLOC + i]) * sc;
     if (tid == 0) {
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(kFactorThreads) k_vanka_factor(DevOp<double> o
     __syncthreads();
     for (int jj = k + 1 + warp; jj < NLOC; jj += nwarps) {
       const TC ukj = S[jj * NLOC + k];
-      if (ukj != TC(0))
+      if (nonzero(ukj))
         for (int ii = k + 1 + lane; ii < NLOC; ii += 32) S[jj * NLOC + ii] -= S[k * NLOC + ii] * ukj;
     }
     if (warp == 0 && k + 1 < NLOC) {
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(kFactorThreads) k_vanka_factor(DevOp<double> o
   for (int t = tid; t < NLOC * NLOC; t += kFactorThreads) {
     const int i = t % NLOC, j = t / NLOC;
     TC v = S[t];
-    if (i == j) v = (v != TC(0)) ? TC(1) / v : TC(0);
+    if (i == j) v = nonzero(v) ? TC(1) / v : TC(0);
     F[t] = (TF)v;
   }
   if (tid < NLOC) perm[(size_t)cell * NLOC + tid] = pm[tid];
@@ -1572,6 +1577,141 @@ __global__ void __launch_bounds__(kDenseThreads) k_lu_panel(double *a, int N, in
   }
 }
 
+// The same panel by a cluster of eight CTAs that share out its rows: the FP64
+// rate of one SM (2 FMA per cycle) held k_lu_panel at 250 us for 992 rows.  A
+// step takes two cluster barriers: the CTAs' pivot candidates are exchanged
+// through distributed shared memory, then the pivot row and the row it changes
+// places with.  Rows stay in shared memory (kLuChunk per CTA at most).  The
+// operations on each entry and the pivot rule are k_lu_panel's.
+constexpr int kLuCluster = 8, kLuPanelThreads = 256;
+constexpr int kLuChunk = 768;  // 196 KB of rows
+struct LuPanelShared {
+  long long cand[2][kLuCluster];  // candidates of every CTA (abs_key), by step parity
+  int cidx[2][kLuCluster];
+  double cval[2][kLuCluster];
+  double prow[2][kLuNb], krow[2][kLuNb];
+  double rcp;
+  long long wv[kLuPanelThreads / 32];
+  int wi[kLuPanelThreads / 32];
+};
+__global__ void __cluster_dims__(kLuCluster, 1, 1) __launch_bounds__(kLuPanelThreads)
+    k_lu_panel_cluster(double *a, int N, int k0, int *ipiv, int *status) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ LuPanelShared sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = (int)cluster.block_rank();
+  const int w = min(kLuNb, N - k0), rows = N - k0;
+  const int chunk = (rows + kLuCluster - 1) / kLuCluster;
+  const int r0 = rank * chunk, nr = max(0, min(chunk, rows - r0));  // panel rows r0 .. r0 + nr - 1
+  double *A = reinterpret_cast<double *>(smem_raw);                 // A[j * chunk + i]
+  for (int j = 0; j < w; ++j)
+    for (int i = tid; i < nr; i += kLuPanelThreads)
+      A[j * chunk + i] = a[(size_t)(k0 + j) * N + k0 + r0 + i];
+  __syncthreads();
+  for (int k = 0; k < w; ++k) {
+    const int b = k & 1;
+    // first maximal |a| of column k in rows >= k
+    long long best = -1;
+    int bidx = k;
+    for (int i = tid; i < nr; i += kLuPanelThreads) {
+      if (r0 + i < k) continue;
+      const long long v = abs_key(A[k * chunk + i]);
+      if (v > best) {
+        best = v;
+        bidx = r0 + i;
+      }
+    }
+    auto better = [&](long long ob, int oi) {
+      const bool take = ob > best || (ob == best && oi < bidx);
+      if (take) {
+        best = ob;
+        bidx = oi;
+      }
+      return take;
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      better(__shfl_xor_sync(kFull, best, o), __shfl_xor_sync(kFull, bidx, o));
+    if (lane == 0) {
+      sh.wv[warp] = best;
+      sh.wi[warp] = bidx;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      best = lane < kLuPanelThreads / 32 ? sh.wv[lane] : -1ll;
+      bidx = lane < kLuPanelThreads / 32 ? sh.wi[lane] : k;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+        better(__shfl_xor_sync(kFull, best, o), __shfl_xor_sync(kFull, bidx, o));
+      best = __shfl_sync(kFull, best, 0);
+      bidx = __shfl_sync(kFull, bidx, 0);
+      if (lane < kLuCluster) {
+        LuPanelShared *to = cluster.map_shared_rank(&sh, lane);
+        to->cand[b][rank] = best;
+        to->cidx[b][rank] = bidx;
+        to->cval[b][rank] = best >= 0 ? A[k * chunk + bidx - r0] : 0.0;
+      }
+    }
+    cluster.sync();
+    best = sh.cand[b][0];
+    bidx = sh.cidx[b][0];
+    double pv = sh.cval[b][0];
+#pragma unroll
+    for (int q = 1; q < kLuCluster; ++q)
+      if (better(sh.cand[b][q], sh.cidx[b][q])) pv = sh.cval[b][q];
+    const int p = best < 0 ? k : bidx;
+    // the owners of rows p and k hand both to every CTA; meanwhile one warp
+    // forms the pivot's reciprocal
+    const int po = p / chunk, ko = k / chunk;
+    if (rank == po && tid < w * kLuCluster) {
+      LuPanelShared *to = cluster.map_shared_rank(&sh, tid / w);
+      to->prow[b][tid % w] = A[(tid % w) * chunk + p - r0];
+    }
+    if (rank == ko && tid < w * kLuCluster) {
+      LuPanelShared *to = cluster.map_shared_rank(&sh, tid / w);
+      to->krow[b][tid % w] = A[(tid % w) * chunk + k - r0];
+    }
+    if (warp == kLuPanelThreads / 32 - 1 && best >= 0) {
+      const double r = nonzero(pv) ? 1.0 / pv : 0.0;
+      if (lane == 0) sh.rcp = r;
+    }
+    cluster.sync();
+    if (p != k && tid < w) {
+      if (rank == ko) A[tid * chunk + k - r0] = sh.prow[b][tid];
+      if (rank == po) A[tid * chunk + p - r0] = sh.krow[b][tid];
+    }
+    __syncthreads();
+    // every candidate a NaN: row k stays and divides as k_lu_panel does
+    const double rp = best >= 0 ? sh.rcp : 1.0 / sh.prow[b][k];
+    if (rank == 0 && tid == 0) {
+      ipiv[k0 + k] = k0 + p;
+      if (!nonzero(rp)) atomicOr(status, 2);
+    }
+    // four lanes per row, each every fourth column
+    for (int i0 = 0; i0 < nr; i0 += kLuPanelThreads / 4) {
+      const int i = i0 + (tid >> 2), g = tid & 3;
+      const bool on = i < nr && r0 + i > k;
+      double l = on ? A[k * chunk + i] : 0.0;
+      if (nonzero(rp)) l *= rp;
+      __syncwarp();
+      if (on) {
+        if (g == 0) A[k * chunk + i] = l;
+        for (int j = k + 1 + g; j < w; j += 4) {
+          const double ukj = sh.prow[b][j];
+          if (nonzero(ukj)) A[j * chunk + i] -= l * ukj;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = 0; j < w; ++j)
+    for (int i = tid; i < nr; i += kLuPanelThreads)
+      a[(size_t)(k0 + j) * N + k0 + r0 + i] = A[j * chunk + i];
+  cluster.sync();  // no CTA leaves while another may still write to its shared memory
+}
+
 // one warp per column outside the panel: the panel's interchanges, then
 // (right of the panel) U12 = L11^{-1} A12
 __global__ void k_lu_swap_trsm(double *a, int N, int k0, const int *ipiv) {
@@ -1581,18 +1721,30 @@ __global__ void k_lu_swap_trsm(double *a, int N, int k0, const int *ipiv) {
   if (w >= N - m) return;  // whole warp
   const int j = w < k0 ? (int)w : (int)w + m;
   double *col = a + (size_t)j * N;
-  if (lane == 0)
-    for (int k = k0; k < kend; ++k) {
-      const int p = ipiv[k];
-      if (p != k) {
-        const double t = col[k];
-        col[k] = col[p];
-        col[p] = t;
-      }
-    }
-  __syncwarp();
-  if (j < k0) return;
+  // the interchanges k <-> ipiv[k] in turn, on values fetched at once: lane q
+  // holds entry k0 + q and the entry below the panel that pivot q names; when
+  // two pivots name the same one, the later finds what the earlier left there
+  const int p = lane < m ? ipiv[k0 + lane] : -1;
   double v = lane < m ? col[k0 + lane] : 0.0;
+  double below = p >= kend ? col[p] : 0.0;
+  for (int k = 0; k < m; ++k) {
+    const int pk = __shfl_sync(kFull, p, k);
+    const double vk = __shfl_sync(kFull, v, k);
+    if (pk < kend) {  // inside the panel's rows
+      const double t = __shfl_sync(kFull, v, pk - k0);
+      if (lane == k) v = t;
+      if (lane == pk - k0) v = vk;
+    } else {
+      const double t = __shfl_sync(kFull, below, k);
+      if (lane == k) v = t;
+      if (p == pk) below = vk;
+    }
+  }
+  if (p >= kend) col[p] = below;  // lanes that name the same entry hold the same value
+  if (j < k0) {
+    if (lane < m) col[k0 + lane] = v;
+    return;
+  }
   for (int k = 0; k < m; ++k) {
     const double xk = __shfl_sync(kFull, v, k);
     if (lane > k && lane < m) v -= a[(size_t)(k0 + k) * N + k0 + lane] * xk;
@@ -1600,8 +1752,9 @@ __global__ void k_lu_swap_trsm(double *a, int N, int k0, const int *ipiv) {
   if (lane < m) col[k0 + lane] = v;
 }
 
-// A22 -= L21 U12: 64 x 64 tiles, 256 threads with 4 x 4 outputs each
-constexpr int kLuTile = 64;
+// A22 -= L21 U12: 32 x 32 tiles, 256 threads with 2 x 2 outputs each (64 x 64
+// tiles left most SMs idle: 46 us instead of 12 at N = 407)
+constexpr int kLuTile = 32;
 __global__ void __launch_bounds__(256) k_lu_gemm(double *a, int N, int k0) {
   __shared__ double Ls[kLuNb][kLuTile + 1];  // [k][i]
   __shared__ double Us[kLuNb][kLuTile + 1];  // [k][j]
@@ -1618,28 +1771,24 @@ __global__ void __launch_bounds__(256) k_lu_gemm(double *a, int N, int k0) {
   }
   __syncthreads();
   const int ti = tid & 15, tj = tid >> 4;
-  double acc[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
   for (int k = 0; k < m; ++k) {
-    double l[4], u[4];
+    double l[2], u[2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) l[r] = Ls[k][ti + 16 * r];
+    for (int r = 0; r < 2; ++r) l[r] = Ls[k][ti + 16 * r];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) u[c] = Us[k][tj + 16 * c];
+    for (int c = 0; c < 2; ++c) u[c] = Us[k][tj + 16 * c];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] += l[r] * u[c];
+      for (int c = 0; c < 2; ++c) acc[r][c] += l[r] * u[c];
   }
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < 2; ++c) {
     const int j = j0 + tj + 16 * c;
     if (j >= N) continue;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < 2; ++r) {
       const int i = i0 + ti + 16 * r;
       if (i < N) a[(size_t)j * N + i] -= acc[r][c];
     }
@@ -1721,6 +1870,61 @@ __global__ void __launch_bounds__(kInvThreads) k_dense_inverse(const double *lu,
     __syncthreads();
   }
   for (int i = tid; i < N; i += kInvThreads) inv[(size_t)i * N + j] = xs[i];  // row-major
+}
+
+// The same by one warp per column with the column in registers (lane l holds
+// rows l, l + 32, ...; at most 32 SLOTS of them): no barriers, and the warps of
+// all columns keep the quarters of every SM busy with their FP64 FMAs.  Steps
+// are unrolled by the register slot of row k.  Same operations in the same
+// order as k_dense_inverse.
+template <int SLOTS>
+__global__ void __launch_bounds__(32) k_dense_inverse_warp(const double *__restrict__ lu,
+                                                           const int *__restrict__ ipiv, int N,
+                                                           double *__restrict__ inv) {
+  const int j = blockIdx.x, lane = threadIdx.x;
+  // P e_j: the interchanges move a single one
+  int pos = j;
+  for (int k = 0; k < N; ++k) {
+    const int p = ipiv[k];
+    pos = pos == k ? p : (pos == p ? k : pos);
+  }
+  double x[SLOTS];
+#pragma unroll
+  for (int q = 0; q < SLOTS; ++q) x[q] = lane + 32 * q == pos ? 1.0 : 0.0;
+  // L: rows before pos stay zero
+#pragma unroll
+  for (int kb = 0; kb < SLOTS; ++kb) {
+    const int ke = min(N, 32 * kb + 32);
+    for (int k = max(32 * kb, pos); k < ke; ++k) {
+      const double xk = __shfl_sync(kFull, x[kb], k & 31);
+      if (!nonzero(xk)) continue;
+      const double *col = lu + (size_t)k * N;
+#pragma unroll
+      for (int q = kb; q < SLOTS; ++q) {
+        const int i = lane + 32 * q;
+        if (i > k && i < N) x[q] -= __ldg(col + i) * xk;
+      }
+    }
+  }
+#pragma unroll
+  for (int kb = SLOTS - 1; kb >= 0; --kb) {
+    for (int k = min(N, 32 * kb + 32) - 1; k >= 32 * kb; --k) {
+      const double *col = lu + (size_t)k * N;
+      if (lane == (k & 31)) x[kb] /= __ldg(col + k);
+      const double xk = __shfl_sync(kFull, x[kb], k & 31);
+      if (!nonzero(xk)) continue;
+#pragma unroll
+      for (int q = 0; q <= kb; ++q) {
+        const int i = lane + 32 * q;
+        if (i < k) x[q] -= __ldg(col + i) * xk;
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < SLOTS; ++q) {
+    const int i = lane + 32 * q;
+    if (i < N) inv[(size_t)i * N + j] = x[q];  // row-major
+  }
 }
 
 // x = A^{-1} b (A^{-1} row-major), b[pin_row] = 0 when pin_row >= 0.  One warp
@@ -1953,7 +2157,16 @@ int launch_dense_lu(double *a, int n, int *ipiv, int *status, cudaStream_t s) {
   int launches = 0;
   for (int k0 = 0; k0 < n; k0 += kLuNb) {
     const int m = std::min(kLuNb, n - k0), rest = n - k0 - m;
-    k_lu_panel<<<1, kDenseThreads, 0, s>>>(a, n, k0, ipiv, status);
+    const int chunk = (n - k0 + kLuCluster - 1) / kLuCluster;
+    if (chunk <= kLuChunk) {
+      const size_t sm = sizeof(double) * kLuNb * (size_t)chunk;
+      if (cudaFuncSetAttribute(k_lu_panel_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sm) != cudaSuccess)
+        return -1;
+      k_lu_panel_cluster<<<kLuCluster, kLuPanelThreads, sm, s>>>(a, n, k0, ipiv, status);
+    } else {
+      k_lu_panel<<<1, kDenseThreads, 0, s>>>(a, n, k0, ipiv, status);
+    }
     ++launches;
     if (n - m > 0) {
       const long long threads = (long long)(n - m) * 32;
@@ -1971,6 +2184,14 @@ int launch_dense_lu(double *a, int n, int *ipiv, int *status, cudaStream_t s) {
 }
 
 int launch_dense_inverse(const double *lu, const int *ipiv, int n, double *inv, cudaStream_t s) {
+  if (n <= 32 * 14) {
+    k_dense_inverse_warp<14><<<n, 32, 0, s>>>(lu, ipiv, n, inv);
+    return ok() < 0 ? -1 : 1;
+  }
+  if (n <= 32 * 36) {
+    k_dense_inverse_warp<36><<<n, 32, 0, s>>>(lu, ipiv, n, inv);
+    return ok() < 0 ? -1 : 1;
+  }
   const size_t sm = sizeof(double) * n;
   if (sm > 48 * 1024)
     cudaFuncSetAttribute(k_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -42,6 +42,7 @@
 
 #include <cstdint>
 
+#include "pm_fp.cuh"
 #include "pm_kernels.h"
 
 namespace pm {
@@ -83,11 +84,6 @@ struct FactorSmem {
   double D[NP_LOC * 3 * NU_LOC];    // D[(k*3+c)*27 + i] = Bc(pdof_k, udof_i)
   int ud[NU_LOC], pd[NP_LOC];
 };
-
-template <typename T>
-__device__ __forceinline__ T abs_of(T v) {
-  return v < T(0) ? -v : v;
-}
 
 template <typename TF, typename TC, int NB>
 __global__ void __launch_bounds__(kFactorWarps * 32) k_schur_factor(DevOp<double> op,
@@ -155,11 +151,12 @@ __global__ void __launch_bounds__(kFactorWarps * 32) k_schur_factor(DevOp<double
 
     // Gauss-Jordan: [A_b | I | G] -> [I | A_b^{-1} | A_b^{-1} G]
     for (int k = 0; k < NU_LOC; ++k) {
-      TC best = (lane >= k && lane < NU_LOC) ? abs_of(my[k]) : TC(-1);
+      typedef typename KeyOf<TC>::type Key;
+      Key best = (lane >= k && lane < NU_LOC) ? abs_key(my[k]) : Key(-1);
       int bi = lane;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        const TC ob = __shfl_xor_sync(kFull, best, o);
+        const Key ob = __shfl_xor_sync(kFull, best, o);
         const int oi = __shfl_xor_sync(kFull, bi, o);
         if (ob > best || (ob == best && oi < bi)) {
           best = ob;
@@ -177,14 +174,14 @@ __global__ void __launch_bounds__(kFactorWarps * 32) k_schur_factor(DevOp<double
       }
       __syncwarp();
       const TC piv = M[k * MS + k];
-      if (piv == TC(0)) singular = true;
-      const TC rp = piv != TC(0) ? TC(1) / piv : TC(0);
+      if (!nonzero(piv)) singular = true;
+      const TC rp = nonzero(piv) ? TC(1) / piv : TC(0);
       __syncwarp();
       for (int c = k + 1 + lane; c < GW; c += 32) M[k * MS + c] *= rp;
       __syncwarp();
       if (lane < NU_LOC && lane != k) {
         const TC f = my[k];
-        if (f != TC(0))
+        if (nonzero(f))
           for (int c = k + 1; c < GW; ++c) my[c] -= f * M[k * MS + c];
       }
       __syncwarp();
