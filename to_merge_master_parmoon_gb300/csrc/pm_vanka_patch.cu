@@ -3,7 +3,7 @@
 //
 // One colour of a sweep (CellVanka, src/FE/NSE_MGLevel4.C:1653-2087, in the
 // colour-block order of CellVanka_GPU, src/FE/NSE_CellVanka.cu:1748-2555) is
-// one launch, one CTA of 192 threads per cell: local residual r = f - K u on
+// one launch of persistent CTAs: local residual r = f - K u on
 // the cell's 85 DOFs, block elimination (pm_vanka_schur.cu) and the update.
 //
 // Why a packed copy.  The rows of a cell couple to the 343 nodes of the cell
@@ -636,9 +636,10 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
 }
 
 // ------------------------------------------------------------------ FP64 ---
+template <int ST>
 struct Smem64 {
-  double values[2][kPatchValues];
-  double fac[2][Schur<1>::stride];
+  double values[ST][kPatchValues];
+  double fac[ST][Schur<1>::stride];
   int ids[3][kPatchIds];
   Tri<double, kPatchNodes + 1> u;
   __align__(16) double p[28][NP_LOC];
@@ -646,27 +647,33 @@ struct Smem64 {
   double yp[3][7 * NU_LOC];  // partial A^{-1} r
   double y[3][32];
   double rp[NP_LOC], t[NP_LOC];
-  uint64_t vbar[2], fbar[2], ibar[3];
+  uint64_t vbar[ST], fbar[ST], ibar[3];
 };
-constexpr int kCtas64 = 2;  // resident CTAs per SM (106 KB of shared memory each)
+// resident CTAs per SM: 63 KB of shared memory with one stage, 106 KB with two
+__host__ __device__ constexpr int ctas64(int stages) { return stages == 1 ? 3 : 2; }
 
 // FP64: the pipe takes half a lane per cycle in each quarter of the SM, so a
 // warp's FMA occupies its quarter for 64 cycles and every phase is spread
 // over the quarters (warp % 4): vertex rows on quarters 0 and 1, edges on 2,
 // 3 and 2, the other rows on 0 and 3, pressure rows on 1; the block solve on
-// all warps instead of one.  Two stages of bulk copies as in FP32.
-__global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
+// all warps instead of one.  With one stage (ST = 1) of packed rows and factors
+// the next cell's rows arrive during the block solve, and the other two CTAs of
+// the SM use the pipe meanwhile (83 % busy at 32^3; 72 % with ST = 2).  Rows and
+// factors from DRAM at 64^3, one colour: 979 us (1.47 TB/s; the CSR kernels
+// take 1,046), 32^3 134 (162), 16^3 29 (69), 8^3 12.6 (52).
+template <int ST>
+__global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
     PatchLevel<double> L, const int *__restrict__ list, int n, const double *__restrict__ factors,
     double damp, int odd, int *err) {
   using S1 = Schur<1>;
   extern __shared__ __align__(16) unsigned char raw[];
-  Smem64 &sm = *reinterpret_cast<Smem64 *>(raw);
+  Smem64<ST> &sm = *reinterpret_cast<Smem64<ST> *>(raw);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, sub = lane >> 3, sl = lane & 7;
   const int nu = L.nu, G = gridDim.x, first = blockIdx.x;
   const int count = (n - first + G - 1) / G;
   start_next();
   if (t == 0) {
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < ST; ++b) {
       mbar_init(&sm.vbar[b], 1);
       mbar_init(&sm.fbar[b], 1);
     }
@@ -685,26 +692,30 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
     return false;
   };
   auto cell_of = [&](int c) { return __ldg(list + first + (size_t)c * G); };
-  auto bring = [&](int c, int cell) {  // thread 0: values and factors of the CTA's cell c
-    bulk_load(sm.values[c & 1], L.values + (size_t)cell * kPatchValues, sizeof(sm.values[0]),
-              &sm.vbar[c & 1]);
-    bulk_load(sm.fac[c & 1], factors + (size_t)cell * S1::stride, sizeof(sm.fac[0]),
-              &sm.fbar[c & 1]);
+  // thread 0: rows, factors and patch list of one cell
+  auto bring_values = [&](int c, int cell) {
+    bulk_load(sm.values[c % ST], L.values + (size_t)cell * kPatchValues, sizeof(sm.values[0]),
+              &sm.vbar[c % ST]);
+  };
+  auto bring_fac = [&](int c, int cell) {
+    bulk_load(sm.fac[c % ST], factors + (size_t)cell * S1::stride, sizeof(sm.fac[0]),
+              &sm.fbar[c % ST]);
   };
   auto bring_ids = [&](int c, int cell) {
     bulk_load(sm.ids[c % 3], L.ids + (size_t)cell * kPatchIds, sizeof(sm.ids[0]), &sm.ibar[c % 3]);
   };
-  int a2 = 0, a3 = 0, issued = 0, issued_ids = 0;  // thread 0
+  int a1 = 0, a2 = 0, a3 = 0, nv = 0, nf = 0, ni = 0;  // thread 0: next cells, copies started
   if (t == 0) {
-    for (int c = 0; c < 2 && c < count; ++c) {
-      const int cell = cell_of(c);
-      bring_ids(c, cell);
-      bring(c, cell);
-    }
+    const int c0 = cell_of(0);
+    bring_ids(0, c0);
+    bring_values(0, c0);
+    bring_fac(0, c0);
+    nv = nf = 1;
+    if (count > 1) bring_ids(1, a1 = cell_of(1));
+    if (ST == 2 && count > 1) bring_values(1, a1), bring_fac(1, a1), nv = nf = 2;
     if (count > 2) bring_ids(2, a2 = cell_of(2));
     if (count > 3) a3 = cell_of(3);
-    issued = count < 2 ? count : 2;
-    issued_ids = count < 3 ? count : 3;
+    ni = count < 3 ? count : 3;
   }
   // row group of a warp: 0, 1 vertices, 2..4 edges, 5, 6 the rest, 7 pressure rows
   const int group = warp < 4 ? warp : (warp == 4 ? 5 : (warp == 5 ? 7 : (warp == 6 ? 4 : 6)));
@@ -748,7 +759,7 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
   if (alive) gather_u(sm.ids[0]);
   int ib = 0, ip = 0;
   for (int j = 0; j < count; ++j) {
-    const int b = j & 1;
+    const int b = j % ST;
     const int *ids = sm.ids[ib];
     const int ibn = ib == 2 ? 0 : ib + 1, ipn = ib == 2 ? ip ^ 1 : ip;
     {
@@ -771,9 +782,8 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
         next_pid = sm.ids[ibn][kPatchPattern];
       }
     }
-    alive = arrived(&sm.vbar[b], j >> 1) && alive;
-    alive = arrived(&sm.fbar[b], j >> 1) && alive;
     if (group < 7) {
+      alive = arrived(&sm.vbar[b], j / ST) && alive;
       double c0, c1, c2;
       row_sum(group, li, sm.values[b], sm.u, &sm.p[0][0], s0, s1, bts, c0, c1, c2);
       // six FP64 additions instead of nine: lanes 0..3 go on with component
@@ -788,10 +798,16 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
       const double d2 = __shfl_xor_sync(kFull, d, 6);
       if (k < NU_LOC && sl < 3) sm.r.ref(row, sl) = fi - (sl == 0 ? c0 : (sl == 1 ? d : d2));
     } else {
+      alive = arrived(&sm.fbar[b], j / ST) && alive;
       const double c = pressure_sum(sub, sm.fac[b], sm.u, bj, o01, o23);
       if (sl == 0) sm.rp[sub] = fi - c;
     }
     __syncthreads();
+    if (alive && t == 0 && j + ST < count) {
+      bring_values(j + ST, ST == 1 ? a1 : a2);
+      nv = j + ST + 1;
+    }
+    alive = arrived(&sm.fbar[b], j / ST) && alive;
     const double *F = sm.fac[b];
     if (t >= 64 && t - 64 < 7 * NU_LOC) {  // y = A^{-1} r: four columns per thread
       const int q = t - 64, gq = q / NU_LOC, i = q - gq * NU_LOC;
@@ -855,8 +871,9 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
     }
     __syncthreads();  // the stage and the gathered values have been read
     if (alive && t == 0) {
-      if (j + 2 < count) bring(j + 2, a2), issued = j + 3;
-      if (j + 3 < count) bring_ids(j + 3, a3), issued_ids = j + 4;
+      if (j + ST < count) bring_fac(j + ST, ST == 1 ? a1 : a2), nf = j + ST + 1;
+      if (j + 3 < count) bring_ids(j + 3, a3), ni = j + 4;
+      a1 = a2;
       a2 = a3;
       if (j + 4 < count) a3 = cell_of(j + 4);
     }
@@ -865,11 +882,9 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas64) k_patch_sweep64(
     ip = ipn;
   }
   if (!alive && t == 0) {  // copies still in flight
-    for (int c = issued > 2 ? issued - 2 : 0; c < issued; ++c) {
-      drain(&sm.vbar[c & 1], c >> 1);
-      drain(&sm.fbar[c & 1], c >> 1);
-    }
-    for (int c = issued_ids > 3 ? issued_ids - 3 : 0; c < issued_ids; ++c)
+    for (int c = nv > ST ? nv - ST : 0; c < nv; ++c) drain(&sm.vbar[c % ST], c / ST);
+    for (int c = nf > ST ? nf - ST : 0; c < nf; ++c) drain(&sm.fbar[c % ST], c / ST);
+    for (int c = ni > 3 ? ni - 3 : 0; c < ni; ++c)
       drain(&sm.ibar[c % 3], c / 3);
   }
 }
@@ -1227,7 +1242,8 @@ int launch_patch_init() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
            cudaSuccess;
   };
-  return set(k_patch_sweep32, sizeof(Smem32)) && set(k_patch_sweep64, sizeof(Smem64))
+  return set(k_patch_sweep32, sizeof(Smem32)) && set(k_patch_sweep64<1>, sizeof(Smem64<1>)) &&
+                 set(k_patch_sweep64<2>, sizeof(Smem64<2>))
              ? 0
              : -1;
 }
@@ -1247,10 +1263,18 @@ int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T 
     return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *>(
         k_patch_sweep32, std::min(n, kCtas32 * num_sms), kPatchThreads, sizeof(Smem32), s, L, list,
         n, factors, damp, odd, err);
-  else
+  else {
+    // Two stages while they hold all the cells of a CTA: with rows that come
+    // from DRAM, two sweeps at 16^3 take 492 us against 541 with one stage.
+    // One stage and a third CTA above: colour at 32^3 134 against 153 us, at
+    // 64^3 979 against 1112.
+    const int two = ctas64(2) * num_sms;
+    const bool all = n <= 2 * two;
     return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *>(
-        k_patch_sweep64, std::min(n, kCtas64 * num_sms), kPatchThreads, sizeof(Smem64), s, L, list,
-        n, factors, damp, odd, err);
+        all ? k_patch_sweep64<2> : k_patch_sweep64<1>,
+        std::min(n, all ? two : ctas64(1) * num_sms), kPatchThreads,
+        all ? sizeof(Smem64<2>) : sizeof(Smem64<1>), s, L, list, n, factors, damp, odd, err);
+  }
 }
 
 template <typename T>
