@@ -34,7 +34,6 @@ struct pm_mlp {
 
 using namespace pm;
 
-static_assert(kPatchIds == kPatchIdsHost, "patch list layout");
 
 namespace {
 double now_s() {
@@ -706,28 +705,25 @@ bool release_patches(pm_handle *h) {
   return true;
 }
 
-// Packed rows of one level: patch lists on the host, patterns and values on
-// the device.  *fits: the mesh and the CSR pattern have the layout's shape.
+// Packed rows of one level, made on the device.  *fits: the mesh and the CSR pattern have the layout's shape.
 template <typename T>
 pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   *fits = false;
-  std::vector<int> ids;
-  std::vector<unsigned char> flips;
-  if (!build_patches(Lv.ncells, Lv.h_udofs.data(), Lv.h_pdofs.data(), Lv.nu, Lv.np, Lv.colouring,
-                     ids, flips))
+  const size_t nc = (size_t)Lv.ncells, room = nc * kPatchValues * sizeof(T);
+  if (Lv.nu >= (1 << 29) || Lv.np % NP_LOC || nc * NU_LOC > INT_MAX ||
+      patch_list_scratch(Lv.ncells, Lv.nu, Lv.np) > room)
     return PM_OK;
-  const size_t nc = (size_t)Lv.ncells;
   if (launch_patch_init() < 0) return cuda_fail(h, "packed sweeps");
   unsigned char *val = nullptr, *u = nullptr, *p = nullptr, *pat = nullptr;
-  PM_TRY(upload(h, &Lv.pk_ids, ids.data(), ids.size()));
-  PM_TRY(upload(h, &Lv.pk_flips, flips.data(), flips.size()));
+  PM_TRY(dalloc(h, &Lv.pk_ids, nc * kPatchIds));
+  PM_TRY(dalloc(h, &Lv.pk_flips, (size_t)Lv.nu));
   PM_TRY(dalloc(h, &u, (size_t)Lv.nu * 12 * sizeof(T)));
   Lv.pk_u = u;
   PM_TRY(dalloc(h, &p, (size_t)Lv.np * 2 * sizeof(T)));
   Lv.pk_p = p;
-  PM_TRY(dalloc(h, &val, nc * kPatchValues * sizeof(T)));
+  PM_TRY(dalloc(h, &val, room));
   Lv.pk_values = val;
-  // one pattern per hash value; the values array is the scratch of this step
+  // one pattern per hash value; the values array is the scratch of these steps
   unsigned long long *d_hash = reinterpret_cast<unsigned long long *>(val);
   int *d_which = reinterpret_cast<int *>(d_hash + nc), *d_pattern = d_which + nc;
   int *bad_d = h->status_d + 2, bad = 0;
@@ -740,6 +736,14 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   };
   if (cudaMemsetAsync(bad_d, 0, sizeof(int), h->stream) != cudaSuccess)
     return cuda_fail(h, "patch flag");
+  std::vector<int> colour(nc, -1);
+  for (size_t k = 0; k + 1 < Lv.colouring.ptr.size(); ++k)
+    for (int q = Lv.colouring.ptr[k]; q < Lv.colouring.ptr[k + 1]; ++q)
+      colour[(size_t)Lv.colouring.order[(size_t)q]] = (int)k;
+  PM_LAUNCH(launch_patch_lists(Lv.cells(), Lv.nu, Lv.np, colour.data(), Lv.pk_ids, Lv.pk_flips, val,
+                               bad_d, h->stream));
+  PM_TRY(check());
+  if (bad) return PM_OK;
   PM_LAUNCH(launch_patch_pattern<T>(0, Lv.pk_ids, op, Lv.ncells, nullptr, nullptr, d_hash, bad_d,
                                     h->stream));
   std::vector<unsigned long long> hash(nc);
@@ -751,9 +755,12 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   std::unordered_map<unsigned long long, int> seen;
   std::vector<int> which, pattern(nc);
   for (size_t c = 0; c < nc; ++c) {
-    const auto it = seen.emplace(hash[c], (int)which.size());
-    if (it.second) which.push_back((int)c);
-    pattern[c] = it.first->second;
+    auto it = seen.find(hash[c]);
+    if (it == seen.end()) {
+      it = seen.emplace(hash[c], (int)which.size()).first;
+      which.push_back((int)c);
+    }
+    pattern[c] = it->second;
   }
   PM_TRY(dalloc(h, &pat, which.size() * kPatchPatternBytes));
   Lv.pk_patterns = pat;

@@ -234,6 +234,14 @@ struct PatchLevel {
   void *f;                 // right-hand side, 4 values per node
   T *fp;                   // and its pressure part
 };
+// Patch lists of a level and the nodes that change copies from sweep to
+// sweep.  colour: of every cell, on the host; scratch: patch_list_scratch
+// bytes; *bad |= 1 when a cell's neighbourhood does not have the canonical
+// shape (more than one neighbour beyond a face, edge or vertex, repeated
+// nodes, shared or unaligned pressure DOFs).
+size_t patch_list_scratch(int ncells, int nu, int np);
+int launch_patch_lists(const DevCells &cells, int nu, int np, const int *colour, int *ids,
+                       unsigned char *flips, void *scratch, int *bad, cudaStream_t s);
 // the level's CSR values into the packed layout
 template <typename T>
 int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cudaStream_t s);

@@ -2,7 +2,6 @@
 #include "pm_setup_host.h"
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -502,97 +501,6 @@ void row_order(const int *rowptr, int rows, std::vector<int> &order) {
     for (int c = 0; c < kClasses; ++c) at[c + 1] += at[c];
     for (int i = w; i < e; ++i) order[(size_t)(w + at[cls(i)]++)] = i;
   }
-}
-
-bool build_patches(int ncells, const int *udofs, const int *pdofs, int nu, int np,
-                   const Colouring &col, std::vector<int> &ids,
-                   std::vector<unsigned char> &flips) {
-  constexpr int NB = 26, NODES = 343, COUNT = 343, OWN = 344, SINGLE = 371, BASE = 372;
-  constexpr int stride = kPatchIdsHost;
-  if (nu >= (1 << 29) || np % 4) return false;
-  std::vector<unsigned char> seen((size_t)np, 0);
-  for (int c = 0; c < ncells; ++c) {
-    const int *p = pdofs + (size_t)c * 4;
-    if (p[0] % 4) return false;
-    for (int m = 0; m < 4; ++m) {
-      if (p[m] != p[0] + m || seen[p[m]]) return false;
-      seen[p[m]] = 1;
-    }
-  }
-  std::vector<int> ptr, ent, colour((size_t)ncells, -1);
-  incidence(ncells, 27, udofs, nu, ptr, ent);
-  for (size_t k = 0; k + 1 < col.ptr.size(); ++k)
-    for (int q = col.ptr[k]; q < col.ptr[k + 1]; ++q) colour[col.order[(size_t)q]] = (int)k;
-  flips.assign((size_t)nu, 0);
-  for (int i = 0; i < nu; ++i) {
-    const int m = ptr[i + 1] - ptr[i];
-    flips[i] = m > 1 && (m & 1);
-  }
-  struct Feature {
-    int pivot;             // its middle node
-    std::vector<int> sup;  // features that contain it (their neighbours touch it too)
-  };
-  std::vector<Feature> feat;
-  std::vector<std::array<int, 3>> fix;
-  patch_features([&](const int *c) { fix.push_back({c[0], c[1], c[2]}); });
-  for (int f = 0; f < NB; ++f) {
-    Feature F;
-    int k[3];
-    for (int d = 0; d < 3; ++d) k[d] = fix[f][d] < 0 ? 1 : fix[f][d];
-    F.pivot = k[0] + 3 * k[1] + 9 * k[2];
-    for (int g = 0; g < f; ++g) {
-      bool in = true;
-      for (int d = 0; d < 3; ++d) in = in && (fix[g][d] < 0 || fix[g][d] == fix[f][d]);
-      if (in) F.sup.push_back(g);
-    }
-    feat.push_back(F);
-  }
-  ids.assign((size_t)ncells * stride, 0);
-  bool good = true;
-#pragma omp parallel for schedule(static, 64) reduction(&& : good)
-  for (int c = 0; c < ncells; ++c) {
-    int nodes[NODES + 27 * NB], nb[NB], n = 0;
-    bool ok = true;
-    for (int k = 0; k < 27; ++k) nodes[n++] = udofs[(size_t)c * 27 + k];
-    for (int f = 0; f < NB && ok; ++f) {
-      const int pv = udofs[(size_t)c * 27 + feat[f].pivot];
-      nb[f] = -1;
-      for (int e = ptr[pv]; e < ptr[pv + 1]; ++e) {
-        const int o = ent[e] / 27;
-        bool known = o == c;
-        for (int g : feat[f].sup) known = known || nb[g] == o;
-        if (known) continue;
-        ok = ok && (nb[f] < 0 || nb[f] == o);
-        nb[f] = o;
-      }
-      if (nb[f] < 0) continue;
-      for (int k = 0; k < 27; ++k) nodes[n++] = udofs[(size_t)nb[f] * 27 + k];
-    }
-    if (ok) {
-      std::sort(nodes, nodes + n);
-      n = (int)(std::unique(nodes, nodes + n) - nodes);
-      ok = n <= NODES;
-    }
-    good = good && ok;
-    if (!ok) continue;
-    int *out = ids.data() + (size_t)c * stride;
-    auto entry = [&](int id) {
-      const int m = ptr[id + 1] - ptr[id];
-      int before = 0;  // updates of this node by earlier colours of a sweep
-      for (int e = ptr[id]; e < ptr[id + 1]; ++e) before += colour[ent[e] / 27] < colour[c];
-      return (id << 2) | (m > 1 ? ((m & 1) << 1) | (before & 1) : 0);
-    };
-    for (int q = 0; q < NODES; ++q) out[q] = entry(nodes[q < n ? q : 0]);
-    out[COUNT] = n;
-    for (int k = 0; k < 27; ++k) {
-      const int id = udofs[(size_t)c * 27 + k];
-      out[OWN + k] = entry(id);
-      if (ptr[id + 1] - ptr[id] == 1) out[SINGLE] |= 1 << k;
-    }
-    out[BASE] = pdofs[(size_t)c * 4];
-    for (int f = 0; f < NB; ++f) out[BASE + 1 + f] = pdofs[(size_t)(nb[f] < 0 ? c : nb[f]) * 4];
-  }
-  return good;
 }
 
 }  // namespace pm

@@ -50,28 +50,6 @@ void build_neighbours(int ncells, const int *udofs, int nu, std::vector<int> &nb
 // 1 / (number of cells containing each velocity node)
 void node_inverse_multiplicity(int ncells, const int *udofs, int nu, std::vector<float> &inv);
 
-// Features of a Q2 cell: 6 faces, 12 edges, 8 vertices, each by its fixed
-// local coordinates (0 or 2; -1: free).
-template <typename F>
-void patch_features(F &&f) {
-  for (int fixed = 1; fixed <= 3; ++fixed)
-    for (int c = 0; c < 27; ++c) {
-      const int d[3] = {c % 3 - 1, (c / 3) % 3 - 1, c / 9 - 1};
-      if ((d[0] != 0) + (d[1] != 0) + (d[2] != 0) != fixed) continue;
-      const int k[3] = {d[0] ? d[0] + 1 : -1, d[1] ? d[1] + 1 : -1, d[2] ? d[2] + 1 : -1};
-      f(k);
-    }
-}
-// Patch entries of every cell (ids: ncells x kPatchIds, see pm_kernels.h) and
-// the nodes that change copies from sweep to sweep.  False when a cell's
-// neighbourhood does not have the canonical shape (more than one neighbour
-// beyond a face, edge or vertex, repeated nodes, shared or unaligned
-// pressure DOFs).
-bool build_patches(int ncells, const int *udofs, const int *pdofs, int nu, int np,
-                   const Colouring &col, std::vector<int> &ids,
-                   std::vector<unsigned char> &flips);
-constexpr int kPatchIdsHost = 400;  // kPatchIds
-
 // Rows of a CSR pattern by descending length class (16 entries) within
 // windows of 4096 rows, in their order otherwise.
 void row_order(const int *rowptr, int rows, std::vector<int> &order);

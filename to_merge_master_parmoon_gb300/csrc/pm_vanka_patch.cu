@@ -46,6 +46,7 @@
 
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cstdint>
 #include <vector>
 
@@ -995,6 +996,172 @@ __global__ void __launch_bounds__(256) k_patch_pack(PatchLevel<T> L, DevOp<T> op
     reinterpret_cast<float4 *>(V)[i] = reinterpret_cast<const float4 *>(stage)[i];
 }
 
+// Cells of every velocity node (slots: the first eight, cnt: all) and the
+// owner count of every pressure block; *bad when a node lies in more than
+// eight cells or a cell's pressure DOFs are not one aligned block of its own.
+__global__ void k_patch_incidence(int ncells, const int *udofs, const int *pdofs, int *cnt,
+                                  int *slots, int *owners, int *bad) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells * NU_LOC;
+       i += gridDim.x * blockDim.x) {
+    const int c = i / NU_LOC, k = i - c * NU_LOC, id = udofs[i], at = atomicAdd(cnt + id, 1);
+    bool wrong = at >= 8;
+    if (!wrong) slots[8 * (size_t)id + at] = c;
+    if (k < NP_LOC) {
+      const int base = pdofs[NP_LOC * (size_t)c];
+      wrong = wrong || base % NP_LOC || pdofs[NP_LOC * (size_t)c + k] != base + k;
+      if (k == 0 && atomicAdd(owners + base / NP_LOC, 1)) wrong = true;
+    }
+    if (wrong) atomicOr(bad, 1);
+  }
+}
+
+// Features of a Q2 cell, 6 faces, 12 edges, 8 vertices: the middle node, and
+// the features that contain it (whose neighbours touch it too).
+__host__ __device__ constexpr bool feature_coords(int f, int d[3]) {
+  for (int fixed = 1; fixed <= 3; ++fixed)
+    for (int c = 0; c < 27; ++c) {
+      d[0] = c % 3 - 1;
+      d[1] = (c / 3) % 3 - 1;
+      d[2] = c / 9 - 1;
+      if ((d[0] != 0) + (d[1] != 0) + (d[2] != 0) == fixed && f-- == 0) return true;
+    }
+  return false;
+}
+struct Features {
+  int pivot[26], sup[26];
+};
+constexpr Features make_features() {
+  Features F = {};
+  for (int f = 0; f < 26; ++f) {
+    int d[3] = {}, e[3] = {};
+    feature_coords(f, d);
+    F.pivot[f] = d[0] + 1 + 3 * (d[1] + 1) + 9 * (d[2] + 1);
+    for (int g = 0; g < f; ++g) {
+      feature_coords(g, e);
+      bool in = true;
+      for (int k = 0; k < 3; ++k) in = in && (e[k] == 0 || e[k] == d[k]);
+      if (in) F.sup[f] |= 1 << g;
+    }
+  }
+  return F;
+}
+__constant__ Features c_feat = make_features();
+
+// Patch list of a cell, once per level at set-up: its neighbours by feature
+// (faces, then edges, then vertices; *bad when more than one lies beyond a
+// feature), their nodes sorted and made unique.  On the host (16 threads) the
+// lists and their upload took 80 ms at 32^3, in a set-up of 119 ms now.
+__global__ void __launch_bounds__(256) k_patch_list(int ncells, const int *udofs, const int *pdofs,
+                                                    const int *cnt, const int *slots,
+                                                    const int *colour, int *ids, int *bad) {
+  __shared__ int key[1024], list[kPatchNodes], nb[26], part[8];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, c = blockIdx.x;
+  const int *own = udofs + (size_t)c * NU_LOC;
+  if (warp == 0) {
+    const int f = lane < 26 ? lane : 25, pv = own[c_feat.pivot[f]], sup = c_feat.sup[f];
+    const int rank = f < 6 ? 0 : (f < 18 ? 1 : 2), m = cnt[pv] < 8 ? cnt[pv] : 8;
+    bool two = false;
+    for (int r = 0; r < 3; ++r) {
+      if (lane < 26 && rank == r) {
+        int mine = -1;
+        for (int e = 0; e < m; ++e) {
+          const int o = slots[8 * (size_t)pv + e];
+          bool known = o == c;
+          for (int g = 0; g < 18; ++g) known = known || ((sup >> g & 1) && nb[g] == o);
+          if (known) continue;
+          two = two || (mine >= 0 && mine != o);
+          mine = o;
+        }
+        nb[lane] = mine;
+      }
+      __syncwarp();
+    }
+    if (two) atomicOr(bad, 1);
+  }
+  __syncthreads();
+  for (int i = t; i < 1024; i += 256) {
+    const int q = i / NU_LOC, k = i - q * NU_LOC;
+    int v = INT_MAX;
+    if (q == 0)
+      v = own[k];
+    else if (q <= 26 && nb[q - 1] >= 0)
+      v = udofs[(size_t)nb[q - 1] * NU_LOC + k];
+    key[i] = v;
+  }
+  for (int size = 2; size <= 1024; size *= 2)
+    for (int step = size / 2; step > 0; step /= 2) {
+      __syncthreads();
+      for (int i = t; i < 512; i += 256) {
+        const int lo = 2 * i - (i & (step - 1)), hi = lo + step;
+        const int a = key[lo], b = key[hi];
+        if ((a > b) == ((lo & size) == 0)) {
+          key[lo] = b;
+          key[hi] = a;
+        }
+      }
+    }
+  __syncthreads();
+  // the first of each run of equal nodes, in order
+  bool first[4];
+  int n = 0;
+  for (int q = 0; q < 4; ++q) {
+    const int i = 4 * t + q;
+    first[q] = key[i] != INT_MAX && (i == 0 || key[i] != key[i - 1]);
+    n += first[q];
+  }
+  int before = n;
+  for (int o = 1; o < 32; o *= 2) {
+    const int v = __shfl_up_sync(kFull, before, o);
+    if (lane >= o) before += v;
+  }
+  if (lane == 31) part[warp] = before;
+  __syncthreads();
+  int total = 0;
+  for (int w = 0; w < 8; ++w) {
+    if (w == warp) before += total - n;
+    total += part[w];
+  }
+  for (int q = 0; q < 4; ++q)
+    if (first[q]) {
+      if (before < kPatchNodes) list[before] = key[4 * t + q];
+      ++before;
+    }
+  __syncthreads();
+  if (total > kPatchNodes) {
+    if (t == 0) atomicOr(bad, 1);
+    return;
+  }
+  int *out = ids + (size_t)c * kPatchIds;
+  const int col = colour[c];
+  auto entry = [&](int id) {  // with the updates by earlier colours of a sweep
+    const int m = cnt[id];
+    int up = 0;
+    for (int e = 0; e < m && e < 8; ++e) up += colour[slots[8 * (size_t)id + e]] < col;
+    return (id << 2) | (m > 1 ? ((m & 1) << 1) | (up & 1) : 0);
+  };
+  for (int q = t; q < kPatchNodes; q += 256) out[q] = entry(list[q < total ? q : 0]);
+  if (warp == 0) {
+    const int id = own[lane < NU_LOC ? lane : 0];
+    if (lane < NU_LOC) out[kPatchOwn + lane] = entry(id);
+    const unsigned single = __ballot_sync(kFull, lane < NU_LOC && cnt[id] == 1);
+    if (lane == 0) {
+      out[kPatchCount] = total;
+      out[kPatchSingle] = (int)single;
+      out[kPatchPattern] = 0;
+    }
+    if (lane < 27) {
+      const int o = lane == 0 || nb[lane - 1] < 0 ? c : nb[lane - 1];
+      out[kPatchBase + lane] = pdofs[NP_LOC * (size_t)o];
+    }
+  }
+}
+
+// nodes that change copies from sweep to sweep: an odd number > 1 of updates
+__global__ void k_patch_flips(int nu, const int *cnt, unsigned char *flips) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nu; i += gridDim.x * blockDim.x)
+    flips[i] = cnt[i] > 1 && (cnt[i] & 1);
+}
+
 __global__ void k_patch_assign(int *ids, const int *pattern, int ncells) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < ncells) ids[(size_t)c * kPatchIds + kPatchPattern] = pattern[c];
@@ -1229,6 +1396,27 @@ void patch_places(void *patterns, long long count) {
     for (uint16_t &e : pt.own) e = (uint16_t)(16 * place[e / 16]);
     for (int n = 0; n <= N; ++n) pt.place[n] = place[n];
   }
+}
+
+size_t patch_list_scratch(int ncells, int nu, int np) {
+  return sizeof(int) * (9 * (size_t)nu + (size_t)np / NP_LOC + (size_t)ncells);
+}
+
+int launch_patch_lists(const DevCells &cells, int nu, int np, const int *colour, int *ids,
+                       unsigned char *flips, void *scratch, int *bad, cudaStream_t s) {
+  if (cells.ncells <= 0) return 0;
+  int *slots = static_cast<int *>(scratch), *cnt = slots + 8 * (size_t)nu, *owners = cnt + nu,
+      *col = owners + np / NP_LOC;
+  if (cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)nu + np / NP_LOC), s) != cudaSuccess ||
+      cudaMemcpyAsync(col, colour, sizeof(int) * (size_t)cells.ncells, cudaMemcpyHostToDevice,
+                      s) != cudaSuccess)
+    return -1;
+  k_patch_incidence<<<node_grid(cells.ncells * NU_LOC), 256, 0, s>>>(
+      cells.ncells, cells.udofs, cells.pdofs, cnt, slots, owners, bad);
+  k_patch_list<<<cells.ncells, 256, 0, s>>>(cells.ncells, cells.udofs, cells.pdofs, cnt, slots, col,
+                                            ids, bad);
+  k_patch_flips<<<node_grid(nu), 256, 0, s>>>(nu, cnt, flips);
+  return cudaPeekAtLastError() == cudaSuccess ? 3 : -1;
 }
 
 int launch_patch_assign(int *ids, const int *pattern, int ncells, cudaStream_t s) {
