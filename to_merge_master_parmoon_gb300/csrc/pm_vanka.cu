@@ -860,55 +860,77 @@ __global__ void __launch_bounds__(((NU + 3) / 4 + 1) * 32) k_vanka_residual_spli
   if (valid && sl < 3) R[sl * NU_LOC + a] = f - (sl == 0 ? s[0] : (sl == 1 ? s[1] : s[2]));
 }
 
-// The flattened-stream residual with one CTA of eight warps per cell, for
-// colours that do not fill the GPU: the stream's blocks of 32 groups are
-// shared out over the warps and the blocks' row sums added in the order of
-// k_vanka_residual (a row of at most 32 groups meets at most two blocks).
-constexpr int kWideWarps = 8;
+// The flattened-stream residual with one CTA per cell, for colours that do
+// not fill the GPU: the stream's blocks of 32 groups are shared out over the
+// warps and the blocks' row sums added in the order of k_vanka_residual (a
+// row of at most 32 groups meets at most two blocks).  A cell of a uniform
+// mesh has 18 + 5 + 1 blocks: with 24 warps their matrix data are in registers
+// before the launch waits, and what follows the wait is one gather and the
+// sums (7.0 us at 8 cells, cold caches; 12.0 with eight warps, which load
+// three blocks each).
 constexpr int kWideBlocks = 2;  // blocks a row may meet, per part
+template <typename T, int VEC>
+struct WideBlock {
+  int seg;
+  long long e0;
+  int ci[VEC];
+  T v[9][VEC];
+};
 template <typename T, int MODE, int VEC>
-__device__ __forceinline__ void wide_rows(const SegTab &t, int nseg, int total, int base,
+__device__ __forceinline__ void wide_load(const SegTab &t, int nseg, int total, int base,
                                           const int *__restrict__ col, const T *const *vals,
+                                          WideBlock<T, VEC> &B, int lane) {
+  const int g = base + lane;
+  B.seg = -1;
+  if (g >= total) return;
+  B.seg = find_seg(t.off, nseg, g);
+  const long long gq = (long long)t.qs[B.seg] + (g - t.off[B.seg]);
+  B.e0 = gq * VEC;
+  VecLd<T, VEC>::idx(col + gq * VEC, B.ci);
+#pragma unroll
+  for (int k = 0; k < (MODE == 0 ? 9 : 3); ++k) VecLd<T, VEC>::val(vals[k] + gq * VEC, B.v[k]);
+}
+template <typename T, int MODE, int VEC>
+__device__ __forceinline__ void wide_rows(const SegTab &t, int base, const WideBlock<T, VEC> &B,
                                           const T *__restrict__ x0, const T *__restrict__ x1,
                                           const T *__restrict__ x2, T *part, int lane) {
-  constexpr int NV = MODE == 0 ? 9 : 3, NO = MODE == 2 ? 1 : 3;
-  const int g = base + lane;
-  int seg = -1;
-  long long gq = 0;
-  if (g < total) {
-    seg = find_seg(t.off, nseg, g);
-    gq = (long long)t.qs[seg] + (g - t.off[seg]);
-  }
+  constexpr int NO = MODE == 2 ? 1 : 3;
+  const int seg = B.seg;
   T s[NO];
 #pragma unroll
   for (int k = 0; k < NO; ++k) s[k] = T(0);
   if (seg >= 0) {
-    int ci[VEC];
-    T v[NV][VEC];
-    VecLd<T, VEC>::idx(col + gq * VEC, ci);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) VecLd<T, VEC>::val(vals[k] + gq * VEC, v[k]);
-    const long long e0 = gq * VEC;
     const int lo = t.rs[seg], hi = t.re[seg];
+    // no branches: entries of other rows gather index 0 and are left out
+    T x[VEC][3];
+    bool in[VEC];
 #pragma unroll
     for (int m = 0; m < VEC; ++m) {
-      const long long e = e0 + m;
-      if (e >= lo && e < hi) {
-        const int c = ci[m];
-        if constexpr (MODE == 1) {
-          const T g0 = __ldcg(x0 + c);
-          s[0] += v[0][m] * g0;
-          s[1 % NO] += v[1][m] * g0;
-          s[2 % NO] += v[2][m] * g0;
-        } else {
-          const T g0 = __ldcg(x0 + c), g1 = __ldcg(x1 + c), g2 = __ldcg(x2 + c);
-          s[0] += dot3(v[0][m], g0, v[1][m], g1, v[2][m], g2);
-          if constexpr (MODE == 0) {
-            s[1 % NO] += dot3(v[3][m], g0, v[4][m], g1, v[5][m], g2);
-            s[2 % NO] += dot3(v[6][m], g0, v[7][m], g1, v[8][m], g2);
-          }
+      in[m] = B.e0 + m >= lo && B.e0 + m < hi;
+      const int c = in[m] ? B.ci[m] : 0;
+      x[m][0] = __ldcg(x0 + c);
+      if constexpr (MODE != 1) {
+        x[m][1] = __ldcg(x1 + c);
+        x[m][2] = __ldcg(x2 + c);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < VEC; ++m) {
+      const T g0 = x[m][0], g1 = x[m][1], g2 = x[m][2];
+      T n[3] = {s[0], s[1 % NO], s[2 % NO]};
+      if constexpr (MODE == 1) {
+        n[0] += B.v[0][m] * g0;
+        n[1] += B.v[1][m] * g0;
+        n[2] += B.v[2][m] * g0;
+      } else {
+        n[0] += dot3(B.v[0][m], g0, B.v[1][m], g1, B.v[2][m], g2);
+        if constexpr (MODE == 0) {
+          n[1] += dot3(B.v[3][m], g0, B.v[4][m], g1, B.v[5][m], g2);
+          n[2] += dot3(B.v[6][m], g0, B.v[7][m], g1, B.v[8][m], g2);
         }
       }
+#pragma unroll
+      for (int k = 0; k < NO; ++k) s[k] = in[m] ? n[k] : s[k];
     }
   }
 #pragma unroll
@@ -928,8 +950,8 @@ __device__ __forceinline__ void wide_rows(const SegTab &t, int nseg, int total, 
   }
 }
 
-template <typename T, int VEC>
-__global__ void __launch_bounds__(kWideWarps * 32) k_vanka_residual_wide(
+template <typename T, int VEC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_vanka_residual_wide(
     DevOp<T> op, DevCells cells, const int *__restrict__ list, const T *__restrict__ u,
     const T *__restrict__ rhs, T *__restrict__ rbuf) {
   __shared__ int s_tab[3][4][32], s_total[3];
@@ -938,7 +960,7 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_vanka_residual_wide(
   start_next();
   const int slot = blockIdx.x, cell = __ldg(list + slot), nu = op.nu;
   const T *u1 = u, *u2 = u + nu, *u3 = u + 2 * nu, *p = u + 3 * nu;
-  for (int i = t; i < kWideBlocks * 3 * 32; i += kWideWarps * 32) {
+  for (int i = t; i < kWideBlocks * 3 * 32; i += WARPS * 32) {
     s_part[0][i] = T(0);
     s_part[1][i] = T(0);
     if (i < kWideBlocks * 32) s_p[i] = T(0);
@@ -965,18 +987,28 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_vanka_residual_wide(
     f = __ldcg(rhs + at);
   }
   __syncthreads();
-  wait_previous();
   const int na = (s_total[0] + 31) / 32, nt = (s_total[1] + 31) / 32, nb = (s_total[2] + 31) / 32;
-  for (int k = warp; k < na + nt + nb; k += kWideWarps) {
+  WideBlock<T, VEC> B;
+  auto load = [&](int k) {
     if (k < na)
-      wide_rows<T, 0, VEC>(tab(0), NU_LOC, s_total[0], 32 * k, op.a_col, op.a, u1, u2, u3,
-                           s_part[0], lane);
+      wide_load<T, 0, VEC>(tab(0), NU_LOC, s_total[0], 32 * k, op.a_col, op.a, B, lane);
     else if (k < na + nt)
-      wide_rows<T, 1, VEC>(tab(1), NU_LOC, s_total[1], 32 * (k - na), op.bt_col, op.bt, p, p, p,
-                           s_part[1], lane);
+      wide_load<T, 1, VEC>(tab(1), NU_LOC, s_total[1], 32 * (k - na), op.bt_col, op.bt, B, lane);
     else
-      wide_rows<T, 2, VEC>(tab(2), NP_LOC, s_total[2], 32 * (k - na - nt), op.b_col, op.b, u1, u2,
-                           u3, s_p, lane);
+      wide_load<T, 2, VEC>(tab(2), NP_LOC, s_total[2], 32 * (k - na - nt), op.b_col, op.b, B, lane);
+  };
+  int k = warp;
+  if (k < na + nt + nb) load(k);
+  wait_previous();
+  while (k < na + nt + nb) {
+    if (k < na)
+      wide_rows<T, 0, VEC>(tab(0), 32 * k, B, u1, u2, u3, s_part[0], lane);
+    else if (k < na + nt)
+      wide_rows<T, 1, VEC>(tab(1), 32 * (k - na), B, p, p, p, s_part[1], lane);
+    else
+      wide_rows<T, 2, VEC>(tab(2), 32 * (k - na - nt), B, u1, u2, u3, s_p, lane);
+    k += WARPS;
+    if (k < na + nt + nb) load(k);
   }
   __syncthreads();
   if (t < NLOC) {
@@ -1993,6 +2025,9 @@ int launch_vanka_factor(const DevOp<double> &op, const DevCells &cells, TF *fact
 
 // Cells of a colour up to which the residual runs with one CTA per cell.
 constexpr int kSplitCells = 2048;
+// Cells up to which the wide residual has a warp per block of its stream (one
+// CTA per SM): 8.1 us against 13.5 at 64 cells, but 28.4 against 24.6 at 512.
+constexpr int kWideCells = 152;
 
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
@@ -2025,7 +2060,8 @@ int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *
     }
     if constexpr (sizeof(T) == 4) {
       if (cells.nl == NU_LOC && !op.structured && !op.diag && max_row + VEC - 1 <= 32 * VEC)
-        return split(k_vanka_residual_wide<T, VEC>, kWideWarps - 1);
+        return ncol <= kWideCells ? split(k_vanka_residual_wide<T, VEC, 24>, 23)
+                                  : split(k_vanka_residual_wide<T, VEC, 8>, 7);
     }
   }
   if (cells.nl == NU_TET) {  // tetrahedra: the row-group kernel
