@@ -1301,7 +1301,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_vanka_apply2(
 // memory by one bulk copy before the launch waits for the residual, so that
 // the substitution's steps wait for shared memory only.  Loading columns from
 // global memory on the way took 11 us (tetrahedra) and 25 us per launch of
-// any size.  Same operations in the same order as k_vanka_apply.
+// any size (now 6 and 8 with cold caches).  Same operations in the same order as k_vanka_apply.
 template <typename T, int NU>
 __global__ void __launch_bounds__(32) k_vanka_apply_staged(
     DevCells cells, int nu, const int *__restrict__ list, const T *__restrict__ F,
@@ -1309,6 +1309,7 @@ __global__ void __launch_bounds__(32) k_vanka_apply_staged(
     int *err) {
   constexpr int NU_LOC = NU, NLOC = Elem<NU>::nloc, kFacStride = Elem<NU>::fac_stride,
                 kRStride = Elem<NU>::r_stride, SL = (NLOC + 31) / 32;
+  static_assert(NLOC % 4 == 1, "blocks of four columns and one");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const T *Fs = reinterpret_cast<const T *>(smem_raw);
   __shared__ uint64_t bar;
@@ -1347,35 +1348,122 @@ __global__ void __launch_bounds__(32) k_vanka_apply_staged(
     y[q] = lane + 32 * q < NLOC ? __ldcg(R + pr[q]) : T(0);
     o[q] = lane + 32 * q < NLOC ? __ldcg(u + dof[q]) : T(0);
   }
-  // forward substitution with the unit lower factor
+  if constexpr (sizeof(T) == sizeof(float)) {
+    // Blocks of four columns: every lane solves the block's 4 x 4 triangle for
+    // itself, so that a block waits for one round of shuffles instead of four,
+    // and applies the four columns to its rows in their order.
+    struct Block {
+      T c[4][SL], d[4], t[6];
+    };
+    auto fetch = [&](int j0, int dir, Block &B) {  // columns j0, j0 + dir, ...
+      int m = 0;
 #pragma unroll
-  for (int jb = 0; jb < SL; ++jb) {
-    const int je = jb == SL - 1 ? NLOC - 1 : 32 * jb + 32;
-#pragma unroll 4
-    for (int j = 32 * jb; j < je; ++j) {
-      const T *col = Fs + j * NLOC;
-      const T yj = __shfl_sync(kFull, y[jb], j & 31);
+      for (int k = 0; k < 4; ++k) {
+        const int j = j0 + dir * k;
+        const T *col = Fs + j * NLOC;
+        B.d[k] = col[j];
 #pragma unroll
-      for (int q = 0; q < SL; ++q) {
-        const int i = lane + 32 * q;
-        const T l = (i > j && i < NLOC) ? col[i] : T(0);
-        y[q] -= l * yj;
+        for (int l = k + 1; l < 4; ++l) B.t[m++] = col[j0 + dir * l];
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          const int i = lane + 32 * q;
+          B.c[k][q] = (dir > 0 ? i > j && i < NLOC : i < j) ? col[i] : T(0);
+        }
+      }
+    };
+    // forward substitution with the unit lower factor
+    Block cur;
+    fetch(0, 1, cur);
+#pragma unroll
+    for (int jb = 0; jb < SL; ++jb) {
+      const int je = jb == SL - 1 ? NLOC - 1 : 32 * jb + 32;
+#pragma unroll 2
+      for (int j = 32 * jb; j < je; j += 4) {
+        const Block B = cur;
+        T x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = __shfl_sync(kFull, y[jb], (j + k) & 31);
+        if (j + 4 < NLOC - 1) fetch(j + 4, 1, cur);
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int l = k + 1; l < 4; ++l) x[l] -= B.t[m++] * x[k];
+#pragma unroll
+          for (int q = 0; q < SL; ++q) y[q] -= B.c[k][q] * x[k];
+        }
       }
     }
-  }
-  // back substitution with U (diagonal stores 1/U_jj)
-#pragma unroll
-  for (int jb = SL - 1; jb >= 0; --jb) {
-    const int jt = jb == SL - 1 ? NLOC - 1 : 32 * jb + 31;
-#pragma unroll 4
-    for (int j = jt; j >= 32 * jb; --j) {
+    // back substitution with U (diagonal stores 1/U_jj): the last column, then
+    // blocks of four
+    {
+      constexpr int j = NLOC - 1;
+      fetch(j - 1, -1, cur);
       const T *col = Fs + j * NLOC;
-      if (lane == (j & 31)) y[jb] *= col[j];
-      const T xj = __shfl_sync(kFull, y[jb], j & 31);
+      if (lane == (j & 31)) y[SL - 1] *= col[j];
+      const T xj = __shfl_sync(kFull, y[SL - 1], j & 31);
 #pragma unroll
       for (int q = 0; q < SL; ++q) {
         const int i = lane + 32 * q;
         if (i < j) y[q] -= col[i] * xj;
+      }
+    }
+#pragma unroll
+    for (int jb = SL - 1; jb >= 0; --jb) {
+      const int jt = jb == SL - 1 ? NLOC - 2 : 32 * jb + 31;
+#pragma unroll 2
+      for (int j = jt; j >= 32 * jb; j -= 4) {
+        const Block B = cur;
+        T x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = __shfl_sync(kFull, y[jb], (j - k) & 31);
+        if (j >= 4) fetch(j - 4, -1, cur);
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          x[k] *= B.d[k];
+#pragma unroll
+          for (int l = k + 1; l < 4; ++l) x[l] -= B.t[m++] * x[k];
+#pragma unroll
+          for (int q = 0; q < SL; ++q)
+            if (lane + 32 * q < j - k) y[q] -= B.c[k][q] * x[k];
+          if (lane == ((j - k) & 31)) y[jb] = x[k];
+        }
+      }
+    }
+  } else {
+    // FP64: each instruction takes the pipe for 64 cycles, the triangles would
+    // cost more than the shuffles (43 us against 31 per launch, hexahedra)
+    // forward substitution with the unit lower factor
+#pragma unroll
+    for (int jb = 0; jb < SL; ++jb) {
+      const int je = jb == SL - 1 ? NLOC - 1 : 32 * jb + 32;
+#pragma unroll 4
+      for (int j = 32 * jb; j < je; ++j) {
+        const T *col = Fs + j * NLOC;
+        const T yj = __shfl_sync(kFull, y[jb], j & 31);
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          const int i = lane + 32 * q;
+          const T l = (i > j && i < NLOC) ? col[i] : T(0);
+          y[q] -= l * yj;
+        }
+      }
+    }
+    // back substitution with U (diagonal stores 1/U_jj)
+#pragma unroll
+    for (int jb = SL - 1; jb >= 0; --jb) {
+      const int jt = jb == SL - 1 ? NLOC - 1 : 32 * jb + 31;
+#pragma unroll 4
+      for (int j = jt; j >= 32 * jb; --j) {
+        const T *col = Fs + j * NLOC;
+        if (lane == (j & 31)) y[jb] *= col[j];
+        const T xj = __shfl_sync(kFull, y[jb], j & 31);
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          const int i = lane + 32 * q;
+          if (i < j) y[q] -= col[i] * xj;
+        }
       }
     }
   }
