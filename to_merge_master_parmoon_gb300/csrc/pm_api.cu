@@ -216,6 +216,8 @@ struct pm_handle {
   double *ydev = nullptr;
   int *status_d = nullptr;
   int *sweep_err = nullptr;  // device flags of bounded waits inside sweep kernels
+  // page-locked: [0] the flags, then the scalars of a read
+  double *host_read = nullptr;
   int *diag_flags = nullptr; // per level: an off-diagonal velocity block is nonzero
   bool asm_tables = false;   // assembly reference tables on the device
   int num_sms = 0;
@@ -365,12 +367,21 @@ bool mixed(const pm_handle *h) { return h->opt.precision == PM_PREC_MIXED; }
 // mixed mode stores each local block's FP32 inverse unless told otherwise
 bool use_inverse(const pm_handle *h) { return mixed(h) && h->opt.vanka_inverse != 0; }
 
+// The flags of bounded waits come with the synchronisation, through
+// page-locked memory: a pageable copy of the scalars and a second one of the
+// flags after it made three stops of the host per FGMRES iteration (solve at
+// 8^3 3.30 -> 3.16 ms, twelve of them stacked 5.24 -> 5.10).
+constexpr int kHostRead = 1024;
+
 pm_status sync(pm_handle *h, const char *what) {
+  const bool flags = h->sweep_err && h->host_read;
+  if (flags && cudaMemcpyAsync(h->host_read, h->sweep_err, sizeof(int), cudaMemcpyDeviceToHost,
+                               h->stream) != cudaSuccess)
+    return cuda_fail(h, what);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return cuda_fail(h, what);
-  if (h->sweep_err) {  // bounded device waits that gave up (bulk-copy barriers)
+  if (flags) {  // bounded device waits that gave up (bulk-copy barriers)
     int e = 0;
-    if (cudaMemcpy(&e, h->sweep_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
-      return cuda_fail(h, what);
+    std::memcpy(&e, h->host_read, sizeof(int));
     if (e) {
       cudaMemset(h->sweep_err, 0, sizeof(int));
       return fail(h, PM_TIMEOUT, std::string(what) + ": a bulk copy into shared memory did not "
@@ -903,10 +914,14 @@ pm_status defect_nse4(pm_handle *h, const double *x, const double *b, double *r)
 }
 
 pm_status read_scalars(pm_handle *h, double *dst, const double *src, int n) {
-  if (cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream) !=
+  const bool held = h->host_read && n < kHostRead;
+  double *to = held ? h->host_read + 1 : dst;
+  if (cudaMemcpyAsync(to, src, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream) !=
       cudaSuccess)
     return cuda_fail(h, "scalar read");
-  return sync(h, "scalar read");
+  PM_TRY(sync(h, "scalar read"));
+  if (held) std::memcpy(dst, to, sizeof(double) * n);
+  return PM_OK;
 }
 
 pm_status norm2(pm_handle *h, const double *x, int n, double *out) {
@@ -2012,6 +2027,9 @@ pm_status pm_setup(pm_handle *h) {
     return cuda_fail(h, "counter reset");
   PM_TRY(dalloc(h, &h->status_d, 4));
   PM_TRY(dalloc(h, &h->sweep_err, 4));
+  if (!h->host_read && cudaMallocHost(reinterpret_cast<void **>(&h->host_read),
+                                      kHostRead * sizeof(double)) != cudaSuccess)
+    return cuda_fail(h, "page-locked scalars");
   if (cudaMemsetAsync(h->sweep_err, 0, sizeof(int), h->stream) != cudaSuccess)
     return cuda_fail(h, "flag reset");
   if (mixed(h) && launch_vanka_apply_tma_init() < 0) return cuda_fail(h, "bulk-copy apply set-up");
@@ -2108,6 +2126,7 @@ pm_status pm_destroy(pm_handle *h) {
   for (cudaEvent_t e : h->evpool) cudaEventDestroy(e);
   for (void *p : h->allocs) cudaFree(p);
   for (void *p : h->pinned) cudaHostUnregister(p);
+  if (h->host_read) cudaFreeHost(h->host_read);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return PM_OK;
