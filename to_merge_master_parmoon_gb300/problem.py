@@ -124,7 +124,8 @@ class OseenProblem:
     def descs_one_block(self):
         """The same levels as NSTYPE-2 descriptors: a[0] carries the block of
         all three components, a[1..8] are NULL (TNSE_MGLevel2's one A
-        matrix).  Valid only when is_one_block(); shares this problem's arrays."""
+        matrix).  Valid only when is_one_block(); shares this problem's arrays
+        and keeps it alive."""
         if not self.is_one_block():
             raise ValueError("the velocity blocks are coupled or differ: not an NSTYPE-2 system")
         out = (PmLevelDesc * self.n_levels)()
@@ -132,6 +133,7 @@ class OseenProblem:
             C.pointer(out[level])[0] = self._descs[level]
             for k in range(1, 9):
                 out[level].a[k] = None
+        out.problem = self  # the descriptors point into its arrays
         return out
 
     def ndof(self, level: int = -1) -> int:
