@@ -182,15 +182,15 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-# DRAM bytes (read + write) per cell of one local-residual launch of the
-# headline kernel (k_vanka_residual_rows<float,1,1,8,27,true,true>: FP32, one
-# A block, interleaved velocity) from one ncu capture (dram__bytes_read.sum +
-# dram__bytes_write.sum = 136.83 + 2.90 MB) of a 32^3 colour launch of 4,096 cells:
-#   ncu --set full --clock-control none -k regex:'k_vanka_residual|k_schur_apply' -s 32 -c 2 \
+# DRAM bytes (read + write) per cell of one launch of the headline kernel
+# (k_patch_sweep32: a colour of a sweep from packed rows, residual, block
+# elimination and update) from one ncu capture (dram__bytes_read.sum +
+# dram__bytes_write.sum = 101.97 + 2.76 MB) of a 32^3 colour launch of 4,096 cells:
+#   ncu --set full --clock-control none -k regex:k_patch_sweep -s 16 -c 2 \
 #       python bench.py --only-sweep mixed --levels 5 --warmup 1 --steps 2
 # Traffic grows with the cells a launch processes (every cell reads its own
 # 27 rows), so it scales to a launch of any size.
-RESIDUAL_DRAM_BYTES_PER_CELL = 34114
+RESIDUAL_DRAM_BYTES_PER_CELL = 25570
 
 
 # the FP32 sweep kernels by level mode (0 nine blocks + LU, 1 three diagonal
@@ -204,9 +204,8 @@ def residual_kernel_name(mode, variant):
         return ("k_vanka_residual<float,4,1> (cell-local residuals over full CSR rows of one "
                 f"colour, flattened entry stream; {blocks}, BT, B)")
     if mode == 2:
-        return ("k_vanka_residual_rows<float,1,1,8,27,true,true> (cell-local residuals over full "
-                "CSR rows of one colour, 8 lanes per row, A and BT rows of a step loaded "
-                f"together, velocity gathered from its interleaved copy; {blocks}, BT, B)")
+        return ("k_patch_sweep32 (one colour of a sweep from packed rows: cell-local residuals, "
+                f"block elimination and update in one launch, persistent CTAs; {blocks}, BT, B)")
     kind = {0: 0, 1: 2}[mode]
     vec, ur = {0: (4, 1), 2: (1, 8)}[kind]
     return (f"k_vanka_residual_rows<float,{vec},{kind},{ur},27> (cell-local "
@@ -218,9 +217,8 @@ APPLY_KERNEL = {
        "registers and L2; substitution + update)",
     1: "k_schur_apply<float,3> (stored FP32 block elimination: three 27x27 inverses, B, A^-1 BT, "
        "4x4 Schur inverse; one cell per warp, GEMVs + update)",
-    2: "k_schur_apply<float,1,true> (stored FP32 block elimination: one 27x27 inverse, B, "
-       "A^-1 BT, 4x4 Schur inverse; one cell per warp, GEMVs + update of the interleaved "
-       "velocity)"}
+    2: "part of k_patch_sweep32 (stored FP32 block elimination: one 27x27 inverse, B, "
+       "A^-1 BT, 4x4 Schur inverse); no launch of its own"}
 
 
 def ncu_traffic(P):
@@ -1131,7 +1129,7 @@ def main():
     prof = results["mixed"].get("profile", {})
 
     def kernel_roof(d):
-        if not d or not d.get("ms"):
+        if not d or not d.get("ms") or not d.get("bytes"):
             return None, None, None
         return (d["bytes"] / (d["ms"] * 1e-3) / 1e9, d["ms"] / d["launches"],
                 d["bytes"] / d["launches"])
@@ -1168,6 +1166,10 @@ def main():
         if pr and pr["ms"]:
             t = pr["ms"] * 1e-3 / args.steps
             fl = 2.0 * sum(fma.values()) * sweeps
+            if not r64["profile"].get("apply", {}).get("bytes"):
+                # packed sweeps: the launch holds the block solve too
+                # (A^-1 r, D y, S^-1 and W: 3 x 729 + 324 + 16 + 324 FMA per cell)
+                fl += 2.0 * 2851 * sweeps * sum(P.desc(l).n_cells for l in range(1, P.n_levels))
             by = pr["bytes"] / args.steps
             res = {"flop_per_solve": fl, "achieved_tflops": fl / t / 1e12,
                    "fp64_frac": fl / t / rate.value, "hbm_frac": by / t / 1e9 / peak,
@@ -1198,7 +1200,7 @@ def main():
                     "sweep_kernels": {
                         k: {"ms_total": v["ms"], "launches": v["launches"],
                             "achieved_gbs": kernel_roof(v)[0],
-                            "frac": (kernel_roof(v)[0] / peak) if v["ms"] else None}
+                            "frac": (kernel_roof(v)[0] / peak) if kernel_roof(v)[0] else None}
                         for k, v in r.get("profile", {}).items()}}
     one = None
     if one_block:
@@ -1213,7 +1215,7 @@ def main():
                          "sweep_kernels": {
                              k: {"ms_total": v["ms"], "launches": v["launches"],
                                  "achieved_gbs": kernel_roof(v)[0],
-                                 "frac": (kernel_roof(v)[0] / peak) if v["ms"] else None}
+                                 "frac": (kernel_roof(v)[0] / peak) if kernel_roof(v)[0] else None}
                              for k, v in r.get("profile", {}).items()}}
         one["e2e"] = e2e1
     nlev = args.levels

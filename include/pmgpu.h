@@ -102,8 +102,10 @@ typedef struct {
                              sweep applies it as a GEMV; 0 (default) keeps
                              the FP32 LU factors and substitution            */
   int residual_variant;   /* local-residual kernel of the Vanka sweep:
-                             0 (default) per level: row groups (8 lanes per
-                             CSR row), except the flattened entry stream with
+                             0 (default) per level: packed rows on one-block
+                             hexahedral levels while memory allows, else row
+                             groups (8 lanes per CSR row), except the
+                             flattened entry stream with
                              segmented sums on FP32 levels that read all
                              nine A blocks (faster there); 1 row groups
                              everywhere; 2 the stream everywhere; -1 time
@@ -393,7 +395,9 @@ long long pm_pinned_bytes(pm_handle *h);
  * enabled: CUDA events on the handle's stream bracket every launch (the
  * V-cycle then runs without graph capture).  kernel 0 = local residual,
  * 1 = factor apply + update.  Totals since pm_profile_enable: device time
- * (ms), launches and algorithmic (unique) bytes of those launches. */
+ * (ms), launches and algorithmic (unique) bytes of those launches.  Levels
+ * that sweep from packed rows do both in one launch, counted under kernel 0
+ * (kernel 1: as many empty intervals, no bytes). */
 pm_status pm_profile_enable(pm_handle *h, int enable);
 pm_status pm_profile_read(pm_handle *h, int kernel, double *ms_total, long long *launches,
                           double *bytes_total);

@@ -731,8 +731,8 @@ int launch_csr_apply(const DevCsr<T> &m, int ncomp, const T *x, int x_stride, T 
   return ok() < 0 ? -1 : 1;
 }
 
-// One block for up to 2,048 cells (4 us instead of 6 + 3 for sum and
-// subtraction over the whole GPU; 9 us at 8,192), else a grid-wide sum.
+// One block for up to 2,048 cells (8 us with cold caches, and one launch, for
+// 6 + 3 us and two launches over the whole GPU), else a grid-wide sum.
 constexpr int kL20Small = 4 * 2048;
 template <typename T>
 int launch_l20_mean(const T *p, int np, double *scratch, unsigned int *counter, double *mean,
