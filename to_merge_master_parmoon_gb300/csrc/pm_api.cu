@@ -2032,6 +2032,7 @@ pm_status pm_setup(pm_handle *h) {
     return cuda_fail(h, "page-locked scalars");
   if (cudaMemsetAsync(h->sweep_err, 0, sizeof(int), h->stream) != cudaSuccess)
     return cuda_fail(h, "flag reset");
+  if (launch_vanka_init() < 0) return cuda_fail(h, "shared-memory limits");
   if (mixed(h) && launch_vanka_apply_tma_init() < 0) return cuda_fail(h, "bulk-copy apply set-up");
   h->restart = std::max(1, std::min(h->opt.restart, h->opt.maxit));
   PM_TRY(dalloc(h, &h->hcol, ((size_t)h->restart + 4) * h->nsys));

@@ -168,6 +168,10 @@ int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *
 int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, const int *cell_list,
                               int ncol, const float *u, const float4 *ux, const float *rhs,
                               float *rbuf, cudaStream_t s);
+// Limits of dynamic shared memory of the apply and coarse kernels, the largest
+// each can take: the limit belongs to the function and handles of several
+// threads share it, so no launch may lower it again.
+int launch_vanka_init();
 // Local solve with the stored factors and u[dofs] += damp * delta, for the
 // same cells (run after launch_vanka_residual of the whole colour).  pairs:
 // two cells per warp (half-warp per cell) instead of one.

@@ -2210,6 +2210,34 @@ int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, con
   return ok() < 0 ? -1 : 1;
 }
 
+int launch_vanka_init() {
+  auto set = [](auto kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
+           cudaSuccess;
+  };
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return -1;
+  auto all = [&](auto kernel) {  // what the kernel's own arrays leave of it
+    cudaFuncAttributes at;
+    return cudaFuncGetAttributes(&at, kernel) == cudaSuccess &&
+           set(kernel, (size_t)optin - at.sharedSizeBytes);
+  };
+  return set(k_lu_panel_cluster, sizeof(double) * kLuNb * kLuChunk) && all(k_dense_inverse) &&
+                 all(k_dense_solve) &&
+                 set(k_vanka_apply_staged<float, NU_LOC>,
+                     sizeof(float) * Elem<NU_LOC>::fac_stride) &&
+                 set(k_vanka_apply_staged<float, NU_TET>,
+                     sizeof(float) * Elem<NU_TET>::fac_stride) &&
+                 set(k_vanka_apply_staged<double, NU_LOC>,
+                     sizeof(double) * Elem<NU_LOC>::fac_stride) &&
+                 set(k_vanka_apply_staged<double, NU_TET>,
+                     sizeof(double) * Elem<NU_TET>::fac_stride)
+             ? 0
+             : -1;
+}
+
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf, T damp,
@@ -2221,9 +2249,6 @@ int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int 
       const size_t sm = (size_t)stride * sizeof(T);
       const int per_sm = std::min(24, (int)(220 * 1024 / (sm + 2048)));
       if (ncol > per_sm * num_sms) return 0;
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-          cudaSuccess)
-        return -1;
       return launch_chained<DevCells, int, const int *, const T *, const uint8_t *, const T *, T,
                             T *, int *>(kernel, dim3((unsigned)ncol), 32, sm, s, cells, nu,
                                         cell_list, factors, perm, rbuf, damp, u, err);
@@ -2284,9 +2309,6 @@ int launch_dense_lu(double *a, int n, int *ipiv, int *status, cudaStream_t s) {
     const int chunk = (n - k0 + kLuCluster - 1) / kLuCluster;
     if (chunk <= kLuChunk) {
       const size_t sm = sizeof(double) * kLuNb * (size_t)chunk;
-      if (cudaFuncSetAttribute(k_lu_panel_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sm) != cudaSuccess)
-        return -1;
       k_lu_panel_cluster<<<kLuCluster, kLuPanelThreads, sm, s>>>(a, n, k0, ipiv, status);
     } else {
       k_lu_panel<<<1, kDenseThreads, 0, s>>>(a, n, k0, ipiv, status);
@@ -2317,8 +2339,6 @@ int launch_dense_inverse(const double *lu, const int *ipiv, int n, double *inv, 
     return ok() < 0 ? -1 : 1;
   }
   const size_t sm = sizeof(double) * n;
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_dense_inverse<<<n, kInvThreads, sm, s>>>(lu, ipiv, n, inv);
   return ok() < 0 ? -1 : 1;
 }
@@ -2337,8 +2357,6 @@ template int launch_dense_gemv<float, float>(const double *, int, const float *,
 int launch_dense_solve(const double *lu, const int *ipiv, int n, const double *b, double *x,
                        int pin_row, cudaStream_t s) {
   const size_t sm = sizeof(double) * n;
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_dense_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_dense_solve<<<1, kDenseSolveThreads, sm, s>>>(lu, ipiv, n, b, x, pin_row);
   return ok() < 0 ? -1 : 1;
 }
