@@ -94,6 +94,9 @@ struct LevelDev {
   // looked at yet, 1 in use, -1 not available (mesh shape, memory)
   int pk = 0;
   bool pk_stale = true;  // matrix values newer than the packed copy
+  // B is not the one of the last factorisation: the packed sweeps read the
+  // pressure rows from the stored factors, so the CSR kernels run meanwhile
+  bool pk_other_b = false;
   int *pk_ids = nullptr;
   uint8_t *pk_flips = nullptr;
   void *pk_patterns = nullptr, *pk_values = nullptr, *pk_u = nullptr, *pk_p = nullptr;
@@ -136,7 +139,7 @@ struct LevelDev {
   // the Schur block solve of one-block levels exists for Q2 hexahedra only
   bool schur() const { return one_block() && nl == NU_LOC; }
   // sweeps run from the packed rows
-  bool packed() const { return pk == 1 && schur(); }
+  bool packed() const { return pk == 1 && schur() && !pk_other_b; }
   // block elimination with three diagonal blocks (decoupled nine-block levels)
   bool schur3() const { return diag == 1 && nl == NU_LOC; }
   size_t fac_bytes = 0;  // allocated factor storage
@@ -807,17 +810,43 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
   return PM_OK;
 }
 
+// Values newer than the packed rows: whether B still is the one whose values
+// lie in the stored factors (none of them are newer when `factoring` follows).
+template <typename T>
+pm_status check_factored_b(pm_handle *h, LevelDev &Lv, bool factoring) {
+  int differ = 0;
+  if (!factoring) {
+    int *flag = h->status_d + 2;
+    if (cudaMemsetAsync(flag, 0, sizeof(int), h->stream) != cudaSuccess)
+      return cuda_fail(h, "B check");
+    PM_LAUNCH(launch_patch_compare_b<T>(patch_level<T>(h, Lv), Lv.op<T>(), Lv.ncells,
+                                        static_cast<const T *>(Lv.factors), flag, h->stream));
+    if (cudaMemcpyAsync(&differ, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream) !=
+        cudaSuccess)
+      return cuda_fail(h, "B check");
+    PM_TRY(sync(h, "B check"));
+  }
+  if (Lv.pk_other_b != (differ != 0)) {
+    Lv.pk_other_b = differ != 0;
+    drop_graphs(h);  // the kernels of the sweeps change
+  }
+  return PM_OK;
+}
+
 // Packed rows of every level that can run from them: built once per level,
 // packed again when the matrix values are newer.  A level whose mesh does not
 // have the shape, or for which there is no memory, keeps the CSR kernels.
+// factoring: the factors are about to be made from the present values.
 template <typename T>
-pm_status ensure_patches(pm_handle *h) {
+pm_status ensure_patches(pm_handle *h, bool factoring) {
   if (h->opt.residual_variant != 0) return PM_OK;  // a CSR kernel is asked for
   for (size_t l = 1; l < h->L.size(); ++l) {
     LevelDev &Lv = h->L[l];
-    if (Lv.pk < 0 || !Lv.schur() || Lv.ncells == 0 || (Lv.pk == 1 && !Lv.pk_stale)) continue;
+    if (Lv.pk < 0 || !Lv.schur() || Lv.ncells == 0) continue;
     if (Lv.pk == 1) {
-      PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), Lv.op<T>(), Lv.ncells, h->stream));
+      if (Lv.pk_stale)
+        PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), Lv.op<T>(), Lv.ncells, h->stream));
+      if (Lv.pk_stale || factoring) PM_TRY(check_factored_b<T>(h, Lv, factoring));
       Lv.pk_stale = false;
       continue;
     }
@@ -833,6 +862,7 @@ pm_status ensure_patches(pm_handle *h) {
       h->err = err;
       continue;
     }
+    PM_TRY(check_factored_b<T>(h, Lv, factoring));
     Lv.pk = 1;
     Lv.pk_stale = false;
     drop_graphs(h);
@@ -840,8 +870,8 @@ pm_status ensure_patches(pm_handle *h) {
   return PM_OK;
 }
 
-pm_status ensure_patches(pm_handle *h) {
-  return mixed(h) ? ensure_patches<float>(h) : ensure_patches<double>(h);
+pm_status ensure_patches(pm_handle *h, bool factoring = false) {
+  return mixed(h) ? ensure_patches<float>(h, factoring) : ensure_patches<double>(h, factoring);
 }
 
 // One V-cycle; with a network attached and enabled the cycle includes the
@@ -1519,7 +1549,7 @@ pm_status factor_all(pm_handle *h) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, h->stream);
-  PM_TRY(ensure_patches(h));
+  PM_TRY(ensure_patches(h, true));
   for (size_t l = 1; l < h->L.size(); ++l) {
     LevelDev &Lv = h->L[l];
     // block elimination in FP32 unless factor_fp32 = 0 (mixed only); the
@@ -2067,7 +2097,6 @@ pm_status pm_setup(pm_handle *h) {
   PM_TRY(dalloc(h, &h->w, N));
   PM_TRY(dalloc(h, &h->xd, N));
   PM_TRY(dalloc(h, &h->bd, N));
-  PM_TRY(ensure_patches(h));
   PM_TRY(factor_all(h));
   for (size_t l = 1; l < h->L.size(); ++l) {
     if (mixed(h))

@@ -249,6 +249,10 @@ int launch_patch_lists(const DevCells &cells, int nu, int np, const int *colour,
 // the level's CSR values into the packed layout
 template <typename T>
 int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cudaStream_t s);
+// *differ |= 1 when a value of B differs from the D block of its cell's factors
+template <typename T>
+int launch_patch_compare_b(const PatchLevel<T> &L, const DevOp<T> &op, int ncells,
+                           const T *factors, int *differ, cudaStream_t s);
 // patterns of a level's cells: mode 0 hashes (n = ncells), 1 the patterns of
 // the cells which[0..n), 2 compare each cell (n = ncells) with its pattern;
 // *bad |= 1 when a row does not fit or a pattern differs

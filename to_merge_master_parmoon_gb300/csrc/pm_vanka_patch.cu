@@ -996,6 +996,24 @@ __global__ void __launch_bounds__(256) k_patch_pack(PatchLevel<T> L, DevOp<T> op
     reinterpret_cast<float4 *>(V)[i] = reinterpret_cast<const float4 *>(stage)[i];
 }
 
+// B against the D blocks of the stored factors: one warp per pressure row
+template <typename T>
+__global__ void __launch_bounds__(32 * NP_LOC) k_patch_compare_b(PatchLevel<T> L, DevOp<T> op,
+                                                                const T *__restrict__ factors,
+                                                                int *differ) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31, cell = blockIdx.x;
+  const int *ids = L.ids + (size_t)cell * kPatchIds;
+  const PatchPattern &pat = L.patterns[ids[kPatchPattern]];
+  const T *D = factors + (size_t)cell * Schur<1>::stride + Schur<1>::offD + k * 3 * NU_LOC;
+  const int rs = op.b_rowptr[ids[kPatchBase] + k], n = op.b_rowptr[ids[kPatchBase] + k + 1] - rs;
+  bool other = false;
+  if (lane < n) {
+    const int at = pat.bj[8 * k + (lane & 7)][lane >> 3];
+    for (int c = 0; c < 3; ++c) other |= !(op.b[c][rs + lane] == D[c * NU_LOC + at]);
+  }
+  if (other) atomicOr(differ, 1);
+}
+
 // Cells of every velocity node (slots: the first eight, cnt: all) and the
 // owner count of every pressure block; *bad when a node lies in more than
 // eight cells or a cell's pressure DOFs are not one aligned block of its own.
@@ -1300,6 +1318,14 @@ int launch_patch_pack(const PatchLevel<T> &L, const DevOp<T> &op, int ncells, cu
 }
 
 template <typename T>
+int launch_patch_compare_b(const PatchLevel<T> &L, const DevOp<T> &op, int ncells,
+                           const T *factors, int *differ, cudaStream_t s) {
+  if (ncells <= 0) return 0;
+  k_patch_compare_b<T><<<ncells, 32 * NP_LOC, 0, s>>>(L, op, factors, differ);
+  return ok();
+}
+
+template <typename T>
 int launch_patch_pattern(int mode, const int *ids, const DevOp<T> &op, int n, const int *which,
                          void *patterns, unsigned long long *hash, int *bad, cudaStream_t s) {
   if (n <= 0) return 0;
@@ -1481,6 +1507,8 @@ int launch_patch_end(const PatchLevel<T> &L, T *u, const T *rhs, int hb, int np,
 
 #define PM_PINST(T)                                                                               \
   template int launch_patch_pack<T>(const PatchLevel<T> &, const DevOp<T> &, int, cudaStream_t);  \
+  template int launch_patch_compare_b<T>(const PatchLevel<T> &, const DevOp<T> &, int, const T *, \
+                                         int *, cudaStream_t);                                    \
   template int launch_patch_pattern<T>(int, const int *, const DevOp<T> &, int, const int *,      \
                                        void *, unsigned long long *, int *, cudaStream_t);        \
   template int launch_patch_begin<T>(const PatchLevel<T> &, const T *, const T *, int, int,       \
