@@ -146,11 +146,13 @@ typedef struct {
                              0: the 85x85 LU and all nine blocks on every
                              nine-block level, as the reference's CellVanka
                              (src/FE/NSE_MGLevel4.C:1784-2031)              */
-  int wait_limit;         /* polls of the first bounded mbarrier wait of the
-                             bulk-copy apply before it gives up (0: the
-                             default 2^22; the wait that drains the copies
-                             in flight keeps the default); a wait that gives
-                             up makes the solve return PM_TIMEOUT           */
+  int wait_limit;         /* polls of a bounded mbarrier wait of the sweep
+                             kernels that are fed by bulk copies (packed
+                             sweeps, LU applies from shared memory) before
+                             it gives up (0: the default 2^22; the waits that
+                             drain the copies in flight keep the default); a
+                             wait that gives up makes the call return
+                             PM_TIMEOUT                                     */
   long long max_device_bytes; /* cap on the device memory the handle
                              allocates (0: none); an allocation beyond it
                              fails with PM_OOM, as a failed cudaMalloc does  */

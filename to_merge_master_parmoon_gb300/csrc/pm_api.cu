@@ -448,7 +448,8 @@ pm_status patch_sweeps(pm_handle *h, LevelDev &Lv, T *u, const T *rhs, int sweep
       if (prof) cudaEventRecord(h->evpool[h->evused], h->stream);
       PM_LAUNCH(launch_patch_colour<T>(L, Lv.colour_cells + b, n,
                                        static_cast<const T *>(Lv.factors), (T)h->opt.smooth_damp,
-                                       s & 1, h->sweep_err, h->num_sms, h->stream));
+                                       s & 1, h->sweep_err, h->num_sms, h->opt.wait_limit,
+                                       h->stream));
       if (prof) {  // residual and local solve are one launch: all of it is kernel 0
         cudaEventRecord(h->evpool[h->evused + 1], h->stream);
         cudaEventRecord(h->evpool[h->evused + 2], h->stream);
@@ -533,7 +534,8 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
       PM_LAUNCH(launch_vanka_apply<T>(cells, Lv.nu, Lv.colour_cells + b, n,
                                       static_cast<const T *>(Lv.factors), Lv.perm, use_inverse(h),
                                       static_cast<const T *>(Lv.dbuf), damp, u,
-                                      Lv.apply_variant == 0, h->sweep_err, h->num_sms, h->stream));
+                                      Lv.apply_variant == 0, h->sweep_err, h->num_sms,
+                                      h->opt.wait_limit, h->stream));
     if (e2) {
       cudaEventRecord(e2, h->stream);
       // algorithmic bytes of this colour: the level's unique Vanka-sweep
@@ -1508,7 +1510,8 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
       } else {
         st = time_it([&] {
           return launch_vanka_apply<T>(Lv.cells(), Lv.nu, list, nb, F, Lv.perm, false, rb, T(1), u,
-                                       v == 0, h->sweep_err, h->num_sms, h->stream);
+                                       v == 0, h->sweep_err, h->num_sms, h->opt.wait_limit,
+                                       h->stream);
         }, t[v]);
       }
     }

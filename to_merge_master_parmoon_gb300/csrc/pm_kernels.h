@@ -174,11 +174,13 @@ int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, con
 int launch_vanka_init();
 // Local solve with the stored factors and u[dofs] += damp * delta, for the
 // same cells (run after launch_vanka_residual of the whole colour).  pairs:
-// two cells per warp (half-warp per cell) instead of one.
+// two cells per warp (half-warp per cell) instead of one.  wait_limit: polls
+// of a wait for a bulk copy before the kernel gives up (0: default).
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf,
-                       T damp, T *u, bool pairs, int *err, int num_sms, cudaStream_t s);
+                       T damp, T *u, bool pairs, int *err, int num_sms, long long wait_limit,
+                       cudaStream_t s);
 
 // Error bits of bounded device waits (sweep kernels, `err` arguments)
 constexpr int PM_ERR_BULK_TIMEOUT = 1;
@@ -265,14 +267,15 @@ int launch_patch_init();  // shared-memory limit of the sweep kernels
 // a run of sweeps: begin (u into the copies), every colour of every sweep,
 // between two sweeps the Dirichlet nodes, end (the copies into u).  begin
 // without u starts from zero, end without rhs leaves zero on the Dirichlet
-// nodes.  odd: the
-// sweep's number & 1; for end the number of sweeps & 1.
+// nodes.  odd: the sweep's number & 1; for end the number of sweeps & 1.
+// wait_limit: as for launch_vanka_apply.
 template <typename T>
 int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb, int np,
                        cudaStream_t s);
 template <typename T>
 int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors,
-                        T damp, int odd, int *err, int num_sms, cudaStream_t s);
+                        T damp, int odd, int *err, int num_sms, long long wait_limit,
+                        cudaStream_t s);
 template <typename T>
 int launch_patch_between(const PatchLevel<T> &L, const T *rhs, int hb, cudaStream_t s);
 template <typename T>

@@ -1306,7 +1306,7 @@ template <typename T, int NU>
 __global__ void __launch_bounds__(32) k_vanka_apply_staged(
     DevCells cells, int nu, const int *__restrict__ list, const T *__restrict__ F,
     const uint8_t *__restrict__ perm, const T *__restrict__ rbuf, T damp, T *__restrict__ u,
-    int *err) {
+    int *err, long long limit) {
   constexpr int NU_LOC = NU, NLOC = Elem<NU>::nloc, kFacStride = Elem<NU>::fac_stride,
                 kRStride = Elem<NU>::r_stride, SL = (NLOC + 31) / 32;
   static_assert(NLOC % 4 == 1, "blocks of four columns and one");
@@ -1334,7 +1334,7 @@ __global__ void __launch_bounds__(32) k_vanka_apply_staged(
                  : (i < NLOC ? 3 * nu + __ldg(cells.pdofs + (size_t)cell * NP_LOC + i - 3 * NU_LOC)
                              : 0);
   }
-  const bool there = mbar_wait(&bar, 0, kMaxPolls);
+  const bool there = mbar_wait(&bar, 0, limit);
   if (!there) {
     if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
     mbar_wait(&bar, 0, kMaxPolls);  // the copy still in flight (bounded)
@@ -2241,8 +2241,10 @@ int launch_vanka_init() {
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf, T damp,
-                       T *u, bool pairs, int *err, int num_sms, cudaStream_t s) {
+                       T *u, bool pairs, int *err, int num_sms, long long wait_limit,
+                       cudaStream_t s) {
   if (ncol <= 0) return 0;
+  const long long limit = wait_limit > 0 ? wait_limit : kMaxPolls;
   if (!inverse && (cells.nl == NU_TET || cells.nl == NU_LOC)) {
     // one wave of CTAs that hold a cell's factors each
     auto staged = [&](auto kernel, int stride) {
@@ -2250,8 +2252,9 @@ int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int 
       const int per_sm = std::min(24, (int)(220 * 1024 / (sm + 2048)));
       if (ncol > per_sm * num_sms) return 0;
       return launch_chained<DevCells, int, const int *, const T *, const uint8_t *, const T *, T,
-                            T *, int *>(kernel, dim3((unsigned)ncol), 32, sm, s, cells, nu,
-                                        cell_list, factors, perm, rbuf, damp, u, err);
+                            T *, int *, long long>(kernel, dim3((unsigned)ncol), 32, sm, s, cells,
+                                                   nu, cell_list, factors, perm, rbuf, damp, u,
+                                                   err, limit);
     };
     const int n = cells.nl == NU_TET
                       ? staged(k_vanka_apply_staged<T, NU_TET>, Elem<NU_TET>::fac_stride)
@@ -2370,7 +2373,7 @@ template int launch_vanka_factor<float>(const DevOp<double> &, const DevCells &,
                                         const T *, const T *, T *, int, int, cudaStream_t);        \
   template int launch_vanka_apply<T>(const DevCells &, int, const int *, int, const T *,           \
                                      const uint8_t *, bool, const T *, T, T *, bool, int *, int,   \
-                                     cudaStream_t);
+                                     long long, cudaStream_t);
 PM_VINST(double)
 PM_VINST(float)
 #undef PM_VINST
