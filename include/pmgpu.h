@@ -121,7 +121,12 @@ typedef struct {
                              cell per warp; -1 time them per level at
                              pm_setup.  pm_level_variant reports residual
                              kernel (0 rows, 1 stream) + 2 * apply kernel
-                             (0 pairs, 1 bulk, 2 single)                     */
+                             (0 pairs, 1 bulk, 2 single).  0 and -1 run
+                             colours too small to fill the GPU with one CTA
+                             per cell, the same sums in the same order
+                             (residual) and the factors in shared memory
+                             (apply); a named variant (1, 2) runs the named
+                             kernel on every colour                          */
   int upload_mode;        /* how pm_add_level / pm_update_matrices move matrix
                              values: 0 (default) copy-engine copies
                              (cudaMemcpyAsync) then device conversions; 1 the

@@ -507,8 +507,8 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
                                           static_cast<float *>(Lv.dbuf), h->stream));
     else
       PM_LAUNCH(launch_vanka_residual<T>(op, cells, Lv.colour_cells + b, n, u, rhs,
-                                         static_cast<T *>(Lv.dbuf), Lv.res_variant, Lv.max_row,
-                                         h->stream));
+                                         static_cast<T *>(Lv.dbuf), Lv.res_variant,
+                                         h->opt.residual_variant > 0, Lv.max_row, h->stream));
     if (e1) cudaEventRecord(e1, h->stream);
     if (aos)
       PM_LAUNCH(launch_schur_apply_aos(cells, Lv.nu, Lv.colour_cells + b, n,
@@ -534,8 +534,8 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
       PM_LAUNCH(launch_vanka_apply<T>(cells, Lv.nu, Lv.colour_cells + b, n,
                                       static_cast<const T *>(Lv.factors), Lv.perm, use_inverse(h),
                                       static_cast<const T *>(Lv.dbuf), damp, u,
-                                      Lv.apply_variant == 0, h->sweep_err, h->num_sms,
-                                      h->opt.wait_limit, h->stream));
+                                      Lv.apply_variant == 0, h->opt.apply_variant > 0,
+                                      h->sweep_err, h->num_sms, h->opt.wait_limit, h->stream));
     if (e2) {
       cudaEventRecord(e2, h->stream);
       // algorithmic bytes of this colour: the level's unique Vanka-sweep
@@ -1488,7 +1488,7 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
     for (int v = 0; v < 2 && st == PM_OK; ++v)
       st = time_it([&] {
         return launch_vanka_residual<T>(op, Lv.cells(), list, nb, u,
-                                        static_cast<const T *>(Lv.rhs), rb, v, Lv.max_row,
+                                        static_cast<const T *>(Lv.rhs), rb, v, false, Lv.max_row,
                                         h->stream);
       }, t[v]);
     Lv.res_variant = t[1] < t[0] ? 1 : 0;  // kernel index: 0 row groups, 1 stream
@@ -1510,8 +1510,8 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
       } else {
         st = time_it([&] {
           return launch_vanka_apply<T>(Lv.cells(), Lv.nu, list, nb, F, Lv.perm, false, rb, T(1), u,
-                                       v == 0, h->sweep_err, h->num_sms, h->opt.wait_limit,
-                                       h->stream);
+                                       v == 0, false, h->sweep_err, h->num_sms,
+                                       h->opt.wait_limit, h->stream);
         }, t[v]);
       }
     }

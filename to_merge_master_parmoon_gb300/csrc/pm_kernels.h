@@ -157,10 +157,11 @@ int launch_vanka_factor(const DevOp<double> &op, const DevCells &cells, TF *fact
 // For the ncol cells listed in cell_list: local residual r = f - K u over the
 // full rows of the cell's 85 DOFs -> rbuf[slot*kRStride + i].
 // variant 0: row groups (8 lanes per row); 1: flattened row stream with
-// segmented sums.  Same result up to summation order.
+// segmented sums.  Same result up to summation order.  Small colours run one
+// CTA per cell with the same sums, unless the caller named the kernel.
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, int max_row,
+                          const T *u, const T *rhs, T *rbuf, int variant, bool named, int max_row,
                           cudaStream_t s);
 // The same (row groups) on an FP32 one-block hexahedral level with the
 // velocity read from its interleaved copy ux (node d: ux[d].x/y/z) and the
@@ -174,13 +175,14 @@ int launch_vanka_residual_aos(const DevOp<float> &op, const DevCells &cells, con
 int launch_vanka_init();
 // Local solve with the stored factors and u[dofs] += damp * delta, for the
 // same cells (run after launch_vanka_residual of the whole colour).  pairs:
-// two cells per warp (half-warp per cell) instead of one.  wait_limit: polls
+// two cells per warp (half-warp per cell) instead of one; small colours run
+// from shared memory, unless the caller named the kernel.  wait_limit: polls
 // of a wait for a bulk copy before the kernel gives up (0: default).
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf,
-                       T damp, T *u, bool pairs, int *err, int num_sms, long long wait_limit,
-                       cudaStream_t s);
+                       T damp, T *u, bool pairs, bool named, int *err, int num_sms,
+                       long long wait_limit, cudaStream_t s);
 
 // Error bits of bounded device waits (sweep kernels, `err` arguments)
 constexpr int PM_ERR_BULK_TIMEOUT = 1;

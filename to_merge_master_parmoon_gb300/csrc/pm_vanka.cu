@@ -2119,14 +2119,14 @@ constexpr int kWideCells = 152;
 
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, int max_row,
+                          const T *u, const T *rhs, T *rbuf, int variant, bool named, int max_row,
                           cudaStream_t s) {
   if (ncol <= 0) return 0;
   constexpr int VEC = sizeof(T) == 4 ? 4 : 2;
   constexpr int U = sizeof(T) == 4 ? 1 : 2;
   const int grid = (ncol + kResWarps - 1) / kResWarps;
   // one CTA per cell where the colour would leave the GPU idle
-  if (ncol <= kSplitCells) {
+  if (!named && ncol <= kSplitCells) {
     auto split = [&](auto kernel, int steps) {
       return launch_chained<DevOp<T>, DevCells, const int *, const T *, const T *, T *>(
           kernel, dim3((unsigned)ncol), (steps + 1) * 32, 0, s, op, cells, cell_list, u, rhs, rbuf);
@@ -2241,11 +2241,11 @@ int launch_vanka_init() {
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf, T damp,
-                       T *u, bool pairs, int *err, int num_sms, long long wait_limit,
+                       T *u, bool pairs, bool named, int *err, int num_sms, long long wait_limit,
                        cudaStream_t s) {
   if (ncol <= 0) return 0;
   const long long limit = wait_limit > 0 ? wait_limit : kMaxPolls;
-  if (!inverse && (cells.nl == NU_TET || cells.nl == NU_LOC)) {
+  if (!inverse && !named && (cells.nl == NU_TET || cells.nl == NU_LOC)) {
     // one wave of CTAs that hold a cell's factors each
     auto staged = [&](auto kernel, int stride) {
       const size_t sm = (size_t)stride * sizeof(T);
@@ -2370,10 +2370,10 @@ template int launch_vanka_factor<float>(const DevOp<double> &, const DevCells &,
                                         uint8_t *, bool, bool, int *, cudaStream_t);
 #define PM_VINST(T)                                                                                 \
   template int launch_vanka_residual<T>(const DevOp<T> &, const DevCells &, const int *, int,      \
-                                        const T *, const T *, T *, int, int, cudaStream_t);        \
+                                        const T *, const T *, T *, int, bool, int, cudaStream_t);  \
   template int launch_vanka_apply<T>(const DevCells &, int, const int *, int, const T *,           \
-                                     const uint8_t *, bool, const T *, T, T *, bool, int *, int,   \
-                                     long long, cudaStream_t);
+                                     const uint8_t *, bool, const T *, T, T *, bool, bool, int *,  \
+                                     int, long long, cudaStream_t);
 PM_VINST(double)
 PM_VINST(float)
 #undef PM_VINST
