@@ -490,6 +490,9 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
   const bool aos = sizeof(T) == sizeof(float) && Lv.ux && Lv.schur() && Lv.res_variant == 0;
   float *uf = reinterpret_cast<float *>(u);
   if (aos) PM_LAUNCH(launch_pack_velocity(uf, Lv.ux, Lv.nu, h->stream));
+  // without Dirichlet nodes the kernel before the first colour may be the one
+  // that wrote rhs, which the residual reads before it waits
+  bool started = false;
   for (int k = 0; k < ncol; ++k) {
     const int b = Lv.colouring.ptr[k], n = Lv.colouring.ptr[k + 1] - b;
     if (n == 0) continue;
@@ -508,7 +511,9 @@ pm_status vanka_sweep(pm_handle *h, LevelDev &Lv, T *u, const T *rhs) {
     else
       PM_LAUNCH(launch_vanka_residual<T>(op, cells, Lv.colour_cells + b, n, u, rhs,
                                          static_cast<T *>(Lv.dbuf), Lv.res_variant,
-                                         h->opt.residual_variant > 0, Lv.max_row, h->stream));
+                                         h->opt.residual_variant > 0, started || Lv.ndir > 0,
+                                         Lv.max_row, h->stream));
+    started = true;
     if (e1) cudaEventRecord(e1, h->stream);
     if (aos)
       PM_LAUNCH(launch_schur_apply_aos(cells, Lv.nu, Lv.colour_cells + b, n,
@@ -1488,8 +1493,8 @@ pm_status tune_level(pm_handle *h, LevelDev &Lv) {
     for (int v = 0; v < 2 && st == PM_OK; ++v)
       st = time_it([&] {
         return launch_vanka_residual<T>(op, Lv.cells(), list, nb, u,
-                                        static_cast<const T *>(Lv.rhs), rb, v, false, Lv.max_row,
-                                        h->stream);
+                                        static_cast<const T *>(Lv.rhs), rb, v, false, true,
+                                        Lv.max_row, h->stream);
       }, t[v]);
     Lv.res_variant = t[1] < t[0] ? 1 : 0;  // kernel index: 0 row groups, 1 stream
   }

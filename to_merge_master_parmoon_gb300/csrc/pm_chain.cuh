@@ -18,10 +18,11 @@ __device__ __forceinline__ void start_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// every block of the kernel has to call wait_previous()
+// every block of the kernel has to call wait_previous(); overlap = false: an
+// ordinary launch of the same kernel, after its predecessor
 template <typename... Args>
-int launch_chained(void (*kernel)(Args...), dim3 grid, int block, size_t smem, cudaStream_t s,
-                   const Args &...args) {
+int launch_overlapped(bool overlap, void (*kernel)(Args...), dim3 grid, int block, size_t smem,
+                      cudaStream_t s, const Args &...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
@@ -31,8 +32,13 @@ int launch_chained(void (*kernel)(Args...), dim3 grid, int block, size_t smem, c
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? 1 : -1;
+}
+template <typename... Args>
+int launch_chained(void (*kernel)(Args...), dim3 grid, int block, size_t smem, cudaStream_t s,
+                   const Args &...args) {
+  return launch_overlapped(true, kernel, grid, block, smem, s, args...);
 }
 
 }  // namespace pm

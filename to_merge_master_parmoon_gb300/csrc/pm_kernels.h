@@ -158,11 +158,13 @@ int launch_vanka_factor(const DevOp<double> &op, const DevCells &cells, TF *fact
 // full rows of the cell's 85 DOFs -> rbuf[slot*kRStride + i].
 // variant 0: row groups (8 lanes per row); 1: flattened row stream with
 // segmented sums.  Same result up to summation order.  Small colours run one
-// CTA per cell with the same sums, unless the caller named the kernel.
+// CTA per cell with the same sums, unless the caller named the kernel; their
+// launch may overlap the kernel before it (overlap), which must not write the
+// matrix or rhs.
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, bool named, int max_row,
-                          cudaStream_t s);
+                          const T *u, const T *rhs, T *rbuf, int variant, bool named, bool overlap,
+                          int max_row, cudaStream_t s);
 // The same (row groups) on an FP32 one-block hexahedral level with the
 // velocity read from its interleaved copy ux (node d: ux[d].x/y/z) and the
 // pressure from u; -1 for any other level.

@@ -799,7 +799,9 @@ __global__ void __launch_bounds__(kResWarps * 32) k_vanka_residual_rows(
 // (the last warp: the pressure rows), for colours that do not fill the GPU:
 // with one warp per cell the row steps' loads follow one another (31 us per
 // launch of any size on tetrahedra).  Each row is summed as by
-// k_vanka_residual_rows.  Matrix data are loaded before the launch waits.
+// k_vanka_residual_rows.  Matrix data and the right-hand side are loaded
+// before the launch waits (the latter after the wait cost 1.5 % of a solve):
+// the kernel before it must not be the one that writes them.
 template <typename T, int VEC, int KIND, int URA, int NU>
 __global__ void __launch_bounds__(((NU + 3) / 4 + 1) * 32) k_vanka_residual_split(
     DevOp<T> op, DevCells cells, const int *__restrict__ list, const T *__restrict__ u,
@@ -2119,8 +2121,8 @@ constexpr int kWideCells = 152;
 
 template <typename T>
 int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *cell_list, int ncol,
-                          const T *u, const T *rhs, T *rbuf, int variant, bool named, int max_row,
-                          cudaStream_t s) {
+                          const T *u, const T *rhs, T *rbuf, int variant, bool named, bool overlap,
+                          int max_row, cudaStream_t s) {
   if (ncol <= 0) return 0;
   constexpr int VEC = sizeof(T) == 4 ? 4 : 2;
   constexpr int U = sizeof(T) == 4 ? 1 : 2;
@@ -2128,8 +2130,9 @@ int launch_vanka_residual(const DevOp<T> &op, const DevCells &cells, const int *
   // one CTA per cell where the colour would leave the GPU idle
   if (!named && ncol <= kSplitCells) {
     auto split = [&](auto kernel, int steps) {
-      return launch_chained<DevOp<T>, DevCells, const int *, const T *, const T *, T *>(
-          kernel, dim3((unsigned)ncol), (steps + 1) * 32, 0, s, op, cells, cell_list, u, rhs, rbuf);
+      return launch_overlapped<DevOp<T>, DevCells, const int *, const T *, const T *, T *>(
+          overlap, kernel, dim3((unsigned)ncol), (steps + 1) * 32, 0, s, op, cells, cell_list, u,
+          rhs, rbuf);
     };
     if (cells.nl == NU_TET) {
       if (op.structured) return split(k_vanka_residual_split<T, VEC, 1, 2, NU_TET>, 4);
@@ -2370,7 +2373,8 @@ template int launch_vanka_factor<float>(const DevOp<double> &, const DevCells &,
                                         uint8_t *, bool, bool, int *, cudaStream_t);
 #define PM_VINST(T)                                                                                 \
   template int launch_vanka_residual<T>(const DevOp<T> &, const DevCells &, const int *, int,      \
-                                        const T *, const T *, T *, int, bool, int, cudaStream_t);  \
+                                        const T *, const T *, T *, int, bool, bool, int,           \
+                                        cudaStream_t);                                             \
   template int launch_vanka_apply<T>(const DevCells &, int, const int *, int, const T *,           \
                                      const uint8_t *, bool, const T *, T, T *, bool, bool, int *,  \
                                      int, long long, cudaStream_t);
