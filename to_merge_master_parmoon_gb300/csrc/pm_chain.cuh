@@ -2,6 +2,11 @@
 // dependent launch): the kernel may start while the previous kernel of the
 // stream still runs and waits for it on the device before it reads its
 // results.
+//
+// A kernel launched this way may be resident while its predecessor writes the
+// vectors that it reads after the wait.  Such vectors are no read-only data of
+// the launch: they are read by ordinary loads (no __ldg, no const __restrict__
+// pointer, which become non-coherent loads) or from L2 (__ldcg).
 #ifndef PM_CHAIN_CUH
 #define PM_CHAIN_CUH
 

@@ -85,8 +85,7 @@ struct VLd<double, 2> {
 // multiplies value k with x_k into s[k]
 template <typename T, int VEC, int NV, int UR, bool DIAG = false>
 __device__ __forceinline__ void rows8_sum(const int *__restrict__ col, const T *const *vals, int rs,
-                                          int re, int sl, const T *__restrict__ x0,
-                                          const T *__restrict__ x1, const T *__restrict__ x2,
+                                          int re, int sl, const T *x0, const T *x1, const T *x2,
                                           T (&s)[3]) {
   for (int g = rs / VEC + sl; g * VEC < re; g += 8 * UR) {
     int ci[UR][VEC];
@@ -116,21 +115,21 @@ __device__ __forceinline__ void rows8_sum(const int *__restrict__ col, const T *
         if (e >= rs && e < re) {
           const int c = ci[q][m];
           if constexpr (DIAG) {
-            s[0] += v[q][0][m] * __ldg(x0 + c);
-            s[1] += v[q][1][m] * __ldg(x1 + c);
-            s[2] += v[q][2][m] * __ldg(x2 + c);
+            s[0] += v[q][0][m] * x0[c];
+            s[1] += v[q][1][m] * x1[c];
+            s[2] += v[q][2][m] * x2[c];
           } else if constexpr (NV == 3) {
-            const T pc = __ldg(x0 + c);
+            const T pc = x0[c];
             s[0] += v[q][0][m] * pc;
             s[1] += v[q][1][m] * pc;
             s[2] += v[q][2][m] * pc;
           } else if constexpr (NV == 1) {
             const T a = v[q][0][m];
-            s[0] += a * __ldg(x0 + c);
-            s[1] += a * __ldg(x1 + c);
-            s[2] += a * __ldg(x2 + c);
+            s[0] += a * x0[c];
+            s[1] += a * x1[c];
+            s[2] += a * x2[c];
           } else {
-            const T g0 = __ldg(x0 + c), g1 = __ldg(x1 + c), g2 = __ldg(x2 + c);
+            const T g0 = x0[c], g1 = x1[c], g2 = x2[c];
             s[0] += v[q][0][m] * g0 + v[q][1][m] * g1 + v[q][2][m] * g2;
             s[1] += v[q][3][m] * g0 + v[q][4][m] * g1 + v[q][5][m] * g2;
             s[2] += v[q][6][m] * g0 + v[q][7][m] * g1 + v[q][8][m] * g2;
@@ -174,27 +173,25 @@ constexpr int pressure_rows_per_group() {
 }
 template <typename T>
 __device__ __forceinline__ T pressure_part(const DevOp<T> &op, int i, int lane,
-                                           const T *__restrict__ u1, const T *__restrict__ u2,
-                                           const T *__restrict__ u3) {
+                                           const T *u1, const T *u2, const T *u3) {
   T s = 0;
   const int rs = op.b_rowptr[i], re = op.b_rowptr[i + 1];
   for (int j = rs + lane; j < re; j += 16) {
     const int c = __ldg(op.b_col + j);
     if constexpr (sizeof(T) == 4) {
-      s += ld_stream(op.b[0] + j) * __ldg(u1 + c) + ld_stream(op.b[1] + j) * __ldg(u2 + c) +
-           ld_stream(op.b[2] + j) * __ldg(u3 + c);
+      s += ld_stream(op.b[0] + j) * u1[c] + ld_stream(op.b[1] + j) * u2[c] +
+           ld_stream(op.b[2] + j) * u3[c];
     } else {
-      s = __dadd_rn(s, __fma_rn(ld_stream(op.b[2] + j), __ldg(u3 + c),
-                                __fma_rn(ld_stream(op.b[0] + j), __ldg(u1 + c),
-                                         __dmul_rn(ld_stream(op.b[1] + j), __ldg(u2 + c)))));
+      s = __dadd_rn(s, __fma_rn(ld_stream(op.b[2] + j), u3[c],
+                                __fma_rn(ld_stream(op.b[0] + j), u1[c],
+                                         __dmul_rn(ld_stream(op.b[1] + j), u2[c]))));
     }
   }
   return s;
 }
 template <typename T>
 __device__ __forceinline__ void pressure_rows(const DevOp<T> &op, long long group,
-                                              const T *__restrict__ x, const T *__restrict__ b,
-                                              T *__restrict__ r, int defect) {
+                                              const T *x, const T *b, T *r, int defect) {
   const int lane = threadIdx.x & 15, nu = op.nu;
   const T *u1 = x, *u2 = x + nu, *u3 = x + 2 * nu;
   long long row;
@@ -225,8 +222,7 @@ __device__ __forceinline__ void pressure_rows(const DevOp<T> &op, long long grou
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_pressure(DevOp<T> op, const T *__restrict__ x,
-                                                     const T *__restrict__ b, T *__restrict__ r,
+__global__ void __launch_bounds__(kBlock) k_pressure(DevOp<T> op, const T *x, const T *b, T *r,
                                                      int defect) {
   wait_previous();
   start_next();
@@ -243,8 +239,7 @@ __global__ void __launch_bounds__(kBlock) k_pressure(DevOp<T> op, const T *__res
 // KIND 0: nine A blocks; 1: one A block for the three components; 2: the
 // three diagonal blocks only (A12..A32 zero on the level)
 template <typename T, int VEC, int KIND, int UR>
-__global__ void __launch_bounds__(kBlock) k_coupled(DevOp<T> op, const T *__restrict__ x,
-                                                    const T *__restrict__ b, T *__restrict__ r,
+__global__ void __launch_bounds__(kBlock) k_coupled(DevOp<T> op, const T *x, const T *b, T *r,
                                                     int defect, int zero_nonactive, int vblocks) {
   // BT rows (at most 32 entries on hexahedra): one load round trip
   constexpr int URB = (16 / (int)sizeof(T)) / VEC > 1 ? (16 / (int)sizeof(T)) / VEC : 1;
@@ -280,9 +275,10 @@ __global__ void __launch_bounds__(kBlock) k_coupled(DevOp<T> op, const T *__rest
     if (skip) {
       r[i] = r[nu + i] = r[2 * nu + i] = T(0);
     } else if (defect) {
-      r[i] = b[i] - s[0];
-      r[nu + i] = b[nu + i] - s[1];
-      r[2 * nu + i] = b[2 * nu + i] - s[2];
+      const T f[3] = {b[i], b[nu + i], b[2 * nu + i]};
+      r[i] = f[0] - s[0];
+      r[nu + i] = f[1] - s[1];
+      r[2 * nu + i] = f[2] - s[2];
     } else {
       r[i] = s[0];
       r[nu + i] = s[1];
@@ -324,7 +320,7 @@ __global__ void __launch_bounds__(kBlock) k_csr_apply(DevCsr<T> m, const T *__re
 // entry) of x as k_l20_sub does.
 template <typename T, int G, int NC>
 __device__ __forceinline__ void csr_row(const DevCsr<T> &m, int i, bool valid,
-                                        const T *__restrict__ x, int x_stride, bool sub, T mean,
+                                        const T *x, int x_stride, bool sub, T mean,
                                         T (&s)[NC]) {
   const int lane = threadIdx.x & (G - 1);
 #pragma unroll
@@ -336,7 +332,7 @@ __device__ __forceinline__ void csr_row(const DevCsr<T> &m, int i, bool valid,
       const T v = __ldg(m.val + j);
 #pragma unroll
       for (int k = 0; k < NC; ++k) {
-        T xv = __ldg(x + (size_t)k * x_stride + c);
+        T xv = x[(size_t)k * x_stride + c];
         if (sub && (c & 3) == 0) xv -= mean;
         s[k] += v * xv;
       }
@@ -351,8 +347,8 @@ __device__ __forceinline__ void csr_row(const DevCsr<T> &m, int i, bool valid,
 // on the way (mean: device scalar or nullptr).
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_restrict(DevCsr<T> ru, DevCsr<T> rp,
-                                                     const T *__restrict__ d, T *__restrict__ cf,
-                                                     int nact, const double *mean, int vblocks) {
+                                                     const T *d, T *cf, int nact,
+                                                     const double *mean, int vblocks) {
   wait_previous();
   start_next();
   const bool lead = (threadIdx.x & 7) == 0;
@@ -380,7 +376,7 @@ __global__ void __launch_bounds__(kBlock) k_restrict(DevCsr<T> ru, DevCsr<T> rp,
 // active velocity rows and the pressure, u = 0 on the Dirichlet rows (from hb)
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_prolongate(DevCsr<T> pu, DevCsr<T> pp,
-                                                       const T *__restrict__ cu, T *__restrict__ u,
+                                                       const T *cu, T *u,
                                                        int hb, T beta, int vblocks) {
   wait_previous();
   start_next();
@@ -473,7 +469,7 @@ __global__ void __launch_bounds__(1024) k_l20_small(T *__restrict__ p, int np, d
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_l20_sum(const T *__restrict__ p, int np,
+__global__ void __launch_bounds__(kBlock) k_l20_sum(const T *p, int np,
                                                     double *partials, unsigned int *counter,
                                                     double *mean) {
   wait_previous();
