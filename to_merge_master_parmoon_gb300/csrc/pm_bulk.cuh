@@ -10,7 +10,7 @@
 namespace pm {
 
 // non-blocking polls of a wait before it gives up (a few hundred ms)
-constexpr long long kMaxPolls = 1ll << 22;
+constexpr int kMaxPolls = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -64,8 +64,8 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
 // when the phase completed.  The result is warp-uniform (every lane has
 // observed the completion itself, so every lane's later shared-memory reads
 // are ordered after the copy).
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long long polls) {
-  for (long long it = 0; it < polls; ++it)
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int polls) {
+  for (int it = 0; it < polls; ++it)
     if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
   return false;
 }

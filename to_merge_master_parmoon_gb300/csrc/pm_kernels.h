@@ -183,8 +183,8 @@ int launch_vanka_init();
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf,
-                       T damp, T *u, bool pairs, bool named, int *err, int num_sms,
-                       long long wait_limit, cudaStream_t s);
+                       T damp, T *u, bool pairs, bool named, int *err, int num_sms, int wait_limit,
+                       cudaStream_t s);
 
 // Error bits of bounded device waits (sweep kernels, `err` arguments)
 constexpr int PM_ERR_BULK_TIMEOUT = 1;
@@ -197,7 +197,7 @@ constexpr int PM_ERR_BULK_TIMEOUT = 1;
 int launch_vanka_apply_tma_init();
 int launch_vanka_apply_tma(const DevCells &cells, int nu, const int *cell_list, int ncol,
                            const float *factors, const uint8_t *perm, const float *rbuf, float damp,
-                           float *u, int *err, int num_sms, long long wait_limit, cudaStream_t s);
+                           float *u, int *err, int num_sms, int wait_limit, cudaStream_t s);
 
 // Block (Schur-complement) local solve of levels without velocity coupling,
 // NB = 1 (one-block operators: one A for the three components) or NB = 3
@@ -278,8 +278,7 @@ int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb,
                        cudaStream_t s);
 template <typename T>
 int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors,
-                        T damp, int odd, int *err, int num_sms, long long wait_limit,
-                        cudaStream_t s);
+                        T damp, int odd, int *err, int num_sms, int wait_limit, cudaStream_t s);
 template <typename T>
 int launch_patch_between(const PatchLevel<T> &L, const T *rhs, int hb, cudaStream_t s);
 template <typename T>

@@ -1308,7 +1308,7 @@ template <typename T, int NU>
 __global__ void __launch_bounds__(32) k_vanka_apply_staged(
     DevCells cells, int nu, const int *__restrict__ list, const T *__restrict__ F,
     const uint8_t *__restrict__ perm, const T *__restrict__ rbuf, T damp, T *__restrict__ u,
-    int *err, long long limit) {
+    int *err, int limit) {
   constexpr int NU_LOC = NU, NLOC = Elem<NU>::nloc, kFacStride = Elem<NU>::fac_stride,
                 kRStride = Elem<NU>::r_stride, SL = (NLOC + 31) / 32;
   static_assert(NLOC % 4 == 1, "blocks of four columns and one");
@@ -2244,10 +2244,10 @@ int launch_vanka_init() {
 template <typename T>
 int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int ncol,
                        const T *factors, const uint8_t *perm, bool inverse, const T *rbuf, T damp,
-                       T *u, bool pairs, bool named, int *err, int num_sms, long long wait_limit,
+                       T *u, bool pairs, bool named, int *err, int num_sms, int wait_limit,
                        cudaStream_t s) {
   if (ncol <= 0) return 0;
-  const long long limit = wait_limit > 0 ? wait_limit : kMaxPolls;
+  const int limit = wait_limit > 0 ? wait_limit : kMaxPolls;
   if (!inverse && !named && (cells.nl == NU_TET || cells.nl == NU_LOC)) {
     // one wave of CTAs that hold a cell's factors each
     auto staged = [&](auto kernel, int stride) {
@@ -2255,7 +2255,7 @@ int launch_vanka_apply(const DevCells &cells, int nu, const int *cell_list, int 
       const int per_sm = std::min(24, (int)(220 * 1024 / (sm + 2048)));
       if (ncol > per_sm * num_sms) return 0;
       return launch_chained<DevCells, int, const int *, const T *, const uint8_t *, const T *, T,
-                            T *, int *, long long>(kernel, dim3((unsigned)ncol), 32, sm, s, cells,
+                            T *, int *, int>(kernel, dim3((unsigned)ncol), 32, sm, s, cells,
                                                    nu, cell_list, factors, perm, rbuf, damp, u,
                                                    err, limit);
     };
@@ -2377,7 +2377,7 @@ template int launch_vanka_factor<float>(const DevOp<double> &, const DevCells &,
                                         cudaStream_t);                                             \
   template int launch_vanka_apply<T>(const DevCells &, int, const int *, int, const T *,           \
                                      const uint8_t *, bool, const T *, T, T *, bool, bool, int *,  \
-                                     int, long long, cudaStream_t);
+                                     int, int, cudaStream_t);
 PM_VINST(double)
 PM_VINST(float)
 #undef PM_VINST

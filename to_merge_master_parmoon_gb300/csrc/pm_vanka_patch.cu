@@ -365,20 +365,9 @@ __device__ __forceinline__ void async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// a wait that ran out: the launch has failed, the CTA is dead
-__device__ __forceinline__ void give_up(int *dead, int *err, int lane) {
-  if (lane == 0) {
-    *reinterpret_cast<volatile int *>(dead) = 1;
-    atomicOr(err, PM_ERR_BULK_TIMEOUT);
-  }
-}
-__device__ __forceinline__ bool is_dead(const int *dead) {
-  return *reinterpret_cast<const volatile int *>(dead) != 0;
-}
-
-// bounded wait for a copy that is to be left behind
+// bounded wait for a copy after a wait for it ran out
 __device__ __forceinline__ void drain(uint64_t *bar, int phase) {
-  for (long long it = 0; it < kMaxPolls; ++it)
+  for (int it = 0; it < kMaxPolls; ++it)
     if (mbar_test_wait(bar, phase & 1)) break;
 }
 
@@ -393,7 +382,6 @@ struct Smem32 {
   Tri<float, NU_LOC> r[2];              // velocity part of the local residual
   float rp[2][NP_LOC];
   uint64_t vbar[2], fbar[2], ibar[4];
-  int dead;                             // a wait of this CTA ran out
 };
 constexpr int kCtas32 = 3;  // resident CTAs per SM (67 KB of shared memory each)
 
@@ -405,10 +393,13 @@ constexpr int kCtas32 = 3;  // resident CTAs per SM (67 KB of shared memory each
 // copies into shared memory two cells ahead: one cell ahead (in registers or
 // in a second buffer) left their latency exposed.
 // Bound by HBM and by shared-memory wavefronts on large levels, by the chain
-// gather -> sums -> solve -> update on small ones.
+// gather -> sums -> solve -> update on small ones.  LIMITED: polls of a wait as
+// the caller says; with the number in a register instead of a constant a solve
+// at 8^3 took 3.42 instead of 3.38 ms.
+template <bool LIMITED>
 __global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
     PatchLevel<float> L, const int *__restrict__ list, int n, const float *__restrict__ factors,
-    float damp, int odd, int *err, long long limit) {
+    float damp, int odd, int *err, int limit) {
   using S1 = Schur<1>;
   extern __shared__ __align__(16) unsigned char raw[];
   Smem32 &sm = *reinterpret_cast<Smem32 *>(raw);
@@ -423,22 +414,19 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
     }
     for (int b = 0; b < 4; ++b) mbar_init(&sm.ibar[b], 1);
     fence_mbar_init();
-    sm.dead = 0;
     for (int b = 0; b < 3; ++b) {
       sm.u[b].set(kZeroSlot, 0.f, 0.f, 0.f);
       sm.p[b][27] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   __syncthreads();
-  // A wait that runs out marks the launch as failed and the CTA as dead: its
-  // warps go on through the barriers, without touching global memory through a
-  // patch list that did not arrive, and no stage is filled again, since its
-  // last copy may still be in flight.
-  long long polls = limit;
+  // a wait that runs out marks the launch as failed; the warp goes on without
+  // touching global memory through a patch list that did not arrive
+  int polls = LIMITED ? limit : kMaxPolls;
   auto arrived = [&](uint64_t *bar, int phase) {
     if (mbar_wait(bar, phase & 1, polls)) return true;
-    give_up(&sm.dead, err, lane);
     polls = 1;
+    if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
     return false;
   };
 
@@ -498,8 +486,7 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
       alive = arrived(&sm.fbar[b], j >> 1) && alive;
       const float *F = sm.fac[b] + (in ? lane : 0);
       bar_sync(kBarFull + b, kPatchThreads);  // the residual is there
-      // the row warps have waited for the values of this cell, not this one
-      alive = alive && !is_dead(&sm.dead);
+      // the row warps have waited for the values of this cell
       if (alive && lane == 0 && j + 2 < count) bring_values(j + 2, a2);
       // y_c = A^{-1} r_c
       float y0 = 0, y1 = 0, y2 = 0;
@@ -630,7 +617,11 @@ __global__ void __launch_bounds__(kPatchThreads, kCtas32) k_patch_sweep32(
     bar_sync(kBarRows, kRowLanes);    // everybody's; and cell j - 1 has been read
     gather(j + 2);
     if (alive) pattern(sm.ids[j & 3][kPatchPattern]);
-    alive = arrived(&sm.vbar[b], j >> 1) && alive;
+    if (!arrived(&sm.vbar[b], j >> 1)) {
+      // warp 7, which fills the stage again, does not wait for it itself
+      drain(&sm.vbar[b], j >> 1);
+      alive = false;
+    }
     float c0, c1, c2;
     row_sum(warp, t, sm.values[b], sm.u[g], &sm.p[g][0].x, s0, s1, bts, c0, c1, c2);
 #pragma unroll
@@ -666,7 +657,6 @@ struct Smem64 {
   double y[3][32];
   double rp[NP_LOC], t[NP_LOC];
   uint64_t vbar[ST], fbar[ST], ibar[3];
-  int dead;  // a wait of this CTA ran out
 };
 // resident CTAs per SM: 63 KB of shared memory with one stage, 106 KB with two
 __host__ __device__ constexpr int ctas64(int stages) { return stages == 1 ? 3 : 2; }
@@ -683,7 +673,7 @@ __host__ __device__ constexpr int ctas64(int stages) { return stages == 1 ? 3 : 
 template <int ST>
 __global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
     PatchLevel<double> L, const int *__restrict__ list, int n, const double *__restrict__ factors,
-    double damp, int odd, int *err, long long limit) {
+    double damp, int odd, int *err, int limit) {
   using S1 = Schur<1>;
   extern __shared__ __align__(16) unsigned char raw[];
   Smem64<ST> &sm = *reinterpret_cast<Smem64<ST> *>(raw);
@@ -698,17 +688,18 @@ __global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
     }
     for (int b = 0; b < 3; ++b) mbar_init(&sm.ibar[b], 1);
     fence_mbar_init();
-    sm.dead = 0;
     sm.u.set(kZeroSlot, 0.0, 0.0, 0.0);
     for (int m = 0; m < NP_LOC; ++m) sm.p[27][m] = 0.0;
     sm.r.set(27, 0.0, 0.0, 0.0);
   }
   __syncthreads();
-  long long polls = limit;  // as in the FP32 kernel
+  // as in the FP32 kernel; thread 0, which starts the copies, has waited for
+  // the last one of a stage itself
+  int polls = limit;
   auto arrived = [&](uint64_t *bar, int phase) {
     if (mbar_wait(bar, phase & 1, polls)) return true;
-    give_up(&sm.dead, err, lane);
     polls = 1;
+    if (lane == 0) atomicOr(err, PM_ERR_BULK_TIMEOUT);
     return false;
   };
   auto cell_of = [&](int c) { return __ldg(list + first + (size_t)c * G); };
@@ -823,7 +814,6 @@ __global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
       if (sl == 0) sm.rp[sub] = fi - c;
     }
     __syncthreads();
-    alive = alive && !is_dead(&sm.dead);
     if (alive && t == 0 && j + ST < count) {
       bring_values(j + ST, ST == 1 ? a1 : a2);
       nv = j + ST + 1;
@@ -1476,7 +1466,9 @@ int launch_patch_init() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
            cudaSuccess;
   };
-  return set(k_patch_sweep32, sizeof(Smem32)) && set(k_patch_sweep64<1>, sizeof(Smem64<1>)) &&
+  return set(k_patch_sweep32<false>, sizeof(Smem32)) &&
+                 set(k_patch_sweep32<true>, sizeof(Smem32)) &&
+                 set(k_patch_sweep64<1>, sizeof(Smem64<1>)) &&
                  set(k_patch_sweep64<2>, sizeof(Smem64<2>))
              ? 0
              : -1;
@@ -1491,13 +1483,14 @@ int launch_patch_begin(const PatchLevel<T> &L, const T *u, const T *rhs, int hb,
 
 template <typename T>
 int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T *factors, T damp,
-                        int odd, int *err, int num_sms, long long wait_limit, cudaStream_t s) {
+                        int odd, int *err, int num_sms, int wait_limit, cudaStream_t s) {
   if (n <= 0) return 0;
-  const long long limit = wait_limit > 0 ? wait_limit : kMaxPolls;
+  const int limit = wait_limit > 0 ? wait_limit : kMaxPolls;
   if constexpr (sizeof(T) == 4)
-    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *, long long>(
-        k_patch_sweep32, std::min(n, kCtas32 * num_sms), kPatchThreads, sizeof(Smem32), s, L, list,
-        n, factors, damp, odd, err, limit);
+    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *, int>(
+        wait_limit > 0 ? k_patch_sweep32<true> : k_patch_sweep32<false>,
+        std::min(n, kCtas32 * num_sms), kPatchThreads, sizeof(Smem32), s, L, list, n, factors,
+        damp, odd, err, limit);
   else {
     // Two stages while they hold all the cells of a CTA: with rows that come
     // from DRAM, two sweeps at 16^3 take 492 us against 541 with one stage.
@@ -1505,7 +1498,7 @@ int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T 
     // 64^3 979 against 1112.
     const int two = ctas64(2) * num_sms;
     const bool all = n <= 2 * two;
-    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *, long long>(
+    return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *, int>(
         all ? k_patch_sweep64<2> : k_patch_sweep64<1>,
         std::min(n, all ? two : ctas64(1) * num_sms), kPatchThreads,
         all ? sizeof(Smem64<2>) : sizeof(Smem64<1>), s, L, list, n, factors, damp, odd, err, limit);
@@ -1535,7 +1528,7 @@ int launch_patch_end(const PatchLevel<T> &L, T *u, const T *rhs, int hb, int np,
   template int launch_patch_begin<T>(const PatchLevel<T> &, const T *, const T *, int, int,       \
                                      cudaStream_t);                                               \
   template int launch_patch_colour<T>(const PatchLevel<T> &, const int *, int, const T *,         \
-                                      T, int, int *, int, long long, cudaStream_t);               \
+                                      T, int, int *, int, int, cudaStream_t);                     \
   template int launch_patch_between<T>(const PatchLevel<T> &, const T *, int, cudaStream_t);      \
   template int launch_patch_end<T>(const PatchLevel<T> &, T *, const T *, int, int, int,          \
                                    cudaStream_t);

@@ -80,7 +80,7 @@ __device__ __forceinline__ void substitute(const float *Fc, int lane, float &y0,
 __global__ void __launch_bounds__(kTmaWarps * 32, 1) k_vanka_apply_tma(
     DevCells cells, int nu, const int *__restrict__ list, int ncol, const float *__restrict__ F,
     const uint8_t *__restrict__ perm, const float *__restrict__ rbuf, float damp,
-    float *__restrict__ u, int *err, long long limit) {
+    float *__restrict__ u, int *err, int limit) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[kTmaWarps][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -153,11 +153,11 @@ int launch_vanka_apply_tma_init() {
 
 int launch_vanka_apply_tma(const DevCells &cells, int nu, const int *cell_list, int ncol,
                            const float *factors, const uint8_t *perm, const float *rbuf, float damp,
-                           float *u, int *err, int num_sms, long long wait_limit, cudaStream_t s) {
+                           float *u, int *err, int num_sms, int wait_limit, cudaStream_t s) {
   if (ncol <= 0) return 0;
   int grid = (ncol + kTmaWarps - 1) / kTmaWarps;
   if (grid > num_sms) grid = num_sms;
-  const long long limit = wait_limit > 0 ? wait_limit : kMaxPolls;
+  const int limit = wait_limit > 0 ? wait_limit : kMaxPolls;
   k_vanka_apply_tma<<<grid, kTmaWarps * 32, kTmaSmem, s>>>(cells, nu, cell_list, ncol, factors,
                                                            perm, rbuf, damp, u, err, limit);
   return ok() < 0 ? -1 : 1;
