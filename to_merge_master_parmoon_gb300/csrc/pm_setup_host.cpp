@@ -490,7 +490,9 @@ bool stack_levels(const pm_level_desc *d, int G, const StackSizes &coarse, Stack
 void row_order(const int *rowptr, int rows, std::vector<int> &order) {
   constexpr int kWindow = 4096, kClasses = 32;
   order.resize((size_t)rows);
-#pragma omp parallel for schedule(static)
+  // for fewer rows waking the threads took longer than the loop (5 to 10 ms in
+  // the first pm_add_level of a hierarchy; the loop takes 2.5 ns per row)
+#pragma omp parallel for schedule(static) if (rows > (1 << 20))
   for (int w = 0; w < rows; w += kWindow) {
     const int e = std::min(rows, w + kWindow);
     int at[kClasses + 1] = {0};
