@@ -798,9 +798,15 @@ pm_status build_patch(pm_handle *h, LevelDev &Lv, bool *fits) {
                                     h->stream));
   PM_TRY(check());
   if (bad) return PM_OK;
-  // places of the nodes in shared memory; a level whose cells hardly share
-  // patterns keeps the list order
-  if (Lv.pk_npat <= 4096) {
+  // Places of the nodes in shared memory that spare the FP32 sweeps bank
+  // conflicts: a sweep at 32^3 takes 201 instead of 207 us (216 for 227 in the
+  // numbering of a refinement tree), at 16^3 53.7 for 55.6; FP64 sweeps, bound
+  // by the FP64 pipe, take the same time with and without.  The search takes
+  // 27 us per pattern, so it is left out where fewer than 32 cells share one
+  // (a random numbering took 260 ms of set-up at 16^3); such a level keeps the
+  // list order.
+  constexpr int kCellsPerPattern = 32;
+  if (sizeof(T) == 4 && Lv.pk_npat * kCellsPerPattern <= Lv.ncells) {
     std::vector<unsigned char> host((size_t)Lv.pk_npat * kPatchPatternBytes);
     if (cudaMemcpyAsync(host.data(), pat, host.size(), cudaMemcpyDeviceToHost, h->stream) !=
         cudaSuccess)
