@@ -390,12 +390,15 @@ int pm_n_systems(pm_handle *h);
 pm_status pm_refactor(pm_handle *h, double *ms);
 
 /* Diagnostics: launches of this library's kernels since the handle was
- * created, and device bytes held (without the packed copy of the matrix rows
- * that the sweeps of one-block hexahedral levels use while memory allows: it
- * counts towards max_device_bytes but is given back when another allocation
- * needs the room). */
+ * created; device bytes that the handle cannot do without; and device bytes of
+ * the packed copy of the matrix rows that the sweeps of one-block hexahedral
+ * levels use while memory allows.  The copy is made for a level when it fits
+ * under max_device_bytes and leaves half of the device's memory free, given
+ * back level by level when another allocation of the handle needs the room, and
+ * made again by a later factorisation when there is room. */
 long long pm_kernel_launches(pm_handle *h);
 long long pm_device_bytes(pm_handle *h);
+long long pm_packed_bytes(pm_handle *h);
 /* Host bytes page-locked by pm_add_level under pin_host (0 if none took). */
 long long pm_pinned_bytes(pm_handle *h);
 /* Per-kernel timing of the two Vanka sweep kernels while profiling is

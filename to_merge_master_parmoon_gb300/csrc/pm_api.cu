@@ -91,7 +91,8 @@ struct LevelDev {
   // gathers from and updates; mixed precision, hexahedral smoothed levels
   float4 *ux = nullptr;
   // packed rows of a one-block hexahedral level (pm_vanka_patch.cu): 0 not
-  // looked at yet, 1 in use, -1 not available (mesh shape, memory)
+  // looked at yet, 1 in use, -1 not available (mesh shape), -2 no room (looked
+  // at again by the next factorisation)
   int pk = 0;
   bool pk_stale = true;  // matrix values newer than the packed copy
   // B is not the one of the last factorisation: the packed sweeps read the
@@ -278,7 +279,7 @@ pm_status cuda_fail(pm_handle *h, const char *what) {
   return (e == cudaErrorMemoryAllocation) ? PM_OOM : PM_CUDA_ERROR;
 }
 
-bool release_patches(pm_handle *h);
+bool release_patch(pm_handle *h, long long need);
 
 template <typename T>
 pm_status dalloc_once(pm_handle *h, T **p, size_t count) {
@@ -304,14 +305,16 @@ pm_status dalloc_once(pm_handle *h, T **p, size_t count) {
 }
 
 // Device memory of the handle.  The packed rows are a copy that the sweeps
-// can do without: when an allocation does not fit, they are given back first.
+// can do without: when an allocation does not fit, they are given back first,
+// one level after the other until it does.
 template <typename T>
 pm_status dalloc(pm_handle *h, T **p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
-  const pm_status s = dalloc_once(h, p, count);
-  if (s != PM_OOM || h->patch_alloc || !release_patches(h)) return s;
-  return dalloc_once(h, p, count);
+  pm_status s = dalloc_once(h, p, count);
+  while (s == PM_OOM && !h->patch_alloc && release_patch(h, (long long)(count * sizeof(T))))
+    s = dalloc_once(h, p, count);
+  return s;
 }
 
 // CSR value / column arrays: padded by 8 zero entries so that the Vanka
@@ -703,7 +706,6 @@ void drop_patch(pm_handle *h, LevelDev &Lv) {
   Lv.pk_ids = nullptr;
   Lv.pk_flips = nullptr;
   Lv.pk_patterns = Lv.pk_values = Lv.pk_u = Lv.pk_p = nullptr;
-  Lv.pk = -1;
 }
 
 void drop_graphs(pm_handle *h) {
@@ -714,16 +716,49 @@ void drop_graphs(pm_handle *h) {
     }
 }
 
-bool release_patches(pm_handle *h) {
-  bool any = false;
+long long patch_bytes(const pm_handle *h, const LevelDev &Lv) {
+  long long n = 0;
+  for (const auto &m : Lv.patch_arrays(mixed(h) ? sizeof(float) : sizeof(double)))
+    if (m.p) n += m.bytes;
+  return n;
+}
+
+// Gives back the packed rows of one level: the smallest that hold `need`
+// bytes, else the largest.  false: none are held.
+bool release_patch(pm_handle *h, long long need) {
+  LevelDev *best = nullptr;
+  long long have = 0;
   for (LevelDev &Lv : h->L) {
-    if (Lv.pk_values) any = true;
+    const long long n = patch_bytes(h, Lv);
+    if (n > 0 && (!best || (have < need ? n > have : n >= need && n < have))) {
+      best = &Lv;
+      have = n;
+    }
   }
-  if (!any) return false;
+  if (!best) return false;
   cudaStreamSynchronize(h->stream);
   drop_graphs(h);  // they launch the packed sweeps
-  for (LevelDev &Lv : h->L) drop_patch(h, Lv);
+  drop_patch(h, *best);
+  best->pk = -2;
   return true;
+}
+
+// Room for the packed rows of a level (their patterns not counted): under the
+// handle's cap, and with half of the device still free after them, so that
+// this copy, which other handles and programs cannot ask back, never takes what
+// they may need (one in FP64 takes 8.7 GB at 64^3).
+bool patch_room(const pm_handle *h, const LevelDev &Lv) {
+  const long long es = mixed(h) ? sizeof(float) : sizeof(double);
+  long long n = 0;
+  for (const auto &m : Lv.patch_arrays(es)) n += m.bytes;
+  if (h->opt.max_device_bytes > 0 && h->bytes + h->patch_bytes + n > h->opt.max_device_bytes)
+    return false;
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (long long)free - n >= (long long)(total / 2);
 }
 
 // Packed rows of one level, made on the device.  *fits: the mesh and the CSR pattern have the layout's shape.
@@ -855,7 +890,7 @@ pm_status ensure_patches(pm_handle *h, bool factoring) {
   if (h->opt.residual_variant != 0) return PM_OK;  // a CSR kernel is asked for
   for (size_t l = 1; l < h->L.size(); ++l) {
     LevelDev &Lv = h->L[l];
-    if (Lv.pk < 0 || !Lv.schur() || Lv.ncells == 0) continue;
+    if (Lv.pk == -1 || (Lv.pk == -2 && !factoring) || !Lv.schur() || Lv.ncells == 0) continue;
     if (Lv.pk == 1) {
       if (Lv.pk_stale)
         PM_LAUNCH(launch_patch_pack<T>(patch_level<T>(h, Lv), Lv.op<T>(), Lv.ncells, h->stream));
@@ -863,15 +898,18 @@ pm_status ensure_patches(pm_handle *h, bool factoring) {
       Lv.pk_stale = false;
       continue;
     }
+    Lv.pk = -2;
+    if (!patch_room(h, Lv)) continue;
     const std::string err = h->err;
     bool fits = false;
     h->patch_alloc = true;
     const pm_status st = build_patch<T>(h, Lv, &fits);
     h->patch_alloc = false;
-    if (st != PM_OK && st != PM_OOM) return st;
-    if (st == PM_OOM || !fits) {
+    if (st != PM_OK || !fits) {
       cudaStreamSynchronize(h->stream);
       drop_patch(h, Lv);
+      if (st != PM_OK && st != PM_OOM) return st;
+      if (st == PM_OK) Lv.pk = -1;
       h->err = err;
       continue;
     }
@@ -2698,6 +2736,7 @@ pm_status pm_solve_batch(pm_handle *const *hs, int n, double *const *sols,
 
 long long pm_kernel_launches(pm_handle *h) { return h ? h->launches : 0; }
 long long pm_device_bytes(pm_handle *h) { return h ? h->bytes : 0; }
+long long pm_packed_bytes(pm_handle *h) { return h ? h->patch_bytes : 0; }
 long long pm_pinned_bytes(pm_handle *h) { return h ? h->pinned_bytes : 0; }
 
 pm_status pm_profile_enable(pm_handle *h, int enable) {

@@ -108,6 +108,10 @@ class PmSolver:
     def device_bytes(self) -> int:
         return self._lib.pm_device_bytes(self._h)
 
+    @property
+    def packed_bytes(self) -> int:
+        return self._lib.pm_packed_bytes(self._h)
+
     def profile(self, enable: bool = True):
         self._check(self._lib.pm_profile_enable(self._h, int(enable)), "pm_profile_enable")
 
