@@ -1196,9 +1196,10 @@ __global__ void k_patch_assign(int *ids, const int *pattern, int ncells) {
 }
 
 // Pattern of a cell from the CSR patterns and its patch list (once per level,
-// at set-up).  MODE 0: a hash of the pattern into hash[cell]; 1: the pattern
-// of cell which[blockIdx.x] into patterns[blockIdx.x]; 2: compare with the
-// pattern that the cell was given.  Rows that do not fit set *bad.
+// at set-up).  MODE 0: a hash of the pattern into hash[cell] (the words through
+// the finaliser of splitmix64, Steele, Lea and Flood 2014, summed); 1: the
+// pattern of cell which[blockIdx.x] into patterns[blockIdx.x]; 2: compare with
+// the pattern that the cell was given.  Rows that do not fit set *bad.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_patch_pattern(
     const int *ids_all, const int *a_rowptr, const int *a_col, const int *b_rowptr,

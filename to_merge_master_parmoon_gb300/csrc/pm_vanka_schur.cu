@@ -377,8 +377,10 @@ __global__ void __launch_bounds__(kApplyWarps * 32) k_schur_apply(
 // compared as values; a NaN counts as different)
 __global__ void __launch_bounds__(256) k_block_structure(DevOp<double> op, long long n,
                                                          int *flag) {
-  // every value is loaded and compared without short-circuit branches: the
-  // version with || left whole levels of fully coupled blocks unflagged
+  // One reduction of both bits: two votes, (any(nz) ? 1 : 0) | (any(differ) ? 2
+  // : 0), gave 0 where both hold (nvcc 13.0.88, every size from one entry on;
+  // either vote alone, and both bits without a vote, were right), so that
+  // levels with coupled and different blocks were taken for decoupled ones.
   unsigned bits = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
