@@ -670,7 +670,7 @@ __host__ __device__ constexpr int ctas64(int stages) { return stages == 1 ? 3 : 
 // the SM use the pipe meanwhile (83 % busy at 32^3; 72 % with ST = 2).  Rows and
 // factors from DRAM at 64^3, one colour: 979 us (1.47 TB/s; the CSR kernels
 // take 1,046), 32^3 134 (162), 16^3 29 (69), 8^3 12.6 (52).
-template <int ST>
+template <int ST, bool LIMITED>
 __global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
     PatchLevel<double> L, const int *__restrict__ list, int n, const double *__restrict__ factors,
     double damp, int odd, int *err, int limit) {
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(kPatchThreads, ctas64(ST)) k_patch_sweep64(
   __syncthreads();
   // as in the FP32 kernel; thread 0, which starts the copies, has waited for
   // the last one of a stage itself
-  int polls = limit;
+  int polls = LIMITED ? limit : kMaxPolls;
   auto arrived = [&](uint64_t *bar, int phase) {
     if (mbar_wait(bar, phase & 1, polls)) return true;
     polls = 1;
@@ -1469,8 +1469,10 @@ int launch_patch_init() {
   };
   return set(k_patch_sweep32<false>, sizeof(Smem32)) &&
                  set(k_patch_sweep32<true>, sizeof(Smem32)) &&
-                 set(k_patch_sweep64<1>, sizeof(Smem64<1>)) &&
-                 set(k_patch_sweep64<2>, sizeof(Smem64<2>))
+                 set(k_patch_sweep64<1, false>, sizeof(Smem64<1>)) &&
+                 set(k_patch_sweep64<1, true>, sizeof(Smem64<1>)) &&
+                 set(k_patch_sweep64<2, false>, sizeof(Smem64<2>)) &&
+                 set(k_patch_sweep64<2, true>, sizeof(Smem64<2>))
              ? 0
              : -1;
 }
@@ -1500,7 +1502,8 @@ int launch_patch_colour(const PatchLevel<T> &L, const int *list, int n, const T 
     const int two = ctas64(2) * num_sms;
     const bool all = n <= 2 * two;
     return launch_chained<PatchLevel<T>, const int *, int, const T *, T, int, int *, int>(
-        all ? k_patch_sweep64<2> : k_patch_sweep64<1>,
+        wait_limit > 0 ? (all ? k_patch_sweep64<2, true> : k_patch_sweep64<1, true>)
+                       : (all ? k_patch_sweep64<2, false> : k_patch_sweep64<1, false>),
         std::min(n, all ? two : ctas64(1) * num_sms), kPatchThreads,
         all ? sizeof(Smem64<2>) : sizeof(Smem64<1>), s, L, list, n, factors, damp, odd, err, limit);
   }
